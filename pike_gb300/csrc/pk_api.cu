@@ -172,6 +172,7 @@ int pk_create(pk_ctx** out, int device) {
     }
     c->ctr.alloc(1);
     c->cam.alloc(1);
+    c->scratch_pool = create_scratch_pool(device);
     c->cast_scratch = noalloc_scratch_address();
     check(cudaMemsetAsync(c->ctr.p, 0, sizeof(Counters), c->stream), "memset");
     check(cudaStreamSynchronize(c->stream), "sync");
@@ -179,6 +180,7 @@ int pk_create(pk_ctx** out, int device) {
   });
   if (rc != PK_OK) {
     std::fprintf(stderr, "pk_create: %s\n", c->err.c_str());
+    if (c->scratch_pool) cudaMemPoolDestroy(c->scratch_pool);
     delete c;
     return rc;
   }
@@ -209,6 +211,7 @@ int pk_destroy(pk_ctx* c) {
   for (auto e : c->event_pool) cudaEventDestroy(e);
   if (c->t0) cudaEventDestroy(c->t0);
   if (c->t1) cudaEventDestroy(c->t1);
+  if (c->scratch_pool) cudaMemPoolDestroy(c->scratch_pool);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return PK_OK;
@@ -383,7 +386,7 @@ int pk_materials_download(pk_ctx* c, uint32_t* n_mats, uint32_t* n_layers, int32
 static int build_wide(pk_ctx* c) {
   std::string why;
   uint32_t n = 0, depth = 0;
-  if (build_wide_bvh_gpu(c->stream, c->nodes5.p, c->n_nodes, c->tri4_leaf.p, c->n_leaf_tris, c->verts4.p,
+  if (build_wide_bvh_gpu(c->scratch(), c->nodes5.p, c->n_nodes, c->tri4_leaf.p, c->n_leaf_tris, c->verts4.p,
                          c->bvh_verts, c->wide, c->wide_tris, n, depth, why))
     return fail(c, PK_ERR_ARG, "wide BVH: " + why);
   c->wide_nodes = n;
@@ -398,7 +401,7 @@ static int build_wide(pk_ctx* c) {
 static int build_exact(pk_ctx* c) {
   int32_t root = 0;
   std::string why;
-  if (build_exact_binary_gpu(c->stream, c->nodes5.p, c->n_nodes, c->tri4_leaf.p, c->n_leaf_tris, c->verts4.p,
+  if (build_exact_binary_gpu(c->scratch(), c->nodes5.p, c->n_nodes, c->tri4_leaf.p, c->n_leaf_tris, c->verts4.p,
                              c->bvh_verts, c->exact, c->exact_tris, root, why))
     return fail(c, PK_ERR_ARG, "exact binary records: " + why);
   c->exact_root = root;
@@ -409,24 +412,28 @@ static int build_exact(pk_ctx* c) {
 
 static int finish_bvh(pk_ctx* c) {
   c->wide_ready = false;
-  c->wide.release();
-  c->wide_tris.release();
   c->exact_ready = false;
-  c->exact.release();
-  c->exact_tris.release();
+  if (!(c->trace_mode & TRACE_WIDE)) {
+    c->wide.release();
+    c->wide_tris.release();
+  }
+  if (!(c->trace_mode & TRACE_EXACT)) {
+    c->exact.release();
+    c->exact_tris.release();
+  }
   c->inner.alloc(4 * (size_t)std::max<uint32_t>(c->n_nodes, 1u));
   c->inner32.alloc(2 * (size_t)std::max<uint32_t>(c->n_nodes, 1u));
   c->tris.alloc(3 * (size_t)std::max<uint32_t>(c->n_leaf_tris, 1u));
-  DevBuf<int> root(1);
-  DevBuf<uint32_t> err(1);
-  check(cudaMemsetAsync(err.p, 0, 4, c->stream), "memset");
-  if (convert_bvh(c->stream, c->nodes5.p, c->n_nodes, c->tri4_leaf.p, c->n_leaf_tris, c->verts4.p, c->bvh_verts,
-                  c->inner.p, c->inner32.p, c->tris.p, root.p, err.p))
+  TmpBuf<uint32_t> out(c->scratch(), 2);  // the root's code, errors
+  check(cudaMemsetAsync(out.p, 0, 8, c->stream), "memset");
+  if (convert_bvh(c->scratch(), c->nodes5.p, c->n_nodes, c->tri4_leaf.p, c->n_leaf_tris, c->verts4.p, c->bvh_verts,
+                  c->inner.p, c->inner32.p, c->tris.p, reinterpret_cast<int*>(out.p), out.p + 1))
     throw CudaError(std::string("convert_bvh: ") + cudaGetErrorString(cudaGetLastError()));
-  uint32_t herr = 0;
-  check(cudaMemcpy(&c->root, root.p, 4, cudaMemcpyDeviceToHost), "D2H");
-  check(cudaMemcpy(&herr, err.p, 4, cudaMemcpyDeviceToHost), "D2H");
-  if (herr) return fail(c, PK_ERR_ARG, "malformed BVH (child index, leaf size >= 128 or vertex index out of range)");
+  uint32_t back[2] = {0, 0};
+  check(cudaMemcpyAsync(back, out.p, 8, cudaMemcpyDeviceToHost, c->stream), "D2H");
+  check(cudaStreamSynchronize(c->stream), "sync");
+  c->root = (int)back[0];
+  if (back[1]) return fail(c, PK_ERR_ARG, "malformed BVH (child index, leaf size >= 128 or vertex index out of range)");
   c->bvh_ready = true;
   if (c->trace_mode & TRACE_WIDE) {
     const int rc = build_wide(c);
@@ -495,8 +502,8 @@ int pk_bvh_build(pk_ctx* c, int mode) {
     BvhOut out;
     std::string why;
     const int rc = mode == PK_BVH_SWEEP
-                       ? build_bvh_sweep(c->stream, c->pos.p, c->n_verts, c->tri4.p, c->n_tris, out, why)
-                       : build_bvh_binned(c->stream, c->pos.p, c->n_verts, c->tri4.p, c->n_tris, out, why);
+                       ? build_bvh_sweep(c->scratch(), c->pos.p, c->n_verts, c->tri4.p, c->n_tris, out, why)
+                       : build_bvh_binned(c->scratch(), c->pos.p, c->n_verts, c->tri4.p, c->n_tris, out, why);
     if (rc) return fail(c, PK_ERR_ARG, "pk_bvh_build: " + why);
     c->nodes5 = std::move(out.nodes5);
     c->node_box_d = std::move(out.node_box);
@@ -536,7 +543,7 @@ int pk_bvh_download(pk_ctx* c, int32_t* nodes5, int32_t* tri4_leaf, float* verts
 // The alias table of PK_ENV_ALIAS from the current environment's texels.
 static int build_alias(pk_ctx* c) {
   std::string why;
-  if (build_env_alias_gpu(c->stream, c->rgbe.p, c->env_w, c->env_h, c->env_alias, c->alias_pdf, why))
+  if (build_env_alias_gpu(c->scratch(), c->rgbe.p, c->env_w, c->env_h, c->env_alias, c->alias_pdf, why))
     return fail(c, PK_ERR_ARG, "alias table: " + why);
   c->alias_ready = true;
   c->invalidate_graph();
@@ -568,7 +575,7 @@ int pk_env_build(pk_ctx* c, const uint8_t* rgbe, uint32_t w, uint32_t h) {
     upload(c->rgbe, rgbe, (size_t)w * h, c->stream);
     std::string why;
     uint32_t nb = 0;
-    if (build_env_tables_gpu(c->stream, c->rgbe.p, w, h, c->bins, nb, c->coords, c->pdf, why)) {
+    if (build_env_tables_gpu(c->scratch(), c->rgbe.p, w, h, c->bins, nb, c->coords, c->pdf, why)) {
       c->env_ready = false;
       return fail(c, PK_ERR_ARG, "pk_env_build: " + why);
     }

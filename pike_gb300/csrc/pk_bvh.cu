@@ -493,47 +493,48 @@ double js_max(double a, double b) { return (a != a || b != b) ? NAN : (a > b ? a
 
 }  // namespace
 
-int build_bvh_sweep(cudaStream_t s, const double* pos3, uint32_t n_verts, const int4* tri4, uint32_t T,
+int build_bvh_sweep(const Scratch& w, const double* pos3, uint32_t n_verts, const int4* tri4, uint32_t T,
                     BvhOut& out, std::string& why) {
   if (T == 0) { why = "no triangles"; return 1; }
   if (T > (1u << 26)) { why = "too many triangles"; return 1; }
+  const cudaStream_t s = w.s;
   int dev = 0, sms = 1;
   cudaGetDevice(&dev);
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
 
-  DevBuf<Box6> tri_box(T);
-  DevBuf<unsigned long long> keys(3 * (size_t)T), keys_tmp(T);
-  DevBuf<uint32_t> vals(3 * (size_t)T), vals_tmp(T);
+  TmpBuf<uint32_t> st_aux(w, 2);
+  check(cudaMemsetAsync(st_aux.p, 0, 8, s), "memset");
+  TmpBuf<Box6> tri_box(w, T);
+  TmpBuf<unsigned long long> keys(w, 3 * (size_t)T), keys_tmp(w, 3 * (size_t)T);
+  TmpBuf<uint32_t> vals(w, 3 * (size_t)T), vals_tmp(w, 3 * (size_t)T);
   k_tri_boxes<<<blocks(T), 256, 0, s>>>(pos3, tri4, T, tri_box.p, keys.p, vals.p);
   check(cudaGetLastError(), "k_tri_boxes");
-  for (int a = 0; a < 3; a++)
-    radix_sort_pairs_u64(s, reinterpret_cast<uint64_t*>(keys.p) + (size_t)a * T, vals.p + (size_t)a * T,
-                         reinterpret_cast<uint64_t*>(keys_tmp.p), vals_tmp.p, T, 64);
+  radix_sort_pairs_u64(w, reinterpret_cast<uint64_t*>(keys.p), vals.p, reinterpret_cast<uint64_t*>(keys_tmp.p),
+                       vals_tmp.p, T, 3, st_aux.p + 1);
   keys.release();
   keys_tmp.release();
   vals_tmp.release();
 
-  DevBuf<int32_t> A(3 * (size_t)T), A2(3 * (size_t)T), seg(T), seg2(T);
+  TmpBuf<int32_t> A(w, 3 * (size_t)T), A2(w, 3 * (size_t)T), seg(w, T), seg2(w, T);
   check(cudaMemcpyAsync(A.p, vals.p, 3 * (size_t)T * 4, cudaMemcpyDeviceToDevice, s), "memcpy");
   vals.release();
   check(cudaMemsetAsync(seg.p, 0, (size_t)T * 4, s), "memset");
-  DevBuf<uint32_t> nstart(T), ncount(T), nbfs(T), nstart2(T), ncount2(T), nbfs2(T);
-  DevBuf<double> saf(T), sab(T), cost(3 * (size_t)T), psa(T);
-  DevBuf<unsigned long long> best_cost(T);
-  DevBuf<uint32_t> best_idx(T), is_inner(T), inner_cnt(T), leaf_cnt(T), split_axis(T), nleft(T);
-  DevBuf<uint32_t> inner_rank(T), new_base(T), leaf_base(T), X(T), fvals(T), totals(4);
-  DevBuf<uint8_t> left(T);
-  DevBuf<Box6> level_box(T);
+  TmpBuf<uint32_t> nstart(w, T), ncount(w, T), nbfs(w, T), nstart2(w, T), ncount2(w, T), nbfs2(w, T);
+  TmpBuf<double> saf(w, T), sab(w, T), cost(w, 3 * (size_t)T), psa(w, T);
+  TmpBuf<unsigned long long> best_cost(w, T);
+  TmpBuf<uint32_t> best_idx(w, T), is_inner(w, T), inner_cnt(w, T), leaf_cnt(w, T), split_axis(w, T), nleft(w, T);
+  TmpBuf<uint32_t> inner_rank(w, T), new_base(w, T), leaf_base(w, T), X(w, T), fvals(w, T), totals(w, 4);
+  TmpBuf<uint8_t> left(w, T);
+  TmpBuf<Box6> level_box(w, T);
   const uint32_t max_nodes = 2 * T - 1;
-  DevBuf<Box6> node_box(max_nodes);
-  DevBuf<int32_t> nodes5(5 * (size_t)max_nodes);
-  DevBuf<int32_t> leaf_ids(T);
+  TmpBuf<Box6> node_box(w, max_nodes);
+  TmpBuf<int32_t> nodes5(w, 5 * (size_t)max_nodes);
+  TmpBuf<int32_t> leaf_ids(w, T);
   const uint32_t seg_tiles = (T + SEG_TILE - 1) / SEG_TILE;
-  DevBuf<uint32_t> st_status(seg_tiles), st_aggflag(seg_tiles), st_aux(2);
-  DevBuf<Box6> st_agg(seg_tiles), st_incl(seg_tiles);
+  TmpBuf<uint32_t> st_status(w, seg_tiles), st_aggflag(w, seg_tiles);
+  TmpBuf<Box6> st_agg(w, seg_tiles), st_incl(w, seg_tiles);
   const SegState st{st_status.p, st_agg.p, st_aggflag.p, st_incl.p, st_aux.p, st_aux.p + 1};
-  check(cudaMemsetAsync(st_aux.p, 0, 8, s), "memset");
-  DevBuf<uint32_t> derr(1);
+  TmpBuf<uint32_t> derr(w, 1);
   check(cudaMemsetAsync(derr.p, 0, 4, s), "memset");
 
   const uint32_t zero = 0;
@@ -571,9 +572,9 @@ int build_bvh_sweep(cudaStream_t s, const double* pos3, uint32_t n_verts, const 
     k_decide<<<blocks(m), 256, 0, s>>>(m, ncount.p, nbfs.p, best_cost.p, best_idx.p, level_box.p, node_box.p,
                                         is_inner.p, inner_cnt.p, leaf_cnt.p, split_axis.p, nleft.p, derr.p);
     check(cudaGetLastError(), "bvh level");
-    scan_exclusive_u32(s, is_inner.p, inner_rank.p, m, totals.p + 0);
-    scan_exclusive_u32(s, inner_cnt.p, new_base.p, m, totals.p + 1);
-    scan_exclusive_u32(s, leaf_cnt.p, leaf_base.p, m, totals.p + 2);
+    scan_exclusive_u32(w, is_inner.p, inner_rank.p, m, totals.p + 0, st_aux.p + 1);
+    scan_exclusive_u32(w, inner_cnt.p, new_base.p, m, totals.p + 1, st_aux.p + 1);
+    scan_exclusive_u32(w, leaf_cnt.p, leaf_base.p, m, totals.p + 2, st_aux.p + 1);
     uint32_t tot[3];
     check(cudaMemcpyAsync(tot, totals.p, 12, cudaMemcpyDeviceToHost, s), "D2H");
     check(cudaStreamSynchronize(s), "sync");
@@ -586,7 +587,7 @@ int build_bvh_sweep(cudaStream_t s, const double* pos3, uint32_t n_verts, const 
       const int32_t* Aa = A.p + (size_t)a * T;
       if (n_inner) {
         k_flag_vals<<<blocks(n), 256, 0, s>>>(Aa, seg.p, n, is_inner.p, left.p, fvals.p);
-        scan_exclusive_u32(s, fvals.p, X.p, n, nullptr);
+        scan_exclusive_u32(w, fvals.p, X.p, n, nullptr, st_aux.p + 1);
       }
       k_scatter<<<blocks(n), 256, 0, s>>>(Aa, seg.p, n, a, nstart.p, ncount.p, is_inner.p, split_axis.p, nleft.p,
                                            inner_rank.p, new_base.p, leaf_base.p, leaf_offset, left.p,
@@ -1132,15 +1133,16 @@ __global__ void k_init_bins(Bin* bins, size_t n) {
 
 }  // namespace
 
-int build_bvh_binned(cudaStream_t s, const double* pos3, uint32_t n_verts, const int4* tri4, uint32_t T,
+int build_bvh_binned(const Scratch& w, const double* pos3, uint32_t n_verts, const int4* tri4, uint32_t T,
                      BvhOut& out, std::string& why) {
   if (T == 0) { why = "no triangles"; return 1; }
   if (T >= (1u << 24)) { why = "too many triangles for the 24-bit leaf base"; return 1; }
+  const cudaStream_t s = w.s;
   const uint32_t max_nodes = 2 * T;
-  DevBuf<Box6> tri_box(T), node_box(max_nodes);
-  DevBuf<uint32_t> A(T), A2(T), flags(T), X(T), counter(1), derr(1);
-  DevBuf<int32_t> nodes5(5 * (size_t)max_nodes);
-  DevBuf<Bin> root_bin(1);
+  TmpBuf<Box6> tri_box(w, T), node_box(w, max_nodes);
+  TmpBuf<uint32_t> A(w, T), A2(w, T), flags(w, T), X(w, T), counter(w, 1), derr(w, 1);
+  TmpBuf<int32_t> nodes5(w, 5 * (size_t)max_nodes);
+  TmpBuf<Bin> root_bin(w, 1);
   check(cudaMemsetAsync(derr.p, 0, 4, s), "memset");
   k_tri_boxes_plain<<<blocks(T), 256, 0, s>>>(pos3, tri4, T, tri_box.p, A.p);
   k_init_bins<<<1, 32, 0, s>>>(root_bin.p, 1);
@@ -1171,9 +1173,9 @@ int build_bvh_binned(cudaStream_t s, const double* pos3, uint32_t n_verts, const
   }
   // per-level buffers at their largest: every large node holds more than BIN_SMALL triangles
   const uint32_t m_max = T / BIN_SMALL + 2;
-  DevBuf<NodeInfo> d_nodes(m_max);
-  DevBuf<Tile> d_tiles(T / BIN_TILE + m_max + 1);
-  DevBuf<Bin> bins((size_t)m_max * 3 * NB);
+  TmpBuf<NodeInfo> d_nodes(w, m_max);
+  TmpBuf<Tile> d_tiles(w, T / BIN_TILE + m_max + 1);
+  TmpBuf<Bin> bins(w, (size_t)m_max * 3 * NB);
   uint32_t depth = 1;
   while (!large.empty()) {
     depth++;
@@ -1191,7 +1193,7 @@ int build_bvh_binned(cudaStream_t s, const double* pos3, uint32_t n_verts, const
     k_choose_large<<<blocks(m, 64), 64, 0, s>>>(d_nodes.p, m, bins.p, next, nodes5.p, node_box.p);
     check(cudaMemsetAsync(flags.p, 0, (size_t)T * 4, s), "memset");
     k_left_flags_binned<<<(unsigned)tiles.size(), BIN_THREADS, 0, s>>>(d_tiles.p, d_nodes.p, A.p, tri_box.p, flags.p);
-    scan_exclusive_u32(s, flags.p, X.p, T, nullptr);
+    scan_exclusive_u32(w, flags.p, X.p, T, nullptr, derr.p);
     check(cudaMemcpyAsync(A2.p, A.p, (size_t)T * 4, cudaMemcpyDeviceToDevice, s), "memcpy");
     k_partition_binned<<<(unsigned)tiles.size(), BIN_THREADS, 0, s>>>(d_tiles.p, d_nodes.p, A.p, flags.p, X.p, A2.p,
                                                                       derr.p);
@@ -1224,7 +1226,7 @@ int build_bvh_binned(cudaStream_t s, const double* pos3, uint32_t n_verts, const
   }
   check(cudaMemcpyAsync(counter.p, &next, 4, cudaMemcpyHostToDevice, s), "H2D");
   if (!small.empty()) {
-    DevBuf<SmallTask> d_small(small.size());
+    TmpBuf<SmallTask> d_small(w, small.size());
     check(cudaMemcpyAsync(d_small.p, small.data(), small.size() * sizeof(SmallTask), cudaMemcpyHostToDevice, s), "H2D");
     const unsigned nb = (unsigned)((small.size() + SMALL_WARPS - 1) / SMALL_WARPS);
     k_build_small<<<nb, SMALL_WARPS * 32, 0, s>>>(d_small.p, (uint32_t)small.size(), A.p, tri_box.p, nodes5.p,

@@ -23,12 +23,12 @@ struct BvhOut {
 // (axis, index) order, `cost > n` makes a leaf, and a stable partition of the
 // other two axis orders forms the children.  Levels are emitted in BFS order,
 // which is serializeTree's order.  Returns non-zero with a reason on failure.
-int build_bvh_sweep(cudaStream_t s, const double* pos3, uint32_t n_verts, const int4* tri4, uint32_t n_tris,
+int build_bvh_sweep(const Scratch& scratch, const double* pos3, uint32_t n_verts, const int4* tri4, uint32_t n_tris,
                     BvhOut& out, std::string& why);
 
 // Binned SAH (16 bins per axis, leaves of at most 8 triangles): a different,
 // faster-to-build topology than bvh.js; same output layout.
-int build_bvh_binned(cudaStream_t s, const double* pos3, uint32_t n_verts, const int4* tri4, uint32_t n_tris,
+int build_bvh_binned(const Scratch& scratch, const double* pos3, uint32_t n_verts, const int4* tri4, uint32_t n_tris,
                      BvhOut& out, std::string& why);
 
 }  // namespace pk

@@ -168,6 +168,8 @@ struct pk_ctx {
   DevBuf<int2> diff_bins, diff_coords;
   DevBuf<float> diff_pdf;
   bool diff_env_ready = false;
+  cudaMemPool_t scratch_pool = nullptr;  // the builders' temporaries (pk_util.h)
+  pk::Scratch scratch() const { return pk::Scratch{stream, scratch_pool}; }
   void* cast_scratch = nullptr;  // pk_cast_rays_noalloc's static scratch on this device (set by pk_create)
 
   RayQ R(int i) { return slot[0].R(i); }

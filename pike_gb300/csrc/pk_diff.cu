@@ -590,7 +590,7 @@ extern "C" int pk_diff_set_env_sampling(pk_ctx* c, const float* env_rgb, uint32_
     std::string why;
     uint32_t nb = 0;
     c->diff_env_ready = false;
-    if (build_env_tables_gpu_f32(c->stream, env_rgb, w, h, c->diff_bins, nb, c->diff_coords, c->diff_pdf, why)) {
+    if (build_env_tables_gpu_f32(c->scratch(), env_rgb, w, h, c->diff_bins, nb, c->diff_coords, c->diff_pdf, why)) {
       c->err = "pk_diff_set_env_sampling: " + why;
       return PK_ERR_ARG;
     }

@@ -236,19 +236,24 @@ namespace {
 
 // The tables from per-texel radiance `rad` with sort keys and values already
 // set (the radiance kernels above).
-int build_from_radiance(cudaStream_t s, uint32_t w, uint32_t h, DevBuf<double>& rad,
-                        DevBuf<unsigned long long>& keys, DevBuf<uint32_t>& vals, DevBuf<int2>& bins_out,
+int build_from_radiance(const Scratch& sc, uint32_t w, uint32_t h, TmpBuf<double>& rad,
+                        TmpBuf<unsigned long long>& keys, TmpBuf<uint32_t>& vals, DevBuf<int2>& bins_out,
                         uint32_t& nb_out, DevBuf<int2>& coords_out, DevBuf<float>& pdf_out, std::string& why) {
+  const cudaStream_t s = sc.s;
   const uint32_t n = w * h;
-  DevBuf<unsigned long long> keys_tmp(n);
-  DevBuf<uint32_t> vals_tmp(n);
+  TmpBuf<unsigned long long> keys_tmp(sc, n);
+  TmpBuf<uint32_t> vals_tmp(sc, n), err(sc, 1);
+  check(cudaMemsetAsync(err.p, 0, 4, s), "memset");
   std::vector<double> r(n);
   check(cudaMemcpyAsync(r.data(), rad.p, (size_t)n * 8, cudaMemcpyDeviceToHost, s), "D2H");
-  radix_sort_pairs_u64(s, reinterpret_cast<uint64_t*>(keys.p), vals.p, reinterpret_cast<uint64_t*>(keys_tmp.p),
-                       vals_tmp.p, n, 64);
+  radix_sort_pairs_u64(sc, reinterpret_cast<uint64_t*>(keys.p), vals.p, reinterpret_cast<uint64_t*>(keys_tmp.p),
+                       vals_tmp.p, n, 1, err.p);
+  uint32_t herr = 0;
+  check(cudaMemcpyAsync(&herr, err.p, 4, cudaMemcpyDeviceToHost, s), "D2H");
   std::vector<uint32_t> order(n);
   check(cudaMemcpyAsync(order.data(), vals.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s), "D2H");
   check(cudaStreamSynchronize(s), "sync");
+  if (herr) { why = "radix sort look-back timed out"; return 1; }
   // totalRadiance += rad (row-major) and brightestTexel = max(rad, brightest)
   double total = 0.0, brightest = 0.0;
   for (uint32_t i = 0; i < n; i++) {
@@ -291,14 +296,14 @@ int build_from_radiance(cudaStream_t s, uint32_t w, uint32_t h, DevBuf<double>& 
 
 // Builds bins (<= 257 entries), sorted coordinates and the pdf for a w x h
 // RGBE image already on the device.  Returns non-zero with a reason on failure.
-int build_env_tables_gpu(cudaStream_t s, const uchar4* rgbe, uint32_t w, uint32_t h, DevBuf<int2>& bins_out,
+int build_env_tables_gpu(const Scratch& sc, const uchar4* rgbe, uint32_t w, uint32_t h, DevBuf<int2>& bins_out,
                          uint32_t& nb_out, DevBuf<int2>& coords_out, DevBuf<float>& pdf_out, std::string& why) {
   const uint32_t n = w * h;
-  DevBuf<double> rad(n);
-  DevBuf<unsigned long long> keys(n);
-  DevBuf<uint32_t> vals(n);
-  k_env_radiance<<<(n + 255) / 256, 256, 0, s>>>(rgbe, n, rad.p, keys.p, vals.p);
-  return build_from_radiance(s, w, h, rad, keys, vals, bins_out, nb_out, coords_out, pdf_out, why);
+  TmpBuf<double> rad(sc, n);
+  TmpBuf<unsigned long long> keys(sc, n);
+  TmpBuf<uint32_t> vals(sc, n);
+  k_env_radiance<<<(n + 255) / 256, 256, 0, sc.s>>>(rgbe, n, rad.p, keys.p, vals.p);
+  return build_from_radiance(sc, w, h, rad, keys, vals, bins_out, nb_out, coords_out, pdf_out, why);
 }
 
 // PK_ENV_ALIAS's table for a w x h RGBE image on the device: per texel
@@ -308,7 +313,7 @@ int build_env_tables_gpu(cudaStream_t s, const uchar4* rgbe, uint32_t w, uint32_
 // and the normalisation are FP64; the weights are then fixed point (2^-frac
 // of the mean, frac = 61 - ceil(log2 n)), so the prefix sums of the sweep are
 // exact integers.
-int build_env_alias_gpu(cudaStream_t s, const uchar4* rgbe, uint32_t w, uint32_t h, DevBuf<uint2>& table_out,
+int build_env_alias_gpu(const Scratch& sc, const uchar4* rgbe, uint32_t w, uint32_t h, DevBuf<uint2>& table_out,
                         DevBuf<float>& pdf_out, std::string& why) {
   const uint32_t n = w * h;
   if (n == 0 || n > (1u << 29)) { why = "environment size out of range"; return 1; }
@@ -317,25 +322,28 @@ int build_env_alias_gpu(cudaStream_t s, const uchar4* rgbe, uint32_t w, uint32_t
   const int frac = 61 - lg;  // >= 32
   const unsigned long long one = 1ull << frac;
   const unsigned nblk = (n + ALIAS_PER_BLOCK - 1) / ALIAS_PER_BLOCK, grid = (n + 255) / 256;
-  DevBuf<double> partial(nblk), scale(1);
-  DevBuf<uint32_t> status(1), light(n), lrank(n), nl_dev(1), lidx(n), hidx(n);
-  DevBuf<unsigned long long> q(n), ldef(n + 1), hexc(n), esum(n), mass(n);
+  const cudaStream_t s = sc.s;
+  TmpBuf<double> partial(sc, nblk), scale(sc, 1);
+  TmpBuf<uint32_t> status(sc, 3), light(sc, n), lrank(sc, n), lidx(sc, n), hidx(sc, n);  // status, lights, errors
+  TmpBuf<unsigned long long> q(sc, n), ldef(sc, (size_t)n + 1), hexc(sc, n), esum(sc, n), mass(sc, n);
+  check(cudaMemsetAsync(status.p, 0, 12, s), "memset");
   k_alias_partial<<<nblk, ALIAS_THREADS, 0, s>>>(rgbe, n, partial.p);
   k_alias_total<<<1, 1024, 0, s>>>(partial.p, nblk, n, frac, scale.p, status.p);
   k_alias_weights<<<grid, 256, 0, s>>>(rgbe, n, scale.p, one, q.p, light.p);
   check(cudaGetLastError(), "alias weights");
-  scan_exclusive_u32(s, light.p, lrank.p, n, nl_dev.p);  // synchronises
-  uint32_t st = 0, nl = 0;
-  check(cudaMemcpyAsync(&st, status.p, 4, cudaMemcpyDeviceToHost, s), "D2H");
-  check(cudaMemcpyAsync(&nl, nl_dev.p, 4, cudaMemcpyDeviceToHost, s), "D2H");
+  scan_exclusive_u32(sc, light.p, lrank.p, n, status.p + 1, status.p + 2);
+  uint32_t st[3] = {0, 0, 0};
+  check(cudaMemcpyAsync(st, status.p, 12, cudaMemcpyDeviceToHost, s), "D2H");
   check(cudaStreamSynchronize(s), "sync");
-  if (st) { why = "black or non-finite environment"; return 1; }
+  const uint32_t nl = st[1];
+  if (st[2]) { why = "prefix sum look-back timed out"; return 1; }
+  if (st[0]) { why = "black or non-finite environment"; return 1; }
   const uint32_t nh = n - nl;
   check(cudaMemsetAsync(ldef.p + nl, 0, 8, s), "memset");  // D(nl) after the scan: all deficits
   k_alias_split<<<grid, 256, 0, s>>>(q.p, light.p, lrank.p, n, one, lidx.p, ldef.p, hidx.p, hexc.p);
   check(cudaGetLastError(), "alias split");
-  scan_exclusive_u64(s, ldef.p, ldef.p, (size_t)nl + 1);  // D(a), a = 0..nl
-  scan_exclusive_u64(s, hexc.p, esum.p, nh);  // E(b)
+  scan_exclusive_u64(sc, ldef.p, ldef.p, (size_t)nl + 1);  // D(a), a = 0..nl
+  scan_exclusive_u64(sc, hexc.p, esum.p, nh);  // E(b)
   table_out.alloc(n);
   pdf_out.alloc(n);
   if (nl) k_alias_lights<<<(nl + 255) / 256, 256, 0, s>>>(lidx.p, ldef.p, nl, hidx.p, esum.p, hexc.p, nh, q.p, one,
@@ -351,14 +359,14 @@ int build_env_alias_gpu(cudaStream_t s, const uchar4* rgbe, uint32_t w, uint32_t
 }
 
 // The same tables for an FP32 RGB map (w x h x 3 on the device).
-int build_env_tables_gpu_f32(cudaStream_t s, const float* rgb, uint32_t w, uint32_t h, DevBuf<int2>& bins_out,
+int build_env_tables_gpu_f32(const Scratch& sc, const float* rgb, uint32_t w, uint32_t h, DevBuf<int2>& bins_out,
                              uint32_t& nb_out, DevBuf<int2>& coords_out, DevBuf<float>& pdf_out, std::string& why) {
   const uint32_t n = w * h;
-  DevBuf<double> rad(n);
-  DevBuf<unsigned long long> keys(n);
-  DevBuf<uint32_t> vals(n);
-  k_env_radiance_f32<<<(n + 255) / 256, 256, 0, s>>>(rgb, n, rad.p, keys.p, vals.p);
-  return build_from_radiance(s, w, h, rad, keys, vals, bins_out, nb_out, coords_out, pdf_out, why);
+  TmpBuf<double> rad(sc, n);
+  TmpBuf<unsigned long long> keys(sc, n);
+  TmpBuf<uint32_t> vals(sc, n);
+  k_env_radiance_f32<<<(n + 255) / 256, 256, 0, sc.s>>>(rgb, n, rad.p, keys.p, vals.p);
+  return build_from_radiance(sc, w, h, rad, keys, vals, bins_out, nb_out, coords_out, pdf_out, why);
 }
 
 }  // namespace pk

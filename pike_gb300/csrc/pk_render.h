@@ -4,6 +4,7 @@
 #include <cstdint>
 
 #include "pk_internal.cuh"
+#include "pk_util.h"
 
 namespace pk {
 
@@ -70,7 +71,7 @@ void launch_math(cudaStream_t s, int fn, const float* x, const float* y, float* 
 // pk_scene.cu
 // Convert the reference 20-byte BFS nodes + leaf-ordered triangles + 16-byte
 // vertices into the traversal format (inner records, v0/e1/e2 triangles).
-int convert_bvh(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4, uint32_t n_tris,
+int convert_bvh(const Scratch& w, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4, uint32_t n_tris,
                 const float4* verts4, uint32_t n_verts, float4* inner, int4* inner32, float4* tris, int* root_code,
                 uint32_t* err);
 // Row S: per-vertex attribute quantisation (scene.js:456-470).

@@ -180,19 +180,20 @@ __global__ void k_tri_edges(const int4* __restrict__ tri4, uint32_t n, const flo
   tris[3 * (size_t)k + 2] = make_float4(e2z, 0.0f, 0.0f, 0.0f);
 }
 
-int convert_bvh(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4, uint32_t n_tris,
+int convert_bvh(const Scratch& w, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4, uint32_t n_tris,
                 const float4* verts4, uint32_t n_verts, float4* inner, int4* inner32, float4* tris, int* root_code,
                 uint32_t* err) {
-  DevBuf<uint32_t> flag(n_nodes), rank(n_nodes);
+  const cudaStream_t s = w.s;
+  TmpBuf<uint32_t> rank(w, n_nodes);
   // records in breadth-first order: the rank of an inner node among the inner
   // nodes in index order (a depth-first order was measured no faster: 3012-3015
   // against 3022-3032 Mrays/s at 1080p)
-  k_inner_flags<<<(n_nodes + 255) / 256, 256, 0, s>>>(nodes5, n_nodes, flag.p);
-  scan_exclusive_u32(s, flag.p, rank.p, n_nodes, nullptr);
+  k_inner_flags<<<(n_nodes + 255) / 256, 256, 0, s>>>(nodes5, n_nodes, rank.p);
+  scan_exclusive_u32(w, rank.p, rank.p, n_nodes, nullptr, err);
   k_inner_records<<<(n_nodes + 255) / 256, 256, 0, s>>>(nodes5, n_nodes, rank.p, n_tris, inner, root_code, err);
   k_inner_records32<<<(n_nodes + 255) / 256, 256, 0, s>>>(nodes5, n_nodes, rank.p, inner, inner32);
   if (n_tris) k_tri_edges<<<(n_tris + 255) / 256, 256, 0, s>>>(tri4, n_tris, verts4, n_verts, tris, err);
-  return cudaStreamSynchronize(s) == cudaSuccess ? 0 : 1;
+  return cudaGetLastError() == cudaSuccess ? 0 : 1;
 }
 
 }  // namespace pk

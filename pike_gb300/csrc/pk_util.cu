@@ -1,5 +1,6 @@
-// pk_util.cu -- device-wide exclusive scan (single pass, decoupled look-back)
-// and a stable LSD radix sort of 64-bit keys, used by the BVH and env builders.
+// pk_util.cu -- device-wide exclusive scan (single pass, decoupled look-back),
+// a stable LSD radix sort of 64-bit keys and the level lists of a binary tree,
+// used by the BVH and env builders.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -11,6 +12,18 @@
 #include "pk_util.h"
 
 namespace pk {
+
+cudaMemPool_t create_scratch_pool(int device) {
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  cudaMemPool_t pool = nullptr;
+  check(cudaMemPoolCreate(&pool, &props), "cudaMemPoolCreate");
+  uint64_t keep = SCRATCH_KEEP;
+  check(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
+  return pool;
+}
 
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
@@ -39,7 +52,10 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_u32(const uint32_t* in, u
     }
     uint32_t ea, eb, ta, tb;
     block_scan2<SCAN_THREADS / 32>(sum, 0u, ea, eb, ta, tb, s_warp);
-    if (threadIdx.x == 0) s_excl = lookback2(tiles, tile, pack2(ta, 0u), err);
+    if (threadIdx.x < 32) {
+      const unsigned long long e = lookback2_warp(tiles, tile, pack2(ta, 0u), err);
+      if (threadIdx.x == 0) s_excl = e;
+    }
     __syncthreads();
     uint32_t run = unpack_a(s_excl) + ea;
 #pragma unroll
@@ -52,26 +68,26 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_u32(const uint32_t* in, u
   }
 }
 
-void scan_exclusive_u32(cudaStream_t s, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* total) {
+static int multiprocessors() {
+  int dev = 0, sms = 1;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return sms;
+}
+
+void scan_exclusive_u32(const Scratch& w, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* total,
+                        uint32_t* err) {
   if (n == 0) {
-    if (total) check(cudaMemsetAsync(total, 0, 4, s), "memset");
+    if (total) check(cudaMemsetAsync(total, 0, 4, w.s), "memset");
     return;
   }
   const uint32_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-  DevBuf<unsigned long long> tiles(ntiles);
-  DevBuf<uint32_t> aux(2);  // ticket, err
-  check(cudaMemsetAsync(tiles.p, 0, tiles.bytes(), s), "memset");
-  check(cudaMemsetAsync(aux.p, 0, aux.bytes(), s), "memset");
-  int dev = 0, sms = 0;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  unsigned grid = (unsigned)std::min<uint32_t>(ntiles, (uint32_t)sms * 4u);
-  k_scan_u32<<<grid, SCAN_THREADS, 0, s>>>(in, out, n, total, tiles.p, aux.p, aux.p + 1);
+  TmpBuf<unsigned long long> state(w, (size_t)ntiles + 1);  // tile states, then the ticket
+  check(cudaMemsetAsync(state.p, 0, state.bytes(), w.s), "memset");
+  const unsigned grid = (unsigned)std::min<uint32_t>(ntiles, (uint32_t)multiprocessors() * 4u);
+  k_scan_u32<<<grid, SCAN_THREADS, 0, w.s>>>(in, out, n, total, state.p, reinterpret_cast<uint32_t*>(state.p + ntiles),
+                                             err);
   check(cudaGetLastError(), "k_scan_u32");
-  uint32_t err = 0;
-  check(cudaMemcpyAsync(&err, aux.p + 1, 4, cudaMemcpyDeviceToHost, s), "memcpy");
-  check(cudaStreamSynchronize(s), "scan sync");
-  if (err) throw CudaError("scan_exclusive_u32: look-back timed out");
 }
 
 // ---------------- exclusive scan of u64 values (three phases) ---------------
@@ -122,112 +138,245 @@ __global__ void k_scan_u64_add(unsigned long long* out, size_t n, const unsigned
   if (i < n) out[i] += tile_offs[i / SCAN_TILE];
 }
 
-void scan_exclusive_u64(cudaStream_t s, const unsigned long long* in, unsigned long long* out, size_t n) {
+void scan_exclusive_u64(const Scratch& w, const unsigned long long* in, unsigned long long* out, size_t n) {
   if (n == 0) return;
   const size_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-  DevBuf<unsigned long long> sums(ntiles);
-  k_scan_u64_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, s>>>(in, out, n, sums.p);
+  TmpBuf<unsigned long long> sums(w, ntiles);
+  k_scan_u64_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, w.s>>>(in, out, n, sums.p);
   check(cudaGetLastError(), "k_scan_u64_tiles");
   if (ntiles > 1) {
-    scan_exclusive_u64(s, sums.p, sums.p, ntiles);
-    k_scan_u64_add<<<(unsigned)((n + 255) / 256), 256, 0, s>>>(out, n, sums.p);
+    scan_exclusive_u64(w, sums.p, sums.p, ntiles);
+    k_scan_u64_add<<<(unsigned)((n + 255) / 256), 256, 0, w.s>>>(out, n, sums.p);
     check(cudaGetLastError(), "k_scan_u64_add");
   }
-  check(cudaStreamSynchronize(s), "scan sync");  // the tile sums are freed on return
 }
 
 // ---------------- stable LSD radix sort -------------------------------------
+// One kernel per 8-bit digit (after Adinets & Merrill, "Onesweep: A Faster
+// Least Significant Digit Radix Sort for GPUs", 2022): one pass over the keys
+// counts all eight digits; then each pass ranks a tile of keys in shared
+// memory, finds the tile's offset per digit by decoupled look-back (256
+// independent chains, one per thread) and writes the tile out in digit order,
+// so every key is read and written once per pass.  Bound by the 24 bytes per
+// pair and pass; several equal-length arrays sort in the same launches
+// (blockIdx.y).
 constexpr int SORT_THREADS = 256;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
-constexpr int SORT_ROUNDS = 16;                       // rounds of 32 keys per warp
-constexpr int SORT_TILE = SORT_THREADS * SORT_ROUNDS; // 4096 keys per block
+constexpr int SORT_ROUNDS = 12;                       // rounds of 32 keys per warp
+constexpr int SORT_TILE = SORT_THREADS * SORT_ROUNDS; // 3072 keys per block: 36 KB of pairs in shared memory
 constexpr int RADIX = 256;
+constexpr int SORT_PASSES = 8;
+static_assert(SORT_THREADS == RADIX, "one thread per digit");
 
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_hist(const uint64_t* __restrict__ keys, uint32_t n, int shift,
-                                                            uint32_t nblocks, uint32_t* __restrict__ hist) {
-  __shared__ uint32_t h[RADIX];
-  for (int i = threadIdx.x; i < RADIX; i += SORT_THREADS) h[i] = 0;
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_hist(const uint64_t* __restrict__ keys, uint32_t n,
+                                                            uint32_t* __restrict__ hist) {
+  __shared__ uint32_t h[SORT_PASSES][RADIX];
+  for (int i = threadIdx.x; i < SORT_PASSES * RADIX; i += SORT_THREADS) (&h[0][0])[i] = 0;
   __syncthreads();
-  const size_t base = (size_t)blockIdx.x * SORT_TILE;
-  for (int k = threadIdx.x; k < SORT_TILE; k += SORT_THREADS) {
-    const size_t i = base + k;
-    if (i < n) atomicAdd(&h[(uint32_t)(keys[i] >> shift) & 0xffu], 1u);
+  const uint64_t* in = keys + (size_t)blockIdx.y * n;
+  const int lane = threadIdx.x & 31;
+  const size_t stride = (size_t)gridDim.x * SORT_THREADS;
+  for (size_t base = (size_t)blockIdx.x * SORT_THREADS + (threadIdx.x - lane); base < n; base += stride) {
+    const size_t i = base + lane;
+    const bool on = i < n;
+    const uint64_t k = on ? in[i] : 0;
+    const uint32_t act = __ballot_sync(0xffffffffu, on);
+    if (on) {
+#pragma unroll
+      for (int p = 0; p < SORT_PASSES; p++) {
+        const uint32_t d = (uint32_t)(k >> (8 * p)) & 0xffu;
+        int same;  // digits that the whole warp shares (the high ones mostly) cost one atomic
+        __match_all_sync(act, d, &same);
+        if (!same) atomicAdd(&h[p][d], 1u);
+        else if (lane == __ffs(act) - 1) atomicAdd(&h[p][d], (uint32_t)__popc(act));
+      }
+    }
   }
   __syncthreads();
-  for (int d = threadIdx.x; d < RADIX; d += SORT_THREADS) hist[(size_t)d * nblocks + blockIdx.x] = h[d];
+  uint32_t* out = hist + (size_t)blockIdx.y * SORT_PASSES * RADIX;
+  for (int i = threadIdx.x; i < SORT_PASSES * RADIX; i += SORT_THREADS) {
+    const uint32_t c = (&h[0][0])[i];
+    if (c) atomicAdd(out + i, c);
+  }
 }
 
-__global__ void __launch_bounds__(SORT_THREADS) k_sort_scatter(const uint64_t* __restrict__ keys,
-                                                               const uint32_t* __restrict__ vals, uint32_t n, int shift,
-                                                               uint32_t nblocks, const uint32_t* __restrict__ offs,
-                                                               uint64_t* __restrict__ keys_out,
-                                                               uint32_t* __restrict__ vals_out) {
-  __shared__ uint32_t wh[SORT_WARPS][RADIX];
+// Look-back words: the top two bits say what the rest holds (1: this tile's
+// count, 2: the inclusive prefix).  32 bits for fewer than 2^30 keys, else 64.
+template <class W>
+struct SortWord;
+template <>
+struct SortWord<uint32_t> {
+  static constexpr uint32_t AGG = 1u << 30, PRE = 2u << 30, VAL = (1u << 30) - 1u;
+  static __device__ __forceinline__ uint32_t load(const uint32_t* p) {
+    uint32_t v;
+    asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(p) : "memory");
+    return v;
+  }
+  static __device__ __forceinline__ void store(uint32_t* p, uint32_t v) {
+    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(p), "r"(v) : "memory");
+  }
+};
+template <>
+struct SortWord<unsigned long long> {
+  static constexpr unsigned long long AGG = TILE_AGG, PRE = TILE_PRE, VAL = TILE_VAL;
+  static __device__ __forceinline__ unsigned long long load(const unsigned long long* p) { return ld_acquire(p); }
+  static __device__ __forceinline__ void store(unsigned long long* p, unsigned long long v) { st_release(p, v); }
+};
+
+// Exclusive prefix over the block's threads (one digit each).
+__device__ __forceinline__ uint32_t digit_scan(uint32_t v, uint32_t* s_warp) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  uint32_t inc = v;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const uint32_t x = __shfl_up_sync(0xffffffffu, inc, o);
+    if (lane >= o) inc += x;
+  }
+  if (lane == 31) s_warp[warp] = inc;
+  __syncthreads();
+  uint32_t before = 0;
+#pragma unroll
+  for (int k = 0; k < SORT_WARPS; k++)
+    if (k < warp) before += s_warp[k];
+  __syncthreads();
+  return before + inc - v;
+}
+
+template <class W>
+__global__ void __launch_bounds__(SORT_THREADS) k_sort_pass(const uint64_t* __restrict__ keys,
+                                                            const uint32_t* __restrict__ vals, uint32_t n, int pass,
+                                                            uint32_t ntiles, const uint32_t* __restrict__ hist,
+                                                            W* __restrict__ state, uint32_t* __restrict__ tickets,
+                                                            uint64_t* __restrict__ keys_out,
+                                                            uint32_t* __restrict__ vals_out, uint32_t* err) {
+  __shared__ uint64_t s_key[SORT_TILE];
+  __shared__ uint32_t s_val[SORT_TILE];
+  __shared__ uint32_t wh[SORT_WARPS][RADIX];
+  __shared__ uint32_t s_out[RADIX];  // where the tile's first key of a digit goes, less its place in the tile
+  __shared__ uint32_t s_warp[SORT_WARPS];
+  __shared__ uint32_t s_tile;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const uint32_t seg = blockIdx.y;
+  if (threadIdx.x == 0) s_tile = atomicAdd(tickets + seg, 1u);  // tiles in the order blocks start
   for (int i = threadIdx.x; i < SORT_WARPS * RADIX; i += SORT_THREADS) (&wh[0][0])[i] = 0;
   __syncthreads();
-  const size_t wbase = (size_t)blockIdx.x * SORT_TILE + (size_t)warp * (SORT_ROUNDS * 32);
+  const uint32_t tile = s_tile;
+  const int shift = 8 * pass;
+  const uint64_t* kin = keys + (size_t)seg * n;
+  const uint32_t* vin = vals + (size_t)seg * n;
+  const size_t wbase = (size_t)tile * SORT_TILE + (size_t)warp * (SORT_ROUNDS * 32);
   const uint32_t lt = (1u << lane) - 1u;
-  uint32_t rank[SORT_ROUNDS];
-  uint32_t dig[SORT_ROUNDS];
+  uint64_t key[SORT_ROUNDS];
+  uint32_t val[SORT_ROUNDS], rank[SORT_ROUNDS];
 #pragma unroll
   for (int r = 0; r < SORT_ROUNDS; r++) {
     const size_t i = wbase + (size_t)r * 32 + lane;
-    const uint32_t d = i < n ? ((uint32_t)(keys[i] >> shift) & 0xffu) : RADIX;
+    key[r] = i < n ? kin[i] : 0;
+    val[r] = i < n ? vin[i] : 0;
+  }
+#pragma unroll
+  for (int r = 0; r < SORT_ROUNDS; r++) {
+    const size_t i = wbase + (size_t)r * 32 + lane;
+    const uint32_t d = i < n ? (uint32_t)(key[r] >> shift) & 0xffu : RADIX;
     const uint32_t peers = __match_any_sync(0xffffffffu, d);
     uint32_t pre = 0;
     if (d < RADIX) pre = wh[warp][d];
     __syncwarp();
     rank[r] = pre + (uint32_t)__popc(peers & lt);
-    dig[r] = d;
     if (d < RADIX && (peers & lt) == 0) wh[warp][d] = pre + (uint32_t)__popc(peers);
     __syncwarp();
   }
   __syncthreads();
-  // per digit: exclusive prefix over warps (in place)
-  for (int d = threadIdx.x; d < RADIX; d += SORT_THREADS) {
-    uint32_t run = 0;
-    for (int w = 0; w < SORT_WARPS; w++) {
-      const uint32_t c = wh[w][d];
-      wh[w][d] = run;
-      run += c;
-    }
+  const int d = threadIdx.x;
+  uint32_t count = 0;
+  for (int k = 0; k < SORT_WARPS; k++) {  // exclusive prefix over warps, in place
+    const uint32_t c = wh[k][d];
+    wh[k][d] = count;
+    count += c;
   }
+  using L = SortWord<W>;
+  W* mine = state + ((size_t)seg * ntiles + tile) * RADIX + d;
+  L::store(mine, (tile == 0 ? L::PRE : L::AGG) | (W)count);
+  const uint32_t local = digit_scan(count, s_warp);
+  const uint32_t global = digit_scan(hist[((size_t)seg * SORT_PASSES + pass) * RADIX + d], s_warp);
+  for (int k = 0; k < SORT_WARPS; k++) wh[k][d] += local;
+  W before = 0;
+  if (tile) {
+    const W* p = mine;
+    for (uint32_t t = tile; t-- > 0;) {
+      p -= RADIX;
+      W v = L::load(p);
+      int spins = 0;
+      while ((v & ~L::VAL) == 0) {
+        if (++spins > LOOKBACK_SPIN_LIMIT) {
+          atomicOr(err, ERR_LOOKBACK);
+          v = L::PRE;
+          break;
+        }
+        __nanosleep(32);
+        v = L::load(p);
+      }
+      before += v & L::VAL;
+      if ((v & ~L::VAL) == L::PRE) break;
+    }
+    L::store(mine, L::PRE | (before + (W)count));
+  }
+  s_out[d] = global + (uint32_t)before - local;
   __syncthreads();
 #pragma unroll
   for (int r = 0; r < SORT_ROUNDS; r++) {
     const size_t i = wbase + (size_t)r * 32 + lane;
     if (i >= n) continue;
-    const uint32_t d = dig[r];
-    const uint32_t pos = offs[(size_t)d * nblocks + blockIdx.x] + wh[warp][d] + rank[r];
-    keys_out[pos] = keys[i];
-    vals_out[pos] = vals[i];
+    const uint32_t pos = wh[warp][(uint32_t)(key[r] >> shift) & 0xffu] + rank[r];
+    s_key[pos] = key[r];
+    s_val[pos] = val[r];
+  }
+  __syncthreads();
+  const size_t first = (size_t)tile * SORT_TILE;
+  const uint32_t here = (uint32_t)(n - first < (size_t)SORT_TILE ? n - first : (size_t)SORT_TILE);
+  for (uint32_t i = threadIdx.x; i < here; i += SORT_THREADS) {
+    const uint64_t k = s_key[i];
+    const uint32_t to = s_out[(uint32_t)(k >> shift) & 0xffu] + i;
+    if (to < n) {  // always, unless a look-back gave up
+      keys_out[(size_t)seg * n + to] = k;
+      vals_out[(size_t)seg * n + to] = s_val[i];
+    }
   }
 }
 
-void radix_sort_pairs_u64(cudaStream_t s, uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* vals_tmp,
-                          uint32_t n, int bits) {
-  if (n <= 1) return;
-  const uint32_t nblocks = (n + SORT_TILE - 1) / SORT_TILE;
-  DevBuf<uint32_t> hist((size_t)RADIX * nblocks);
+void radix_sort_pairs_u64(const Scratch& w, uint64_t* keys, uint32_t* vals, uint64_t* keys_tmp, uint32_t* vals_tmp,
+                          uint32_t n, uint32_t segs, uint32_t* err) {
+  if (n <= 1 || segs == 0) return;
+  const uint32_t ntiles = (n + SORT_TILE - 1) / SORT_TILE;
+  const bool wide = n >= (1u << 30);
+  const size_t words = (size_t)segs * ntiles * RADIX;  // look-back words of one pass
+  const size_t head = (size_t)segs * SORT_PASSES * (RADIX + 1) * 4;
+  const size_t head8 = (head + 7) / 8;
+  TmpBuf<unsigned long long> space(w, head8 + (words * SORT_PASSES * (wide ? 8 : 4) + 7) / 8);
+  check(cudaMemsetAsync(space.p, 0, space.bytes(), w.s), "memset");
+  uint32_t* hist = reinterpret_cast<uint32_t*>(space.p);
+  uint32_t* tickets = hist + (size_t)segs * SORT_PASSES * RADIX;  // [pass][seg]
+  const unsigned hgrid = (unsigned)std::min<uint32_t>((n + 4 * SORT_THREADS - 1) / (4 * SORT_THREADS),
+                                                      (uint32_t)multiprocessors() * 4u);
+  k_sort_hist<<<dim3(hgrid, segs), SORT_THREADS, 0, w.s>>>(keys, n, hist);
   uint64_t* kin = keys;
   uint32_t* vin = vals;
   uint64_t* kout = keys_tmp;
   uint32_t* vout = vals_tmp;
-  const int passes = (bits + 7) / 8;
-  for (int p = 0; p < passes; p++) {
-    const int shift = 8 * p;
-    k_sort_hist<<<nblocks, SORT_THREADS, 0, s>>>(kin, n, shift, nblocks, hist.p);
-    scan_exclusive_u32(s, hist.p, hist.p, (uint32_t)hist.n, nullptr);
-    k_sort_scatter<<<nblocks, SORT_THREADS, 0, s>>>(kin, vin, n, shift, nblocks, hist.p, kout, vout);
-    check(cudaGetLastError(), "radix sort");
+  const dim3 grid(ntiles, segs);
+  for (int p = 0; p < SORT_PASSES; p++) {  // an even number of passes: the result ends in keys, vals
+    if (wide)
+      k_sort_pass<unsigned long long><<<grid, SORT_THREADS, 0, w.s>>>(kin, vin, n, p, ntiles, hist,
+                                                                      space.p + head8 + p * words,
+                                                                      tickets + p * segs, kout, vout, err);
+    else
+      k_sort_pass<uint32_t><<<grid, SORT_THREADS, 0, w.s>>>(kin, vin, n, p, ntiles, hist,
+                                                            reinterpret_cast<uint32_t*>(space.p + head8) + p * words,
+                                                            tickets + p * segs, kout, vout, err);
     std::swap(kin, kout);
     std::swap(vin, vout);
   }
-  if (kin != keys) {
-    check(cudaMemcpyAsync(keys, kin, (size_t)n * 8, cudaMemcpyDeviceToDevice, s), "memcpy");
-    check(cudaMemcpyAsync(vals, vin, (size_t)n * 4, cudaMemcpyDeviceToDevice, s), "memcpy");
-  }
+  check(cudaGetLastError(), "radix sort");
 }
 
 // ---- levels of a binary tree ------------------------------------------------
@@ -255,12 +404,13 @@ __global__ void k_level_children(const int32_t* __restrict__ nodes5, uint32_t* _
   order[e + 2 * rank[k] + 1] = (uint32_t)l + 1;
 }
 
-int tree_levels(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, DevBuf<uint32_t>& order,
+int tree_levels(const Scratch& w, const int32_t* nodes5, uint32_t n_nodes, TmpBuf<uint32_t>& order,
                 std::vector<uint32_t>& level) {
+  const cudaStream_t s = w.s;
   order.alloc(std::max<uint32_t>(n_nodes, 1u));
   check(cudaMemsetAsync(order.p, 0, 4, s), "memset");  // the root
-  DevBuf<uint32_t> flag(std::max<uint32_t>(n_nodes, 1u)), tot(1), err(1);
-  check(cudaMemsetAsync(err.p, 0, 4, s), "memset");
+  TmpBuf<uint32_t> flag(w, std::max<uint32_t>(n_nodes, 1u)), tot(w, 2);  // tot: inner nodes of the level, errors
+  check(cudaMemsetAsync(tot.p, 0, 8, s), "memset");
   level.assign(1, 0u);
   uint32_t b = 0, e = n_nodes ? 1u : 0u;
   uint32_t c = 0;
@@ -268,17 +418,17 @@ int tree_levels(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, DevBuf<
     level.push_back(e);
     const unsigned blocks = (e - b + 127) / 128;
     k_level_flags<<<blocks, 128, 0, s>>>(nodes5, order.p, b, e, flag.p);
-    scan_exclusive_u32(s, flag.p, flag.p, e - b, tot.p);
+    scan_exclusive_u32(w, flag.p, flag.p, e - b, tot.p, tot.p + 1);
     check(cudaMemcpyAsync(&c, tot.p, 4, cudaMemcpyDeviceToHost, s), "D2H");
     check(cudaStreamSynchronize(s), "sync");
     const uint64_t next_end = (uint64_t)e + 2ull * c;
     if (next_end > n_nodes) return 1;
-    k_level_children<<<blocks, 128, 0, s>>>(nodes5, order.p, b, e, flag.p, n_nodes, err.p);
+    k_level_children<<<blocks, 128, 0, s>>>(nodes5, order.p, b, e, flag.p, n_nodes, tot.p + 1);
     b = e;
     e = (uint32_t)next_end;
   }
   uint32_t herr = 0;
-  check(cudaMemcpyAsync(&herr, err.p, 4, cudaMemcpyDeviceToHost, s), "D2H");
+  check(cudaMemcpyAsync(&herr, tot.p + 1, 4, cudaMemcpyDeviceToHost, s), "D2H");
   check(cudaStreamSynchronize(s), "sync");
   return (e != n_nodes || herr) ? 1 : 0;
 }

@@ -543,17 +543,19 @@ const char* error_text(uint32_t e) {
 // boxes and records, widened node boxes.
 struct Prepared {
   std::vector<uint32_t> level;  // level d = order[level[d], level[d + 1])
-  DevBuf<uint32_t> order;
-  DevBuf<BoxD> tbox, nbox;
-  DevBuf<float> brecs;
+  TmpBuf<uint32_t> order;
+  TmpBuf<BoxD> tbox, nbox;
+  TmpBuf<float> brecs;
+  explicit Prepared(const Scratch& w) : order(w), tbox(w), nbox(w), brecs(w) {}
 };
-int prepare(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4, uint32_t n_tris,
-            const float4* verts4, uint32_t n_verts, DevBuf<uint32_t>& err, Prepared& P, std::string& why) {
+int prepare(const Scratch& w, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4, uint32_t n_tris,
+            const float4* verts4, uint32_t n_verts, TmpBuf<uint32_t>& err, Prepared& P, std::string& why) {
+  const cudaStream_t s = w.s;
   P.tbox.alloc(std::max<uint32_t>(n_tris, 1u));
   P.brecs.alloc((size_t)WIDE_TRI_FLOATS * std::max<uint32_t>(n_tris, 1u));
   P.nbox.alloc(n_nodes);
   if (n_tris) k_tri_data<<<blocks(n_tris), 128, 0, s>>>(tri4, n_tris, verts4, n_verts, P.tbox.p, P.brecs.p, err.p);
-  if (tree_levels(s, nodes5, n_nodes, P.order, P.level)) { why = error_text(E_ORDER); return 1; }
+  if (tree_levels(w, nodes5, n_nodes, P.order, P.level)) { why = error_text(E_ORDER); return 1; }
   if (uint32_t ev = read_u32(s, err.p)) { why = error_text(ev); return 1; }
   for (size_t d = P.level.size() - 1; d-- > 0;)
     k_node_boxes<<<blocks(P.level[d + 1] - P.level[d]), 128, 0, s>>>(nodes5, P.order.p, P.level[d], P.level[d + 1],
@@ -566,17 +568,18 @@ int prepare(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, const int4*
 
 }  // namespace
 
-int build_wide_bvh_gpu(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4, uint32_t n_tris,
+int build_wide_bvh_gpu(const Scratch& w, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4, uint32_t n_tris,
                        const float4* verts4, uint32_t n_verts, DevBuf<float4>& nodes_out, DevBuf<float4>& tris_out,
                        uint32_t& n_wide, uint32_t& depth, std::string& why) {
   if (n_nodes == 0) { why = "empty BVH"; return 1; }
-  DevBuf<uint32_t> err(1);
+  const cudaStream_t s = w.s;
+  TmpBuf<uint32_t> err(w, 1);
   check(cudaMemsetAsync(err.p, 0, 4, s), "memset");
-  Prepared P;
-  if (prepare(s, nodes5, n_nodes, tri4, n_tris, verts4, n_verts, err, P, why)) return 1;
-  DevBuf<float> cost(8 * (size_t)n_nodes);
-  DevBuf<uint8_t> opt(8 * (size_t)n_nodes), split(n_nodes);
-  DevBuf<uint32_t> ntri(n_nodes);
+  Prepared P(w);
+  if (prepare(w, nodes5, n_nodes, tri4, n_tris, verts4, n_verts, err, P, why)) return 1;
+  TmpBuf<float> cost(w, 8 * (size_t)n_nodes);
+  TmpBuf<uint8_t> opt(w, 8 * (size_t)n_nodes), split(w, n_nodes);
+  TmpBuf<uint32_t> ntri(w, n_nodes);
   for (size_t d = P.level.size() - 1; d-- > 0;)
     k_collapse<<<blocks(P.level[d + 1] - P.level[d]), 128, 0, s>>>(nodes5, P.order.p, P.level[d], P.level[d + 1],
                                                                     P.nbox.p, cost.p, opt.p, split.p, ntri.p);
@@ -584,9 +587,9 @@ int build_wide_bvh_gpu(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, 
   const BuildView V{nodes5, P.tbox.p, P.nbox.p, opt.p, split.p, ntri.p};
   // top down; node capacity grows geometrically
   size_t cap = std::max<size_t>(1024, n_nodes / 4);
-  DevBuf<float> W((size_t)WIDE_NODE_FLOATS * cap);
-  DevBuf<float> T((size_t)WIDE_TRI_FLOATS * std::max<uint32_t>(n_tris, 1u));
-  DevBuf<Item> items(1), next;
+  TmpBuf<float> W(w, (size_t)WIDE_NODE_FLOATS * cap);
+  TmpBuf<float> T(w, (size_t)WIDE_TRI_FLOATS * std::max<uint32_t>(n_tris, 1u));
+  TmpBuf<Item> items(w, 1), next(w);
   Item root;  // item_of(0)
   {
     int32_t nd1 = 0;
@@ -597,24 +600,24 @@ int build_wide_bvh_gpu(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, 
   check(cudaMemcpyAsync(items.p, &root, sizeof(Item), cudaMemcpyHostToDevice, s), "H2D");
   uint32_t n = 1, node_base = 0, tri_base = 0;
   depth = 0;
-  DevBuf<uint32_t> n_inner, n_tri, tot(2);
+  TmpBuf<uint32_t> n_inner(w), n_tri(w), tot(w, 2);
   while (n) {
     depth++;
     n_inner.alloc(n);
     n_tri.alloc(n);
     k_wide_count<<<blocks(n), 128, 0, s>>>(V, items.p, n, n_inner.p, n_tri.p);
     check(cudaGetLastError(), "k_wide_count");
-    scan_exclusive_u32(s, n_inner.p, n_inner.p, n, tot.p);
-    scan_exclusive_u32(s, n_tri.p, n_tri.p, n, tot.p + 1);
+    scan_exclusive_u32(w, n_inner.p, n_inner.p, n, tot.p, err.p);
+    scan_exclusive_u32(w, n_tri.p, n_tri.p, n, tot.p + 1, err.p);
     uint32_t th[2];
     check(cudaMemcpyAsync(th, tot.p, 8, cudaMemcpyDeviceToHost, s), "D2H");
     check(cudaStreamSynchronize(s), "sync");
     if ((uint64_t)tri_base + th[1] > n_tris) { why = "internal: triangle count mismatch"; return 1; }
     if ((size_t)node_base + n > cap) {
       const size_t ncap = std::max((size_t)node_base + n, 2 * cap);
-      DevBuf<float> W2((size_t)WIDE_NODE_FLOATS * ncap);
+      TmpBuf<float> W2(w, (size_t)WIDE_NODE_FLOATS * ncap);
       check(cudaMemcpyAsync(W2.p, W.p, (size_t)WIDE_NODE_FLOATS * 4 * node_base, cudaMemcpyDeviceToDevice, s), "D2D");
-      W = std::move(W2);
+      W.swap(W2);
       cap = ncap;
     }
     next.alloc(std::max<uint32_t>(th[0], 1u));
@@ -624,7 +627,7 @@ int build_wide_bvh_gpu(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, 
     node_base += n;
     tri_base += th[1];
     n = th[0];
-    std::swap(items, next);
+    items.swap(next);
   }
   if (uint32_t ev = read_u32(s, err.p)) { why = error_text(ev); return 1; }
   if (tri_base != n_tris) { why = "internal: triangle count mismatch"; return 1; }
@@ -640,21 +643,22 @@ int build_wide_bvh_gpu(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, 
   return 0;
 }
 
-int build_exact_binary_gpu(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4,
+int build_exact_binary_gpu(const Scratch& w, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4,
                            uint32_t n_tris, const float4* verts4, uint32_t n_verts, DevBuf<float4>& records,
                            DevBuf<float4>& tris, int32_t& root_code, std::string& why) {
   if (n_nodes == 0) { why = "empty BVH"; return 1; }
-  DevBuf<uint32_t> err(1);
+  const cudaStream_t s = w.s;
+  TmpBuf<uint32_t> err(w, 1);
   check(cudaMemsetAsync(err.p, 0, 4, s), "memset");
-  Prepared P;
-  if (prepare(s, nodes5, n_nodes, tri4, n_tris, verts4, n_verts, err, P, why)) return 1;
-  DevBuf<uint32_t> rank(n_nodes), tot(1);
+  Prepared P(w);
+  if (prepare(w, nodes5, n_nodes, tri4, n_tris, verts4, n_verts, err, P, why)) return 1;
+  TmpBuf<uint32_t> rank(w, n_nodes), tot(w, 1);
   k_inner_flags<<<blocks(n_nodes), 128, 0, s>>>(nodes5, n_nodes, rank.p);
-  scan_exclusive_u32(s, rank.p, rank.p, n_nodes, tot.p);
+  scan_exclusive_u32(w, rank.p, rank.p, n_nodes, tot.p, err.p);
   const uint32_t n_inner = read_u32(s, tot.p);
   records.alloc(4 * (size_t)std::max<uint32_t>(n_inner, 1u));
   check(cudaMemsetAsync(records.p, 0, records.bytes(), s), "memset");
-  DevBuf<int32_t> rc(1);
+  TmpBuf<int32_t> rc(w, 1);
   k_exact_records<<<blocks(n_nodes), 128, 0, s>>>(nodes5, n_nodes, rank.p, P.nbox.p,
                                                   reinterpret_cast<float*>(records.p), rc.p);
   check(cudaGetLastError(), "k_exact_records");

@@ -46,7 +46,7 @@ constexpr int WIDE_TRI_FLOATS = 12;
 // The compressed 8-wide BVH: nodes_out (5 float4 per node), tris_out (3
 // float4 per triangle, in the wide BVH's own leaf order), the node count and
 // the depth in wide levels.
-int build_wide_bvh_gpu(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4, uint32_t n_tris,
+int build_wide_bvh_gpu(const Scratch& w, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4, uint32_t n_tris,
                        const float4* verts4, uint32_t n_verts, DevBuf<float4>& nodes_out, DevBuf<float4>& tris_out,
                        uint32_t& n_wide, uint32_t& depth, std::string& why);
 
@@ -56,7 +56,7 @@ int build_wide_bvh_gpu(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, 
 // the reference's inward-truncated snorm16 boxes, and the binary leaf order's
 // triangle records in the format above.  Traversed with (t, slot) ties and
 // slack in the box tests, closest hits equal brute force.
-int build_exact_binary_gpu(cudaStream_t s, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4,
+int build_exact_binary_gpu(const Scratch& w, const int32_t* nodes5, uint32_t n_nodes, const int4* tri4,
                            uint32_t n_tris, const float4* verts4, uint32_t n_verts, DevBuf<float4>& records,
                            DevBuf<float4>& tris, int32_t& root_code, std::string& why);
 
