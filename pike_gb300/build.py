@@ -16,8 +16,8 @@ CSRC = os.path.join(HERE, "csrc")
 OUT = os.path.join(HERE, "libpike.so")
 BUILD_DIR = os.path.join(HERE, "_build")
 
-SOURCES = ["pk_api.cu", "pk_render.cu", "pk_scene.cu", "pk_util.cu", "pk_bvh.cu", "pk_cast.cu", "pk_env.cu", "pk_diff.cu", "pk_batch.cu", "pk_probe.cu", "pk_wide.cu", "pk_host_tables.cpp"]
-HEADERS = ["pk_internal.cuh", "pk_math.cuh", "pk_render.h", "pk_util.h", "pk_bvh.h", "pk_host_tables.h", "pk_ctx.h",
+SOURCES = ["pk_api.cu", "pk_render.cu", "pk_scene.cu", "pk_util.cu", "pk_bvh.cu", "pk_bvh_sweep.cu", "pk_cast.cu", "pk_env.cu", "pk_diff.cu", "pk_batch.cu", "pk_probe.cu", "pk_wide.cu", "pk_host_tables.cpp"]
+HEADERS = ["pk_internal.cuh", "pk_math.cuh", "pk_render.h", "pk_util.h", "pk_bvh.h", "pk_bvh_pack.cuh", "pk_host_tables.h", "pk_ctx.h",
            "pk_traverse.cuh", "pk_traverse_wide.cuh", "pk_wide.h", "pk_shade.cuh"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 NVFLAGS = ["-O3", "-std=c++17", "-lineinfo", "-fmad=false", "-prec-div=true", "-prec-sqrt=true", "-ftz=false",
