@@ -234,7 +234,7 @@ int pk_configure(pk_ctx* c, uint32_t width, uint32_t height, uint32_t batch) {
     }
     c->ct = compact_tiles(c->cap);
     c->st = shade_tiles(c->cap);
-    kernel_grids(c->sms, c->cap, &c->g_trace, &c->g_compact, &c->g_shade, &c->g_trace_wide);
+    c->grids = kernel_grids(c->sms, c->cap);
     for (int i = 0; i < 3; i++) c->mq[i].alloc(2 * (size_t)c->cap);
     alloc_slot(c, 0);
     for (int k = 1; k < MAX_IN_FLIGHT; k++) release_slot(c->slot[k]);  // sized again on first use

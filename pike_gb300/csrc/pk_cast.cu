@@ -112,7 +112,7 @@ int cast_enqueue(pk_ctx* c, const float4* o4, const float4* d4, uint32_t n, int 
   LaunchCtx L = c->launch();
   L.scene = c->dropin_scene();  // the drop-in's records whatever the trace mode
   const unsigned warps = (unsigned)((n + 31) / 32);
-  const unsigned grid = std::max(1u, std::min(L.trace_blocks, (warps + CAST_THREADS / 32 - 1) / (CAST_THREADS / 32)));
+  const unsigned grid = std::max(1u, std::min(L.grids.trace.full, (warps + CAST_THREADS / 32 - 1) / (CAST_THREADS / 32)));
   if (n) {
     if (any_hit)
       k_cast<true><<<grid, CAST_THREADS, 0, stream>>>(L.scene, o4, d4, n, hits4, s.flags, s.tickets, s.tickets + 2);

@@ -85,7 +85,7 @@ struct pk_ctx {
   // configuration
   uint32_t W = 0, H = 0, B = 0, cap = 0, npix = 0;
   uint32_t ct = 0, st = 0;  // look-back tiles per compaction / shade launch
-  unsigned g_trace = 1, g_compact = 1, g_shade = 1, g_trace_wide = 1;  // persistent grid sizes
+  pk::Grids grids;          // persistent grid sizes
   int trace_mode = pk::TRACE_PERSISTENT;
   unsigned long long state_version = 1;
   pk::FrameSlot slot[pk::MAX_IN_FLIGHT];
@@ -201,12 +201,9 @@ struct pk_ctx {
     L.npix = npix;
     L.capacity = cap;
     L.miss_capacity = 2 * cap;
-    L.trace_blocks = g_trace;
-    L.trace_blocks_wide = g_trace_wide;
+    L.grids = grids;
     L.accum_sum = kahan ? accum_sum.p : nullptr;
     L.accum_comp = kahan ? accum_comp.p : nullptr;
-    L.compact_blocks = g_compact;
-    L.shade_blocks = g_shade;
     L.trace_mode = trace_mode;
     return L;
   }

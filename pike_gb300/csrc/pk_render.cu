@@ -120,7 +120,8 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_trace(SceneDev sc, EnvDev env
 // inner-node loop and a leaf loop (while-while).  There is no speculation: a
 // leaf is intersected as soon as the ray reaches it, so each ray visits the
 // same nodes in the same order as trace.wgsl's loop and gets the same hit.
-// Hit bits are set with atomicOr in a flag array zeroed before the launch.
+// Hit bits are set with atomicOr in a flag array that the compaction before
+// left zero.
 #ifndef PK_REFILL_MIN
 #define PK_REFILL_MIN 16
 #endif
@@ -541,31 +542,41 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_CW_MINBLOCKS) k_trace_cw(Sce
 //   MODE 0: closest-hit flags -> hit list (+ miss queue when MISSQ; + the
 //           contributions of misses parked in miss_rec when given)
 //   MODE 1: any-hit flags     -> unoccluded shadow rays appended to the miss queue
+// A tile is 32 R flag words: one warp scans their counts and takes the tile's
+// prefix (lookback2_warp), then every lane moves the rays of its bit position,
+// COMPACT_PER words per warp at once, so all copies are coalesced and
+// independent.  (One thread per flag word, walking its 32 bits one after the
+// other, cost 35-39 us a launch on a 256x256 frame, where eight tiles were all
+// there were: latency of up to 32 dependent copies.)  The flags are left zero
+// for the next traversal, which sets bits in them.
+// R: small queues take 1024 rays per tile, to spread over the SMs; large ones
+// COMPACT_R_LARGE times as many, fewer look-back steps and blocks beside the
+// other frames' kernels (1080p, eight frames in flight: see compact_r).
 // =====================================================================
-// (1080p: 256 threads 3734-3748 Mrays/s, 512: 3738-3760, 1024: 3698-3711)
-#ifndef PK_COMPACT_THREADS
-#define PK_COMPACT_THREADS 256
+constexpr int COMPACT_THREADS = 256;
+constexpr int COMPACT_WARPS = COMPACT_THREADS / 32;
+constexpr int COMPACT_WORDS = 32;  // flag words per round
+constexpr int COMPACT_PER = COMPACT_WORDS / COMPACT_WARPS;
+#ifndef PK_COMPACT_R
+#define PK_COMPACT_R 4
 #endif
-constexpr int COMPACT_THREADS = PK_COMPACT_THREADS;
-// The compaction and shade kernels take their tile's prefix with a whole warp
-// (lookback2_warp) rather than one thread (lookback2): 3137-3140 against
-// 3020-3026 Mrays/s at 1080p when it was introduced.
+constexpr int COMPACT_R_LARGE = PK_COMPACT_R;
 
-template <int MODE, bool MISSQ>
-__global__ void __launch_bounds__(COMPACT_THREADS) k_compact(Counters* __restrict__ ctr,
-                                                              const uint32_t* __restrict__ flags,
+template <int MODE, bool MISSQ, int R>
+__global__ void __launch_bounds__(COMPACT_THREADS) k_compact(Counters* __restrict__ ctr, uint32_t* __restrict__ flags,
                                                               uint32_t* __restrict__ hit_list, RayQ src, RayQ M,
                                                               uint32_t miss_capacity, uint32_t* __restrict__ ticket,
                                                               unsigned long long* __restrict__ tiles,
                                                               const uint4* __restrict__ miss_rec,
                                                               float4* __restrict__ color, uint32_t npix) {
   __shared__ uint32_t s_tile;
-  __shared__ uint32_t s_warp[COMPACT_THREADS / 32 + 1][2];
-  __shared__ unsigned long long s_excl;
+  __shared__ uint32_t s_hit[R * COMPACT_WORDS], s_miss[R * COMPACT_WORDS];  // bits of each word
+  __shared__ uint32_t s_a[R * COMPACT_WORDS], s_b[R * COMPACT_WORDS];       // outputs before it
   const uint32_t n = MODE == 0 ? ctr->num_rays : ctr->num_shadow;
   const uint32_t miss_base = MODE == 0 ? 0u : ctr->num_misses;
   const uint32_t nwords = (n + 31) >> 5;
-  const uint32_t ntiles = (nwords + COMPACT_THREADS - 1) / COMPACT_THREADS;
+  const uint32_t ntiles = (nwords + R * COMPACT_WORDS - 1) / (R * COMPACT_WORDS);
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, ltmask = (1u << lane) - 1u;
   if (ntiles == 0) {
     if (blockIdx.x == 0 && threadIdx.x == 0) {
       if (MODE == 0) { ctr->num_hits = 0; if (MISSQ) ctr->num_misses = 0; }
@@ -577,71 +588,97 @@ __global__ void __launch_bounds__(COMPACT_THREADS) k_compact(Counters* __restric
     __syncthreads();
     const uint32_t tile = s_tile;
     if (tile >= ntiles) break;
-    const uint32_t w = tile * COMPACT_THREADS + threadIdx.x;
-    uint32_t valid = 0u, hm = 0u;
-    if (w < nwords) {
-      valid = (w == nwords - 1 && (n & 31u)) ? ((1u << (n & 31u)) - 1u) : 0xffffffffu;
-      hm = flags[w] & valid;
-    }
-    const uint32_t mm = valid & ~hm;
-    // MODE 0 counts hits (a) and misses (b); MODE 1 counts unoccluded rays (b).
-    const uint32_t ca = MODE == 0 ? (uint32_t)__popc(hm) : 0u;
-    const uint32_t cb = (MODE == 1 || MISSQ) ? (uint32_t)__popc(mm) : 0u;
-    uint32_t ea, eb, ta, tb;
-    block_scan2<COMPACT_THREADS / 32>(ca, cb, ea, eb, ta, tb, s_warp);
-    if (threadIdx.x < 32) {
-      const unsigned long long e = lookback2_warp(tiles, tile, pack2(ta, tb), &ctr->err);
-      if (threadIdx.x == 0) s_excl = e;
+    const uint32_t w0 = tile * (R * COMPACT_WORDS);
+    if (warp == 0) {
+      uint32_t hm[R], mm[R], run = 0;  // run: hits and misses of the rounds so far, 16 bits each
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const uint32_t w = w0 + r * COMPACT_WORDS + lane;
+        hm[r] = mm[r] = 0u;
+        if (w < nwords) {
+          const uint32_t valid = (w == nwords - 1 && (n & 31u)) ? ((1u << (n & 31u)) - 1u) : 0xffffffffu;
+          hm[r] = flags[w] & valid;
+          mm[r] = valid & ~hm[r];
+        }
+      }
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        const uint32_t w = w0 + r * COMPACT_WORDS + lane;
+        if (w < nwords) flags[w] = 0u;
+        // MODE 0 counts hits (a) and misses (b); MODE 1 counts unoccluded rays (b).
+        const uint32_t c = (MODE == 0 ? (uint32_t)__popc(hm[r]) : 0u) |
+                           ((MODE == 1 || MISSQ) ? (uint32_t)__popc(mm[r]) << 16 : 0u);
+        uint32_t sum = c;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const uint32_t x = __shfl_up_sync(0xffffffffu, sum, o);
+          if (lane >= (uint32_t)o) sum += x;
+        }
+        s_hit[r * COMPACT_WORDS + lane] = hm[r];
+        s_miss[r * COMPACT_WORDS + lane] = mm[r];
+        const uint32_t before = run + sum - c;
+        s_a[r * COMPACT_WORDS + lane] = before & 0xffffu;
+        s_b[r * COMPACT_WORDS + lane] = before >> 16;
+        run += __shfl_sync(0xffffffffu, sum, 31);
+      }
+      const unsigned long long e = lookback2_warp(tiles, tile, pack2(run & 0xffffu, run >> 16), &ctr->err);
+      const uint32_t ea = unpack_a(e), eb = miss_base + unpack_b(e);
+#pragma unroll
+      for (int r = 0; r < R; r++) {
+        s_a[r * COMPACT_WORDS + lane] += ea;
+        s_b[r * COMPACT_WORDS + lane] += eb;
+      }
+      if (tile == ntiles - 1 && lane == 0) {
+        if (MODE == 0) {
+          ctr->num_hits = ea + (run & 0xffffu);
+          if (MISSQ) ctr->num_misses = eb + (run >> 16);
+        } else {
+          ctr->num_misses = eb + (run >> 16);
+        }
+      }
     }
     __syncthreads();
-    const uint32_t pa = unpack_a(s_excl) + ea;
-    uint32_t pb = unpack_b(s_excl) + eb;
-    if (MODE == 0) {
-      uint32_t bits = hm, k = pa;
-      while (bits) {
-        const int b = __ffs(bits) - 1;
-        bits &= bits - 1u;
-        hit_list[k++] = w * 32u + (uint32_t)b;
-      }
-    }
-    if (MODE == 0 && !MISSQ && miss_rec) {  // misses parked by a deferring closest-hit trace
-      uint32_t bits = mm;
-      while (bits) {
-        const int b = __ffs(bits) - 1;
-        bits &= bits - 1u;
-        const uint4 m = miss_rec[w * 32u + (uint32_t)b];
-        add_color(color, npix, m.w, __uint_as_float(m.x), __uint_as_float(m.y), __uint_as_float(m.z), 1.0f,
-                  &ctr->err);
-      }
-    }
-    if (MODE == 1 || MISSQ) {
-      uint32_t bits = mm, k = miss_base + pb;
-      while (bits) {
-        const int b = __ffs(bits) - 1;
-        bits &= bits - 1u;
-        const uint32_t j = w * 32u + (uint32_t)b;
-        if (k < miss_capacity) {
-          M.o[k] = src.o[j];
-          M.d[k] = src.d[j];
-          M.t[k] = src.t[j];
-        } else {
-          atomicOr(&ctr->err, ERR_QUEUE);
-        }
-        ++k;
-      }
-    }
-    if (tile == ntiles - 1 && threadIdx.x == 0) {
-      const uint32_t tot_a = unpack_a(s_excl) + ta, tot_b = unpack_b(s_excl) + tb;
+#pragma unroll 1
+    for (int r = 0; r < R; r++) {
+      const uint32_t k0 = r * COMPACT_WORDS + warp * COMPACT_PER;
       if (MODE == 0) {
-        ctr->num_hits = tot_a;
-        if (MISSQ) ctr->num_misses = tot_b;
-      } else {
-        ctr->num_misses = miss_base + tot_b;
+#pragma unroll
+        for (int q = 0; q < COMPACT_PER; q++) {
+          const uint32_t k = k0 + q, bits = s_hit[k];
+          if ((bits >> lane) & 1u) hit_list[s_a[k] + __popc(bits & ltmask)] = (w0 + k) * 32u + lane;
+        }
+      }
+      if (MODE == 0 && !MISSQ && miss_rec) {  // misses parked by a deferring closest-hit trace
+        uint4 m[COMPACT_PER];
+#pragma unroll
+        for (int q = 0; q < COMPACT_PER; q++)
+          if ((s_miss[k0 + q] >> lane) & 1u) m[q] = __ldcs(miss_rec + (w0 + k0 + q) * 32u + lane);
+#pragma unroll
+        for (int q = 0; q < COMPACT_PER; q++)
+          if ((s_miss[k0 + q] >> lane) & 1u)
+            add_color(color, npix, m[q].w, __uint_as_float(m[q].x), __uint_as_float(m[q].y), __uint_as_float(m[q].z),
+                      1.0f, &ctr->err);
+      }
+      if (MODE == 1 || MISSQ) {
+#pragma unroll
+        for (int q = 0; q < COMPACT_PER; q++) {
+          const uint32_t k = k0 + q, bits = s_miss[k];
+          if (!((bits >> lane) & 1u)) continue;
+          const uint32_t to = s_b[k] + __popc(bits & ltmask), j = (w0 + k) * 32u + lane;
+          if (to < miss_capacity) {
+            M.o[to] = src.o[j];
+            M.d[to] = src.d[j];
+            M.t[to] = src.t[j];
+          } else {
+            atomicOr(&ctr->err, ERR_QUEUE);
+          }
+        }
       }
     }
     __syncthreads();
   }
 }
+static int compact_r(uint32_t capacity) { return capacity >= (1u << 20) ? COMPACT_R_LARGE : 1; }
 
 // k_shade: shade_hit.wgsl main (:407-483).  Tiles of SHADE_THREADS hits are
 // claimed in order; bounce and shadow rays are written at their stable ranks
@@ -950,11 +987,11 @@ __global__ void k_math(int fn, const float* __restrict__ x, const float* __restr
 // =====================================================================
 static unsigned grid_for(uint32_t n, unsigned block) { return (unsigned)((n + block - 1) / block); }
 
-uint32_t compact_tiles(uint32_t capacity) { return ((capacity + 31u) / 32u + COMPACT_THREADS - 1) / COMPACT_THREADS; }
+uint32_t compact_tiles(uint32_t capacity) {
+  const uint32_t words = (uint32_t)(COMPACT_WORDS * compact_r(capacity));
+  return ((capacity + 31u) / 32u + words - 1) / words;
+}
 uint32_t shade_tiles(uint32_t capacity) { return (capacity + SHADE_THREADS - 1) / SHADE_THREADS; }
-
-// Persistent grids: enough resident blocks to fill every multiprocessor, never
-// more blocks than there can be work items.
 
 // =====================================================================
 // Form (2): one persistent launch renders many requests (camera, resolution,
@@ -1170,19 +1207,16 @@ void launch_batch(cudaStream_t s, const BatchConfig& c, unsigned grid, const Bat
 
 void launch_batch_next_frame(cudaStream_t s, uint32_t* frame) { k_batch_next_frame<<<1, 1, 0, s>>>(frame); }
 
-void kernel_grids(int sms, uint32_t capacity, unsigned* trace, unsigned* compact, unsigned* shade,
-                  unsigned* trace_wide) {
+Grids kernel_grids(int sms, uint32_t capacity) {
   int t = 0, c = 0, s = 0, w = 0;
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t, k_trace_dyn<false, true, false, false>, TRACE_THREADS, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&w, k_trace_cw<false, true, false>, TRACE_THREADS, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_compact<0, true>, COMPACT_THREADS, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_compact<0, true, COMPACT_R_LARGE>, COMPACT_THREADS, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s, k_shade, SHADE_THREADS, 0);
-  const unsigned warps = (capacity + 31u) / 32u;
-  *trace = std::max(1u, std::min((unsigned)(sms * std::max(t, 1)), (warps + TRACE_THREADS / 32 - 1) / (TRACE_THREADS / 32)));
-  *compact = std::max(1u, std::min((unsigned)(sms * std::max(c, 1)), compact_tiles(capacity)));
-  *shade = std::max(1u, std::min((unsigned)(sms * std::max(s, 1)), shade_tiles(capacity)));
-  *trace_wide =
-      std::max(1u, std::min((unsigned)(sms * std::max(w, 1)), (warps + TRACE_THREADS / 32 - 1) / (TRACE_THREADS / 32)));
+  const unsigned n = (unsigned)sms;
+  const unsigned rays = std::max(1u, ((capacity + 31u) / 32u + TRACE_THREADS / 32 - 1) / (TRACE_THREADS / 32));
+  return Grids{Grid{n * std::max(t, 1), rays}, Grid{n * std::max(c, 1), std::max(1u, compact_tiles(capacity))},
+               Grid{n * std::max(s, 1), std::max(1u, shade_tiles(capacity))}, Grid{n * std::max(w, 1), rays}};
 }
 
 void launch_camera(const LaunchCtx& L, RayQ R, uint32_t n_threads, int64_t offset) {
@@ -1192,14 +1226,12 @@ void launch_camera(const LaunchCtx& L, RayQ R, uint32_t n_threads, int64_t offse
 
 void launch_trace(const LaunchCtx& L, bool any_hit, bool fused, bool count, const uint32_t* countp, RayQ R,
                   uint4* hrec, uint32_t* flags, uint32_t* ticket) {
-  const dim3 grid(L.trace_blocks), block(TRACE_THREADS);
+  const dim3 grid(L.grids.trace.at(10)), block(TRACE_THREADS);
   const int defer = (L.defer_miss && fused && !any_hit) ? 1 : 0;
   if (L.trace_mode & TRACE_WIDE) {
     // (concurrent-work grids: 1080p, eight frames in flight, 3399-3423
     // Mrays/s against 3348-3379 with the full grid)
-    const dim3 grid(std::max(1u, L.trace_blocks_wide * (any_hit ? L.any_tenths : L.closest_tenths) / 10u));
-    const unsigned words = (L.capacity + 31u) / 32u + 1u;
-    if (!(any_hit && fused)) cudaMemsetAsync(flags, 0, (size_t)words * 4, L.stream);
+    const dim3 grid(L.grids.wide.at(any_hit ? L.any_tenths : L.closest_tenths));
 #define PK_TRACEW(A, F, C) \
   k_trace_cw<A, F, C><<<grid, block, 0, L.stream>>>(L.scene, L.env, L.ctr, countp, R, hrec, flags, L.color, L.npix, \
                                                       ticket, defer)
@@ -1214,9 +1246,7 @@ void launch_trace(const LaunchCtx& L, bool any_hit, bool fused, bool count, cons
     return;
   }
   if (L.trace_mode & TRACE_PERSISTENT) {
-    const dim3 grid(std::max(1u, L.trace_blocks * (any_hit ? L.any_tenths : L.closest_tenths) / 10u));
-    const unsigned words = (L.capacity + 31u) / 32u + 1u;
-    if (!(any_hit && fused)) cudaMemsetAsync(flags, 0, (size_t)words * 4, L.stream);
+    const dim3 grid(L.grids.trace.at(any_hit ? L.any_tenths : L.closest_tenths));
 #define PK_TRACED(A, F, C)                                                                                         \
   do {                                                                                                             \
     if (L.trace_mode & TRACE_EXACT)                                                                                \
@@ -1248,28 +1278,34 @@ void launch_trace(const LaunchCtx& L, bool any_hit, bool fused, bool count, cons
 #undef PK_TRACE
 }
 
-void launch_compact_trace(const LaunchCtx& L, bool missq, const uint32_t* flags, uint32_t* hit_list, RayQ src,
+void launch_compact_trace(const LaunchCtx& L, bool missq, uint32_t* flags, uint32_t* hit_list, RayQ src,
                           RayQ M, uint32_t* ticket, unsigned long long* tiles, const uint4* miss_rec) {
-  const unsigned grid = std::max(1u, L.compact_blocks * L.compact_tenths / 10u);
-  if (missq)
-    k_compact<0, true><<<grid, COMPACT_THREADS, 0, L.stream>>>(L.ctr, flags, hit_list, src, M, L.miss_capacity,
-                                                                ticket, tiles, nullptr, L.color, L.npix);
-  else
-    k_compact<0, false><<<grid, COMPACT_THREADS, 0, L.stream>>>(L.ctr, flags, hit_list, src, M, L.miss_capacity,
-                                                                 ticket, tiles, miss_rec, L.color, L.npix);
+  const unsigned grid = L.grids.compact.at(L.compact_tenths);
+#define PK_COMPACT(Q, R, REC)                                                                                    \
+  k_compact<0, Q, R><<<grid, COMPACT_THREADS, 0, L.stream>>>(L.ctr, flags, hit_list, src, M, L.miss_capacity, ticket, \
+                                                              tiles, REC, L.color, L.npix)
+  if (compact_r(L.capacity) == 1) {
+    if (missq) PK_COMPACT(true, 1, nullptr); else PK_COMPACT(false, 1, miss_rec);
+  } else {
+    if (missq) PK_COMPACT(true, COMPACT_R_LARGE, nullptr); else PK_COMPACT(false, COMPACT_R_LARGE, miss_rec);
+  }
+#undef PK_COMPACT
 }
 
-void launch_compact_shadow(const LaunchCtx& L, const uint32_t* flags, RayQ S, RayQ M, uint32_t* ticket,
+void launch_compact_shadow(const LaunchCtx& L, uint32_t* flags, RayQ S, RayQ M, uint32_t* ticket,
                            unsigned long long* tiles) {
-  k_compact<1, true><<<L.compact_blocks, COMPACT_THREADS, 0, L.stream>>>(L.ctr, flags, nullptr, S, M,
-                                                                           L.miss_capacity, ticket, tiles, nullptr,
-                                                                           L.color, L.npix);
+#define PK_COMPACT(R)                                                                                              \
+  k_compact<1, true, R><<<L.grids.compact.at(10), COMPACT_THREADS, 0, L.stream>>>(L.ctr, flags, nullptr, S, M,       \
+                                                                                   L.miss_capacity, ticket, tiles, \
+                                                                                   nullptr, L.color, L.npix)
+  if (compact_r(L.capacity) == 1) PK_COMPACT(1); else PK_COMPACT(COMPACT_R_LARGE);
+#undef PK_COMPACT
 }
 
 void launch_shade(const LaunchCtx& L, const uint32_t* hit_list, const uint4* hrec, RayQ Rin, RayQ Rout, RayQ S,
                   uint32_t* ticket, unsigned long long* tiles) {
-  k_shade<<<std::max(1u, L.shade_blocks * L.shade_tenths / 10u), SHADE_THREADS, 0, L.stream>>>(L.scene, L.env, L.ctr, hit_list, hrec, Rin, Rout, S,
-                                                          L.capacity, L.color, L.npix, ticket, tiles);
+  k_shade<<<L.grids.shade.at(L.shade_tenths), SHADE_THREADS, 0, L.stream>>>(L.scene, L.env, L.ctr, hit_list, hrec, Rin, Rout, S,
+                                                                          L.capacity, L.color, L.npix, ticket, tiles);
 }
 
 void launch_shade_miss(const LaunchCtx& L, RayQ M) {

@@ -12,6 +12,22 @@ namespace pk {
 // batched refill.  Both visit every ray's nodes in the reference order.
 enum TraceMode : int { TRACE_CHUNKED = 0, TRACE_PERSISTENT = 1, TRACE_WIDE = 4, TRACE_EXACT = 8 };
 
+// Blocks of the persistent kernels: what fills the GPU, and what the work of
+// a queue capacity can use.
+struct Grid {
+  unsigned full = 1, need = 1;
+  // A share of the full grid (tenths), no more than the work needs.  (The share
+  // used to be taken of the smaller of the two: a 256x256 frame with frames in
+  // flight traced 65,536 rays with half the blocks it had rays for.)
+  unsigned at(unsigned tenths) const {
+    const unsigned g = full * tenths / 10u;
+    return g < 1u ? 1u : (g < need ? g : need);
+  }
+};
+struct Grids {
+  Grid trace, compact, shade, wide;
+};
+
 // Everything a launch needs that is fixed for a configured context.
 struct LaunchCtx {
   cudaStream_t stream;
@@ -26,14 +42,14 @@ struct LaunchCtx {
   uint32_t npix;
   uint32_t capacity;       // ray / hit / shadow queue capacity (batch rounded up to 128)
   uint32_t miss_capacity;  // 2 * capacity
-  unsigned trace_blocks, compact_blocks, shade_blocks, trace_blocks_wide;
+  Grids grids;
   float4* accum_sum = nullptr;   // compensated accumulation (pk_set_accumulation), else null
   float4* accum_comp = nullptr;
   int trace_mode;
   // Closest-hit misses park their contribution in the hit record for the
   // compaction to add (frames whose shadow traversal overlaps the next bounce).
   bool defer_miss = false;
-  // Persistent grid of the binary traversals in tenths of trace_blocks:
+  // Persistent grids of the traversals in tenths of the full grid:
   // smaller when other work runs beside them (frames in flight, overlap).
   unsigned closest_tenths = 10, any_tenths = 10;
   unsigned shade_tenths = 10, compact_tenths = 10;  // the same for the shade and compaction grids
@@ -43,19 +59,20 @@ struct LaunchCtx {
 void launch_camera(const LaunchCtx& L, RayQ R, uint32_t n_threads, int64_t offset = -1);
 // Kernels that claim work through an atomic ticket take it as `ticket`; the
 // look-back kernels also take a zeroed tile-state array (one word per tile).
+// The persistent traversals set bits in `flags`, which must hold zeros; the
+// compaction that reads them leaves zeros.
 void launch_trace(const LaunchCtx& L, bool any_hit, bool fused, bool count, const uint32_t* countp, RayQ R,
                   uint4* hrec, uint32_t* flags, uint32_t* ticket);
 // miss_rec: the hit records of a trace launched with L.defer_miss (whose parked
 // miss contributions this compaction adds), else null.
-void launch_compact_trace(const LaunchCtx& L, bool missq, const uint32_t* flags, uint32_t* hit_list, RayQ src,
+void launch_compact_trace(const LaunchCtx& L, bool missq, uint32_t* flags, uint32_t* hit_list, RayQ src,
                           RayQ M, uint32_t* ticket, unsigned long long* tiles, const uint4* miss_rec);
-void launch_compact_shadow(const LaunchCtx& L, const uint32_t* flags, RayQ S, RayQ M, uint32_t* ticket,
+void launch_compact_shadow(const LaunchCtx& L, uint32_t* flags, RayQ S, RayQ M, uint32_t* ticket,
                            unsigned long long* tiles);
 void launch_shade(const LaunchCtx& L, const uint32_t* hit_list, const uint4* hrec, RayQ Rin, RayQ Rout, RayQ S,
                   uint32_t* ticket, unsigned long long* tiles);
 // Grid sizes for a queue capacity on a GPU with `sms` multiprocessors.
-void kernel_grids(int sms, uint32_t capacity, unsigned* trace, unsigned* compact, unsigned* shade,
-                  unsigned* trace_wide);
+Grids kernel_grids(int sms, uint32_t capacity);
 // Tile counts the look-back kernels need for a given queue capacity.
 uint32_t compact_tiles(uint32_t capacity);
 uint32_t shade_tiles(uint32_t capacity);
