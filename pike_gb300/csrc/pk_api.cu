@@ -173,6 +173,9 @@ int pk_create(pk_ctx** out, int device) {
     c->ctr.alloc(1);
     c->cam.alloc(1);
     c->scratch_pool = create_scratch_pool(device);
+    check(cudaHostAlloc(reinterpret_cast<void**>(&c->host_words), 64, cudaHostAllocMapped), "cudaHostAlloc");
+    check(cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->host_words_dev), c->host_words, 0),
+          "cudaHostGetDevicePointer");
     c->cast_scratch = noalloc_scratch_address();
     check(cudaMemsetAsync(c->ctr.p, 0, sizeof(Counters), c->stream), "memset");
     check(cudaStreamSynchronize(c->stream), "sync");
@@ -181,6 +184,7 @@ int pk_create(pk_ctx** out, int device) {
   if (rc != PK_OK) {
     std::fprintf(stderr, "pk_create: %s\n", c->err.c_str());
     if (c->scratch_pool) cudaMemPoolDestroy(c->scratch_pool);
+    if (c->host_words) cudaFreeHost(c->host_words);
     delete c;
     return rc;
   }
@@ -212,6 +216,7 @@ int pk_destroy(pk_ctx* c) {
   if (c->t0) cudaEventDestroy(c->t0);
   if (c->t1) cudaEventDestroy(c->t1);
   if (c->scratch_pool) cudaMemPoolDestroy(c->scratch_pool);
+  if (c->host_words) cudaFreeHost(c->host_words);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;
   return PK_OK;

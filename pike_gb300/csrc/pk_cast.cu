@@ -17,112 +17,263 @@ namespace pk {
 namespace {
 
 constexpr int CAST_THREADS = TRACE_THREADS;
-constexpr int LIST_THREADS = 256;
 
-// Every ray gets a record {t bits, triangle index or 0xffffffff, bary_mask, 0};
-// bit j of flags is set when ray j hit.
+// Every ray gets a record {t bits, triangle index or 0xffffffff, bary_mask, 0}.
+//
+// Large queries: persistent lanes.  A lane owns one ray at a time; when at
+// least CAST_REFILL lanes of a warp are idle they claim new rays together, and
+// a lane takes at most CAST_BUDGET inner steps before the warp meets again, so
+// no lane waits for the longest of a fixed group of 32 rays.  No speculation:
+// each ray visits the nodes and leaves of trace.wgsl's loop in its order.
+// Any hit reports the closest triangle of the first leaf with a hit
+// (trace_shadow.wgsl:154-158), so a leaf is always tested whole.
+// Bound by the latency of dependent node and triangle fetches.  The grid fills
+// the GPU whatever frame size the context is configured for (it used to be the
+// frame's: 32 blocks for a 64x64 one).  2,097,143 incoherent closest-hit rays in
+// the 1.3M-triangle scene: 13.3 ms -> 0.49 ms (4.3 Grays/s), 999,983 any-hit
+// rays in 327,690 triangles: 3.52 -> 0.23 ms.  Rays sorted beforehand by octant
+// and Morton code of the origin measured 0.46 and 0.20 ms, less than a sort
+// would cost.
+constexpr int CAST_REFILL = 16;
+constexpr int CAST_BUDGET = 8;
+constexpr int CAST_SMEM = 8;  // stack entries per lane in shared memory, the rest of 64 in local memory
+constexpr int CAST_LOCAL = 64 - CAST_SMEM;
+constexpr int CAST_BLOCKS = 10;  // resident blocks per SM
+
 template <bool ANY>
-__global__ void __launch_bounds__(CAST_THREADS) k_cast(SceneDev sc, const float4* __restrict__ o4,
-                                                        const float4* __restrict__ d4, uint32_t n,
-                                                        uint4* __restrict__ hits4, uint32_t* __restrict__ flags,
-                                                        uint32_t* __restrict__ ticket, uint32_t* __restrict__ err) {
-  __shared__ int sstack[STACK_SMEM][TRACE_THREADS];
-  const int lane = threadIdx.x & 31;
-  uint32_t nf = 0, nt = 0;
+__global__ void __launch_bounds__(CAST_THREADS, CAST_BLOCKS) k_cast(SceneDev sc, const float4* __restrict__ o4,
+                                                                    const float4* __restrict__ d4, uint32_t n,
+                                                                    uint4* __restrict__ hits4,
+                                                                    uint32_t* __restrict__ ticket,
+                                                                    uint32_t* __restrict__ err) {
+  __shared__ int sstack[CAST_SMEM][CAST_THREADS];
+  int lstack[CAST_LOCAL];
+  const int lane = threadIdx.x & 31, tid = threadIdx.x;
+  const uint32_t ltmask = (1u << lane) - 1u;
+  const float eps = ANY ? 1e-7f : 1e-8f;
+  uint32_t j = 0;
+  bool have = false, exhausted = false;
+  float ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f, ix = 0.f, iy = 0.f, iz = 0.f;
+  float best_t = MAX_T;
+  int best_i = -1;
+  uint32_t best_b = 0u;
+  int sp = 0, cur = 0;
   for (;;) {
-    uint32_t base = 0;
-    if (lane == 0) base = atomicAdd(ticket, 32u);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    if (base >= n) break;
-    const uint32_t j = base + lane;
-    bool hit = false;
-    if (j < n) {
-      const float4 o = o4[j], d = d4[j];
-      float bt;
-      int bi;
-      uint32_t bb;
-      traverse<ANY, false>(sc, o.x, o.y, o.z, d.x, d.y, d.z, bt, bi, bb, sstack, err, nf, nt);
-      hit = bi != -1;
-      hits4[j] = make_uint4(__float_as_uint(bt), (uint32_t)bi, bb, 0u);
+    const uint32_t idle = __ballot_sync(0xffffffffu, !have && !exhausted);
+    const uint32_t busy = __ballot_sync(0xffffffffu, have);
+    if (idle && (__popc(idle) >= CAST_REFILL || busy == 0u)) {
+      const int leader = __ffs(idle) - 1;
+      uint32_t base = 0;
+      if (lane == leader) base = atomicAdd(ticket, (uint32_t)__popc(idle));
+      base = __shfl_sync(0xffffffffu, base, leader);
+      if (!have && !exhausted) {
+        j = base + (uint32_t)__popc(idle & ltmask);
+        if (j < n) {
+          const float4 o = __ldcs(o4 + j), d = __ldcs(d4 + j);
+          ox = o.x; oy = o.y; oz = o.z;
+          dx = d.x; dy = d.y; dz = d.z;
+          ix = 1.0f / dx; iy = 1.0f / dy; iz = 1.0f / dz;
+          best_t = MAX_T; best_i = -1; best_b = 0u;
+          sp = 0;
+          cur = sc.root;
+          have = true;
+        } else {
+          exhausted = true;
+        }
+      }
     }
-    const uint32_t m = __ballot_sync(0xffffffffu, hit);
-    if (lane == 0) flags[base >> 5] = m;
+    if (!__any_sync(0xffffffffu, have)) break;
+    if (!have) continue;
+    bool fin = false;
+    int budget = CAST_BUDGET;
+    while (cur >= 0 && budget-- > 0) {
+      float lh, rh;
+      int cl, cr;
+      inner_children(sc, cur, ox, oy, oz, ix, iy, iz, lh, rh, cl, cr);
+      const bool lok = lh < best_t, rok = rh < best_t;
+      if (lok && rok) {
+        int nearc, farc;
+        if (lh > rh) { nearc = cr; farc = cl; } else { nearc = cl; farc = cr; }
+        if (sp < CAST_SMEM) sstack[sp][tid] = farc;
+        else if (sp < CAST_SMEM + CAST_LOCAL) lstack[sp - CAST_SMEM] = farc;
+        else { atomicOr(err, ERR_STACK); fin = true; break; }
+        ++sp;
+        cur = nearc;
+        continue;
+      }
+      if (lok) { cur = cl; continue; }
+      if (rok) { cur = cr; continue; }
+      if (sp == 0) { fin = true; break; }
+      --sp;
+      cur = sp < CAST_SMEM ? sstack[sp][tid] : lstack[sp - CAST_SMEM];
+    }
+    while (!fin && cur < 0) {
+      const uint32_t word = (uint32_t)cur & 0x7fffffffu;
+      const int size = (int)(word >> 24);
+      const int base = (int)(word & 0x00ffffffu);
+#pragma unroll 4
+      for (int i = 0; i < size; i++) {
+        float res, u, v;
+        if (!mt_test(sc, base + i, ox, oy, oz, dx, dy, dz, eps, res, u, v)) continue;
+        if (res < best_t) {
+          best_t = res;
+          best_i = base + i;
+          best_b = pack_unorm16(u) | (pack_unorm16(v) << 16);
+        }
+      }
+      if (ANY && best_i != -1) { fin = true; break; }
+      if (sp == 0) { fin = true; break; }
+      --sp;
+      cur = sp < CAST_SMEM ? sstack[sp][tid] : lstack[sp - CAST_SMEM];
+    }
+    if (fin) {
+      __stcs(hits4 + j, make_uint4(__float_as_uint(best_t), (uint32_t)best_i, best_b, 0u));
+      have = false;
+    }
   }
 }
 
-// Stable list of the rays that hit (increasing ray index) and its length.
-__global__ void __launch_bounds__(LIST_THREADS) k_hit_list(const uint32_t* __restrict__ flags, uint32_t n,
+// Stable list of the rays that hit (increasing ray index) and its length, from
+// the records' triangle indices: a lane per ray, tiles of LIST_TILE rays
+// claimed in order, a warp-wide look-back per tile.
+constexpr int LIST_THREADS = 256;
+constexpr int LIST_WARPS = LIST_THREADS / 32;
+constexpr int LIST_ROUNDS = 8;
+constexpr uint32_t LIST_TILE = LIST_THREADS * LIST_ROUNDS;
+__global__ void __launch_bounds__(LIST_THREADS) k_hit_list(const uint4* __restrict__ hits4, uint32_t n,
                                                             uint32_t* __restrict__ list, uint32_t* __restrict__ count,
                                                             uint32_t* __restrict__ ticket,
                                                             unsigned long long* __restrict__ tiles,
-                                                            uint32_t* __restrict__ err) {
-  __shared__ uint32_t s_tile;
-  __shared__ uint32_t s_warp[LIST_THREADS / 32 + 1][2];
-  __shared__ unsigned long long s_excl;
-  const uint32_t nwords = (n + 31) >> 5;
-  const uint32_t ntiles = (nwords + LIST_THREADS - 1) / LIST_THREADS;
-  if (ntiles == 0) {
-    if (blockIdx.x == 0 && threadIdx.x == 0) *count = 0;
-    return;
-  }
+                                                            uint32_t* __restrict__ err, uint32_t* host_err) {
+  __shared__ uint32_t s_tile, s_base;
+  __shared__ uint32_t s_warp[LIST_WARPS];
+  const uint32_t ntiles = (n + LIST_TILE - 1) / LIST_TILE;
+  const uint32_t lane = threadIdx.x & 31u, warp = threadIdx.x >> 5, ltmask = (1u << lane) - 1u;
+  if (ntiles == 0 && blockIdx.x == 0 && threadIdx.x == 0) *count = 0;
   for (;;) {
     if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
     __syncthreads();
     const uint32_t tile = s_tile;
     if (tile >= ntiles) break;
-    const uint32_t w = tile * LIST_THREADS + threadIdx.x;
-    uint32_t hm = 0u;
-    if (w < nwords) {
-      const uint32_t valid = (w == nwords - 1 && (n & 31u)) ? ((1u << (n & 31u)) - 1u) : 0xffffffffu;
-      hm = flags[w] & valid;
+    const uint32_t j0 = tile * LIST_TILE + warp * (LIST_ROUNDS * 32u) + lane;
+    uint32_t word[LIST_ROUNDS], mine = 0;
+#pragma unroll
+    for (int r = 0; r < LIST_ROUNDS; r++) {
+      const uint32_t j = j0 + 32u * r;
+      const bool hit = j < n && __ldg(&hits4[j].y) != 0xffffffffu;
+      word[r] = __ballot_sync(0xffffffffu, hit);
+      mine += (uint32_t)__popc(word[r]);
     }
-    uint32_t ea, eb, ta, tb;
-    block_scan2<LIST_THREADS / 32>((uint32_t)__popc(hm), 0u, ea, eb, ta, tb, s_warp);
-    if (threadIdx.x == 0) s_excl = lookback2(tiles, tile, pack2(ta, 0u), err);
+    if (lane == 0) s_warp[warp] = mine;
     __syncthreads();
-    uint32_t k = unpack_a(s_excl) + ea;
-    uint32_t bits = hm;
-    while (bits) {
-      const int b = __ffs(bits) - 1;
-      bits &= bits - 1u;
-      list[k++] = w * 32u + (uint32_t)b;
+    uint32_t before = 0, total = 0;
+#pragma unroll
+    for (int k = 0; k < LIST_WARPS; k++) {
+      if ((uint32_t)k < warp) before += s_warp[k];
+      total += s_warp[k];
     }
-    if (tile == ntiles - 1 && threadIdx.x == 0) *count = unpack_a(s_excl) + ta;
+    if (warp == 0) {
+      const uint32_t e = unpack_a(lookback2_warp(tiles, tile, pack2(total, 0u), err));
+      if (lane == 0) {
+        s_base = e;
+        if (tile == ntiles - 1) *count = e + total;
+      }
+    }
     __syncthreads();
+    uint32_t at = s_base + before;
+#pragma unroll
+    for (int r = 0; r < LIST_ROUNDS; r++) {
+      if ((word[r] >> lane) & 1u) list[at + __popc(word[r] & ltmask)] = j0 + 32u * r;
+      at += (uint32_t)__popc(word[r]);
+    }
+    __syncthreads();
+  }
+  // every block sees the traversal's errors and its own look-back's
+  if (threadIdx.x == 0 && *(volatile uint32_t*)err) *(volatile uint32_t*)host_err = 1u;
+}
+
+// Small queries (at most CAST_ONE rays): one launch of one block traces a ray
+// per thread and lists the hits, since launches, memsets and a copy are most
+// of such a query: 257 rays in the 770-triangle scene, the whole call from
+// Python, 59 -> 45 us.
+constexpr uint32_t CAST_ONE = 1024;
+constexpr int ONE_SMEM = 8;
+template <bool ANY>
+__global__ void __launch_bounds__(CAST_ONE) k_cast_one(SceneDev sc, const float4* __restrict__ o4,
+                                                       const float4* __restrict__ d4, uint32_t n,
+                                                       uint4* __restrict__ hits4, uint32_t* __restrict__ list,
+                                                       uint32_t* __restrict__ count, uint32_t* host_err) {
+  __shared__ int sstack[ONE_SMEM][CAST_ONE];
+  __shared__ uint32_t s_warp[CAST_ONE / 32];
+  __shared__ uint32_t s_err;
+  const uint32_t j = threadIdx.x, lane = j & 31u, warp = j >> 5;
+  if (j == 0) s_err = 0;
+  __syncthreads();
+  bool hit = false;
+  if (j < n) {
+    const float4 o = o4[j], d = d4[j];
+    float bt;
+    int bi;
+    uint32_t bb, nf = 0, nt = 0;
+    traverse<ANY, false, (int)CAST_ONE, ONE_SMEM>(sc, o.x, o.y, o.z, d.x, d.y, d.z, bt, bi, bb, sstack, &s_err, nf, nt);
+    hit = bi != -1;
+    hits4[j] = make_uint4(__float_as_uint(bt), (uint32_t)bi, bb, 0u);
+  }
+  const uint32_t m = __ballot_sync(0xffffffffu, hit);
+  if (lane == 0) s_warp[warp] = (uint32_t)__popc(m);
+  __syncthreads();
+  uint32_t before = 0, total = 0;
+  for (uint32_t k = 0; k < blockDim.x / 32; k++) {
+    if (k < warp) before += s_warp[k];
+    total += s_warp[k];
+  }
+  if (hit) list[before + __popc(m & ((1u << lane) - 1u))] = j;
+  if (j == 0) {
+    *count = total;
+    if (s_err) *(volatile uint32_t*)host_err = 1u;
   }
 }
 
 }  // namespace
 
-// Scratch words the two kernels need for n rays: two tickets, an error word,
-// the hit bitmask, and one look-back tile state per LIST_THREADS words.
+// Scratch words the two kernels need for n rays: two tickets and an error
+// word, and one look-back state per LIST_TILE rays; all start at zero.
 struct CastScratch {
   uint32_t* tickets;  // [0] trace, [1] list, [2] error flags, [3] unused
-  uint32_t* flags;
   unsigned long long* tiles;
 };
-size_t cast_flag_words(uint32_t n) { return ((size_t)n + 31) / 32; }
-size_t cast_tiles(uint32_t n) { return (cast_flag_words(n) + LIST_THREADS - 1) / LIST_THREADS; }
+size_t cast_tiles(uint32_t n) { return ((size_t)n + LIST_TILE - 1) / LIST_TILE; }
+size_t cast_bytes(uint32_t n) { return 16 + 8 * cast_tiles(n); }
 
-// Enqueue the query on `stream`: zero what must start at zero, then trace and list.
-int cast_enqueue(pk_ctx* c, const float4* o4, const float4* d4, uint32_t n, int any_hit, uint4* hits4,
-                 uint32_t* hit_index, uint32_t* n_hits, const CastScratch& s, cudaStream_t stream) {
-  check(cudaMemsetAsync(s.tickets, 0, 16, stream), "memset");
-  if (cast_tiles(n)) check(cudaMemsetAsync(s.tiles, 0, cast_tiles(n) * 8, stream), "memset");
-  LaunchCtx L = c->launch();
-  L.scene = c->dropin_scene();  // the drop-in's records whatever the trace mode
-  const unsigned warps = (unsigned)((n + 31) / 32);
-  const unsigned grid = std::max(1u, std::min(L.grids.trace.full, (warps + CAST_THREADS / 32 - 1) / (CAST_THREADS / 32)));
-  if (n) {
-    if (any_hit)
-      k_cast<true><<<grid, CAST_THREADS, 0, stream>>>(L.scene, o4, d4, n, hits4, s.flags, s.tickets, s.tickets + 2);
-    else
-      k_cast<false><<<grid, CAST_THREADS, 0, stream>>>(L.scene, o4, d4, n, hits4, s.flags, s.tickets, s.tickets + 2);
+// The query on the context's stream; returns when it has finished.  `space`:
+// cast_bytes(n) bytes of scratch when n > CAST_ONE.
+int cast_run(pk_ctx* c, const char* what, const float4* o4, const float4* d4, uint32_t n, int any_hit, uint4* hits4,
+             uint32_t* hit_index, uint32_t* n_hits, unsigned char* space) {
+  const cudaStream_t st = c->stream;
+  const SceneDev sc = c->dropin_scene();  // the drop-in's records whatever the trace mode
+  volatile uint32_t* bad = c->host_words;
+  *bad = 0;
+  if (n <= CAST_ONE) {
+    const unsigned threads = std::max(32u, (n + 31u) / 32u * 32u);
+    if (any_hit) k_cast_one<true><<<1, threads, 0, st>>>(sc, o4, d4, n, hits4, hit_index, n_hits, c->host_words_dev);
+    else k_cast_one<false><<<1, threads, 0, st>>>(sc, o4, d4, n, hits4, hit_index, n_hits, c->host_words_dev);
+  } else {
+    const CastScratch s{reinterpret_cast<uint32_t*>(space), reinterpret_cast<unsigned long long*>(space + 16)};
+    check(cudaMemsetAsync(space, 0, cast_bytes(n), st), "memset");
+    const unsigned warps = (unsigned)((n + 31) / 32);
+    const unsigned grid = std::min((unsigned)c->sms * CAST_BLOCKS, (warps + CAST_THREADS / 32 - 1) / (CAST_THREADS / 32));
+    if (any_hit) k_cast<true><<<grid, CAST_THREADS, 0, st>>>(sc, o4, d4, n, hits4, s.tickets, s.tickets + 2);
+    else k_cast<false><<<grid, CAST_THREADS, 0, st>>>(sc, o4, d4, n, hits4, s.tickets, s.tickets + 2);
+    const unsigned lgrid = (unsigned)std::min<size_t>(cast_tiles(n), (size_t)c->sms * 4);
+    k_hit_list<<<lgrid, LIST_THREADS, 0, st>>>(hits4, n, hit_index, n_hits, s.tickets + 1, s.tiles, s.tickets + 2,
+                                                c->host_words_dev);
   }
-  const unsigned lgrid = (unsigned)std::max<size_t>(1, std::min<size_t>(cast_tiles(n), (size_t)c->sms * 4));
-  k_hit_list<<<lgrid, LIST_THREADS, 0, stream>>>(s.flags, n, hit_index, n_hits, s.tickets + 1, s.tiles,
-                                                  s.tickets + 2);
-  check(cudaGetLastError(), "pk_cast_rays");
+  check(cudaGetLastError(), what);
+  check(cudaStreamSynchronize(st), "sync");
+  if (*bad) {
+    c->err = std::string(what) + ": device error flags";
+    return PK_ERR_DEVICE;
+  }
   return PK_OK;
 }
 
@@ -138,16 +289,9 @@ extern "C" int pk_cast_rays(pk_ctx* c, const float* ray_o4, const float* ray_d4,
     if (!c->bvh_ready) { c->err = "pk_cast_rays: no BVH"; return PK_ERR_STATE; }
     if ((n && (!ray_o4 || !ray_d4 || !hits4 || !hit_index)) || !n_hits) { c->err = "pk_cast_rays: null buffer"; return PK_ERR_ARG; }
     if (n > (1u << 30)) { c->err = "pk_cast_rays: too many rays"; return PK_ERR_ARG; }
-    DevBuf<uint32_t> tickets(4), flags(std::max<size_t>(cast_flag_words(n), 1));
-    DevBuf<unsigned long long> tiles(std::max<size_t>(cast_tiles(n), 1));
-    const CastScratch s{tickets.p, flags.p, tiles.p};
-    cast_enqueue(c, reinterpret_cast<const float4*>(ray_o4), reinterpret_cast<const float4*>(ray_d4), n, any_hit,
-                 reinterpret_cast<uint4*>(hits4), hit_index, n_hits, s, c->stream);
-    uint32_t err = 0;
-    check(cudaMemcpyAsync(&err, tickets.p + 2, 4, cudaMemcpyDeviceToHost, c->stream), "D2H");
-    check(cudaStreamSynchronize(c->stream), "sync");
-    if (err) { c->err = "pk_cast_rays: device error flags"; return PK_ERR_DEVICE; }
-    return PK_OK;
+    TmpBuf<unsigned char> space(c->scratch(), n > CAST_ONE ? cast_bytes(n) : 0);
+    return cast_run(c, "pk_cast_rays", reinterpret_cast<const float4*>(ray_o4), reinterpret_cast<const float4*>(ray_d4),
+                    n, any_hit, reinterpret_cast<uint4*>(hits4), hit_index, n_hits, space.p);
   } catch (CudaError& e) {
     c->err = e.what();
     return PK_ERR_CUDA;
@@ -155,20 +299,17 @@ extern "C" int pk_cast_rays(pk_ctx* c, const float* ray_o4, const float* ray_d4,
 }
 
 // ---- allocation-free variant -------------------------------------------------
-// pk_cast_rays allocates its scratch (work tickets, the per-ray hit bitmask and
-// the look-back tile states of the hit list) with cudaMalloc on every call.
+// pk_cast_rays takes its scratch (work tickets and the look-back states of the
+// hit list) from the context's pool, which can allocate.
 // pk_cast_rays_noalloc takes it from the file-scope array below instead, so it
-// calls neither cudaMalloc nor cudaFree.  Every GPU that loads the library
-// holds one copy of the array until the process exits.
+// allocates and frees nothing.  Every GPU that loads the library holds one copy
+// of the array until the process exits.
 namespace pk {
 namespace {
 
-constexpr uint32_t NOALLOC_MAX_RAYS = 1u << 20;                      // rays per call
-constexpr size_t NOALLOC_FLAG_WORDS = NOALLOC_MAX_RAYS / 32;          // 32768 u32
-constexpr size_t NOALLOC_TILES = (NOALLOC_FLAG_WORDS + LIST_THREADS - 1) / LIST_THREADS;  // 128 u64
-constexpr size_t NOALLOC_FLAGS_OFF = 256;
-constexpr size_t NOALLOC_TILES_OFF = NOALLOC_FLAGS_OFF + NOALLOC_FLAG_WORDS * 4;
-constexpr size_t NOALLOC_BYTES = NOALLOC_TILES_OFF + NOALLOC_TILES * 8;  // 132,352 bytes
+constexpr uint32_t NOALLOC_MAX_RAYS = 1u << 20;  // rays per call
+constexpr size_t NOALLOC_BYTES = 132352;         // as documented; the states of 2^20 rays take 4112
+static_assert(16 + 8 * ((size_t)NOALLOC_MAX_RAYS / LIST_TILE) <= NOALLOC_BYTES, "scratch too small");
 
 static __device__ __align__(256) unsigned char g_cast_scratch[NOALLOC_BYTES];
 
@@ -203,16 +344,9 @@ extern "C" int pk_cast_rays_noalloc(pk_ctx* c, const float* ray_o4, const float*
       return PK_ERR_ARG;
     }
     if (!c->cast_scratch) { c->err = "pk_cast_rays_noalloc: scratch address not set up"; return PK_ERR_STATE; }
-    unsigned char* base = static_cast<unsigned char*>(c->cast_scratch);
-    const CastScratch s{reinterpret_cast<uint32_t*>(base), reinterpret_cast<uint32_t*>(base + NOALLOC_FLAGS_OFF),
-                        reinterpret_cast<unsigned long long*>(base + NOALLOC_TILES_OFF)};
-    cast_enqueue(c, reinterpret_cast<const float4*>(ray_o4), reinterpret_cast<const float4*>(ray_d4), n, any_hit,
-                 reinterpret_cast<uint4*>(hits4), hit_index, n_hits, s, c->stream);
-    uint32_t err = 0;
-    check(cudaMemcpyAsync(&err, s.tickets + 2, 4, cudaMemcpyDeviceToHost, c->stream), "D2H");
-    check(cudaStreamSynchronize(c->stream), "sync");
-    if (err) { c->err = "pk_cast_rays_noalloc: device error flags"; return PK_ERR_DEVICE; }
-    return PK_OK;
+    return cast_run(c, "pk_cast_rays_noalloc", reinterpret_cast<const float4*>(ray_o4),
+                    reinterpret_cast<const float4*>(ray_d4), n, any_hit, reinterpret_cast<uint4*>(hits4), hit_index,
+                    n_hits, static_cast<unsigned char*>(c->cast_scratch));
   } catch (CudaError& e) {
     c->err = e.what();
     return PK_ERR_CUDA;

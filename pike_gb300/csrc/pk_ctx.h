@@ -170,6 +170,10 @@ struct pk_ctx {
   bool diff_env_ready = false;
   cudaMemPool_t scratch_pool = nullptr;  // the builders' temporaries (pk_util.h)
   pk::Scratch scratch() const { return pk::Scratch{stream, scratch_pool}; }
+  // A few page-locked words that a kernel can write and the host read after a
+  // synchronise: an error status without a copy.
+  uint32_t* host_words = nullptr;
+  uint32_t* host_words_dev = nullptr;
   void* cast_scratch = nullptr;  // pk_cast_rays_noalloc's static scratch on this device (set by pk_create)
 
   RayQ R(int i) { return slot[0].R(i); }
