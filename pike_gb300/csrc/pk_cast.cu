@@ -20,13 +20,9 @@ constexpr int CAST_THREADS = TRACE_THREADS;
 
 // Every ray gets a record {t bits, triangle index or 0xffffffff, bary_mask, 0}.
 //
-// Large queries: persistent lanes.  A lane owns one ray at a time; when at
-// least CAST_REFILL lanes of a warp are idle they claim new rays together, and
-// a lane takes at most CAST_BUDGET inner steps before the warp meets again, so
-// no lane waits for the longest of a fixed group of 32 rays.  No speculation:
-// each ray visits the nodes and leaves of trace.wgsl's loop in its order.
-// Any hit reports the closest triangle of the first leaf with a hit
-// (trace_shadow.wgsl:154-158), so a leaf is always tested whole.
+// Large queries: persistent lanes (trace_lanes); any hit reports the closest
+// triangle of the first leaf with a hit (trace_shadow.wgsl:154-158), so a leaf is
+// always tested whole.
 // Bound by the latency of dependent node and triangle fetches.  The grid fills
 // the GPU whatever frame size the context is configured for (it used to be the
 // frame's: 32 blocks for a 64x64 one).  2,097,143 incoherent closest-hit rays in
@@ -34,103 +30,22 @@ constexpr int CAST_THREADS = TRACE_THREADS;
 // rays in 327,690 triangles: 3.52 -> 0.23 ms.  Rays sorted beforehand by octant
 // and Morton code of the origin measured 0.46 and 0.20 ms, less than a sort
 // would cost.
-constexpr int CAST_REFILL = 16;
-constexpr int CAST_BUDGET = 8;
-constexpr int CAST_SMEM = 8;  // stack entries per lane in shared memory, the rest of 64 in local memory
-constexpr int CAST_LOCAL = 64 - CAST_SMEM;
-constexpr int CAST_BLOCKS = 10;  // resident blocks per SM
-
 template <bool ANY>
-__global__ void __launch_bounds__(CAST_THREADS, CAST_BLOCKS) k_cast(SceneDev sc, const float4* __restrict__ o4,
-                                                                    const float4* __restrict__ d4, uint32_t n,
-                                                                    uint4* __restrict__ hits4,
-                                                                    uint32_t* __restrict__ ticket,
-                                                                    uint32_t* __restrict__ err) {
-  __shared__ int sstack[CAST_SMEM][CAST_THREADS];
-  int lstack[CAST_LOCAL];
-  const int lane = threadIdx.x & 31, tid = threadIdx.x;
-  const uint32_t ltmask = (1u << lane) - 1u;
-  const float eps = ANY ? 1e-7f : 1e-8f;
-  uint32_t j = 0;
-  bool have = false, exhausted = false;
-  float ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f, ix = 0.f, iy = 0.f, iz = 0.f;
-  float best_t = MAX_T;
-  int best_i = -1;
-  uint32_t best_b = 0u;
-  int sp = 0, cur = 0;
-  for (;;) {
-    const uint32_t idle = __ballot_sync(0xffffffffu, !have && !exhausted);
-    const uint32_t busy = __ballot_sync(0xffffffffu, have);
-    if (idle && (__popc(idle) >= CAST_REFILL || busy == 0u)) {
-      const int leader = __ffs(idle) - 1;
-      uint32_t base = 0;
-      if (lane == leader) base = atomicAdd(ticket, (uint32_t)__popc(idle));
-      base = __shfl_sync(0xffffffffu, base, leader);
-      if (!have && !exhausted) {
-        j = base + (uint32_t)__popc(idle & ltmask);
-        if (j < n) {
-          const float4 o = __ldcs(o4 + j), d = __ldcs(d4 + j);
-          ox = o.x; oy = o.y; oz = o.z;
-          dx = d.x; dy = d.y; dz = d.z;
-          ix = 1.0f / dx; iy = 1.0f / dy; iz = 1.0f / dz;
-          best_t = MAX_T; best_i = -1; best_b = 0u;
-          sp = 0;
-          cur = sc.root;
-          have = true;
-        } else {
-          exhausted = true;
-        }
-      }
-    }
-    if (!__any_sync(0xffffffffu, have)) break;
-    if (!have) continue;
-    bool fin = false;
-    int budget = CAST_BUDGET;
-    while (cur >= 0 && budget-- > 0) {
-      float lh, rh;
-      int cl, cr;
-      inner_children(sc, cur, ox, oy, oz, ix, iy, iz, lh, rh, cl, cr);
-      const bool lok = lh < best_t, rok = rh < best_t;
-      if (lok && rok) {
-        int nearc, farc;
-        if (lh > rh) { nearc = cr; farc = cl; } else { nearc = cl; farc = cr; }
-        if (sp < CAST_SMEM) sstack[sp][tid] = farc;
-        else if (sp < CAST_SMEM + CAST_LOCAL) lstack[sp - CAST_SMEM] = farc;
-        else { atomicOr(err, ERR_STACK); fin = true; break; }
-        ++sp;
-        cur = nearc;
-        continue;
-      }
-      if (lok) { cur = cl; continue; }
-      if (rok) { cur = cr; continue; }
-      if (sp == 0) { fin = true; break; }
-      --sp;
-      cur = sp < CAST_SMEM ? sstack[sp][tid] : lstack[sp - CAST_SMEM];
-    }
-    while (!fin && cur < 0) {
-      const uint32_t word = (uint32_t)cur & 0x7fffffffu;
-      const int size = (int)(word >> 24);
-      const int base = (int)(word & 0x00ffffffu);
-#pragma unroll 4
-      for (int i = 0; i < size; i++) {
-        float res, u, v;
-        if (!mt_test(sc, base + i, ox, oy, oz, dx, dy, dz, eps, res, u, v)) continue;
-        if (res < best_t) {
-          best_t = res;
-          best_i = base + i;
-          best_b = pack_unorm16(u) | (pack_unorm16(v) << 16);
-        }
-      }
-      if (ANY && best_i != -1) { fin = true; break; }
-      if (sp == 0) { fin = true; break; }
-      --sp;
-      cur = sp < CAST_SMEM ? sstack[sp][tid] : lstack[sp - CAST_SMEM];
-    }
-    if (fin) {
-      __stcs(hits4 + j, make_uint4(__float_as_uint(best_t), (uint32_t)best_i, best_b, 0u));
-      have = false;
-    }
-  }
+__global__ void __launch_bounds__(CAST_THREADS, LANES_BLOCKS) k_cast(SceneDev sc, const float4* __restrict__ o4,
+                                                                     const float4* __restrict__ d4, uint32_t n,
+                                                                     uint4* __restrict__ hits4,
+                                                                     uint32_t* __restrict__ ticket,
+                                                                     uint32_t* __restrict__ err) {
+  __shared__ int sstack[LANES_SMEM][CAST_THREADS];
+  trace_lanes<ANY, true>(
+      sc, n, ticket, err, sstack,
+      [&](uint32_t j, float4& o, float4& d) {
+        o = __ldcs(o4 + j);
+        d = __ldcs(d4 + j);
+      },
+      [&](uint32_t j, float, float, float, float t, int i, uint32_t b) {
+        __stcs(hits4 + j, make_uint4(__float_as_uint(t), (uint32_t)i, b, 0u));
+      });
 }
 
 // Stable list of the rays that hit (increasing ray index) and its length, from
@@ -261,7 +176,7 @@ int cast_run(pk_ctx* c, const char* what, const float4* o4, const float4* d4, ui
     const CastScratch s{reinterpret_cast<uint32_t*>(space), reinterpret_cast<unsigned long long*>(space + 16)};
     check(cudaMemsetAsync(space, 0, cast_bytes(n), st), "memset");
     const unsigned warps = (unsigned)((n + 31) / 32);
-    const unsigned grid = std::min((unsigned)c->sms * CAST_BLOCKS, (warps + CAST_THREADS / 32 - 1) / (CAST_THREADS / 32));
+    const unsigned grid = std::min((unsigned)c->sms * LANES_BLOCKS, (warps + CAST_THREADS / 32 - 1) / (CAST_THREADS / 32));
     if (any_hit) k_cast<true><<<grid, CAST_THREADS, 0, st>>>(sc, o4, d4, n, hits4, s.tickets, s.tickets + 2);
     else k_cast<false><<<grid, CAST_THREADS, 0, st>>>(sc, o4, d4, n, hits4, s.tickets, s.tickets + 2);
     const unsigned lgrid = (unsigned)std::min<size_t>(cast_tiles(n), (size_t)c->sms * 4);

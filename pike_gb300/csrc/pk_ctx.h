@@ -168,6 +168,7 @@ struct pk_ctx {
   DevBuf<int2> diff_bins, diff_coords;
   DevBuf<float> diff_pdf;
   bool diff_env_ready = false;
+  DevBuf<unsigned char> diff_space;  // path queues and records of the differentiable renderer
   cudaMemPool_t scratch_pool = nullptr;  // the builders' temporaries (pk_util.h)
   pk::Scratch scratch() const { return pk::Scratch{stream, scratch_pool}; }
   // A few page-locked words that a kernel can write and the host read after a

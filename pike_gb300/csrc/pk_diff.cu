@@ -59,23 +59,7 @@
 
 namespace pk {
 
-constexpr int DIFF_THREADS = 128;  // = TRACE_THREADS (traversal stack layout)
 constexpr int DIFF_MAX_DEPTH = 8;
-// traversal stack entries per lane in shared memory (the rest of 64 in local
-// memory): a small shared stack leaves more of the SM's L1 to node records
-constexpr int DIFF_SSTACK = 8;
-// The forward inlines its traversal (twice: closest and shadow rays); the
-// out-of-line copy the adjoint calls measured slower there (771-780 against
-// 866-872 Mrays/s on the differentiation workload).
-// 8 resident blocks per SM (64 registers, some spilled) for both kernels:
-// forward 795 against 764 Mrays/s unconstrained, adjoint 592 against 531
-// (the differentiation workload, same call; 6 blocks: 788 and 557).
-#ifndef PK_DIFF_FWD_BLOCKS
-#define PK_DIFF_FWD_BLOCKS 8
-#endif
-#ifndef PK_DIFF_ADJ_BLOCKS
-#define PK_DIFF_ADJ_BLOCKS 8
-#endif
 
 struct DiffParams {
   const float* albedo;  // n_mats x 3 (base colour)
@@ -284,232 +268,307 @@ __device__ __forceinline__ void shade_diff(const SceneDev& sc, const EnvDev& env
   }
 }
 
-// One recorded vertex of a path: the throughput T reaching it, its factor P
-// to the next vertex's throughput, its contribution factor Q (contribution =
-// T * Q), the derivatives of P and Q by the material's albedo (per channel)
-// and roughness, dQ/dE (environment texel `tex`) and the material.  The
-// backward sweep overwrites dQa with dLoss/dalbedo, dQr[0] with
-// dLoss/droughness and QE with dLoss/dE.
-struct DVert {
-  float T[3], P[3], dPa[3], dPr[3], Q[3], dQa[3], dQr[3], QE[3];
-  int tex, mat;
+// ---- the wavefront --------------------------------------------------------
+// Paths are rendered a chunk at a time, all of a chunk's paths one bounce per
+// round: closest hits (trace_lanes), shading, shadow rays (trace_lanes).  The
+// random numbers of a vertex depend on pixel, sample and bounce only, so the
+// queues need no order: blocks append rays as they come.  What a path adds to
+// its pixel at each bounce is kept and summed afterwards in the order in which
+// one thread per pixel would meet it (sample by sample, bounce by bounce), so
+// the image has the same bits as a path-by-path loop.
+//   A thread per pixel that walks its samples one after the other (the form
+// before) kept 32 paths of different lengths in lockstep through traversal and
+// shading: 0.8 Grays/s forward on the 512x512, 16 spp, 1.3M-triangle workload,
+// where the same rays as queues run at the frame renderer's rate.
+struct PathCount {  // one per chunk, zero at its start
+  uint32_t rays[DIFF_MAX_DEPTH + 1], shadow[DIFF_MAX_DEPTH];
+  uint32_t ticket[DIFF_MAX_DEPTH], shadow_ticket[DIFF_MAX_DEPTH];
+};
+struct PathTotal {
+  unsigned long long rays;
+  uint32_t err, pad;
 };
 
-__device__ __forceinline__ void set3(float* d, V3 v) { d[0] = v.x; d[1] = v.y; d[2] = v.z; }
-__device__ __forceinline__ void set3(float* d, float x, float y, float z) { d[0] = x; d[1] = y; d[2] = z; }
+// Buffers of a chunk of n paths.  Ray queues {origin, path}, {direction, -},
+// {throughput, pixel}; per path the number of bounces it lived.
+struct PathDev {
+  float4 *o[2], *d[2], *t[2], *so, *sd, *st;
+  uint4* hit;
+  uint8_t* lived;
+  float4* add;     // forward: [bounce][path] contribution
+  float4* rec[6];  // adjoint: [bounce][path] vertex record
+  uint32_t n;
+  PathCount* count;
+  PathTotal* total;
+};
 
-// trace.wgsl (any = false) or trace_shadow.wgsl (any = true) on the drop-in's records.
-__device__ __forceinline__ void diff_trace(bool any, const SceneDev& sc, float4 o, float4 d, float& t, int& idx,
-                                           uint32_t& bary, int (*sstack)[TRACE_THREADS], uint32_t* err) {
-  uint32_t nf = 0, nt = 0;
-  traverse_rt<false, TRACE_THREADS, DIFF_SSTACK>(any, sc, o.x, o.y, o.z, d.x, d.y, d.z, t, idx, bary, sstack, err, nf,
-                                                nt);
-}
-// The adjoint calls the shading and the traversal out of line: with them
-// inlined its path loop overflows the instruction cache (ncu: instruction
-// fetch was its largest stall).  Measured on the differentiation workload:
-// adjoint 648 against 587 Mrays/s inlined; the forward kernel is faster
-// inlined (783 against 738), so it keeps them inline.
-__device__ __noinline__ void diff_trace_out(bool any, const SceneDev& sc, float4 o, float4 d, float& t, int& idx,
-                                            uint32_t& bary, int (*sstack)[TRACE_THREADS], uint32_t* err) {
-  diff_trace(any, sc, o, d, t, idx, bary, sstack, err);
-}
-__device__ __noinline__ void shade_diff_out(const SceneDev& sc, const EnvDev& env, const DiffParams& P, float theta,
-                                            int32_t samples, uint32_t r, float4 o4, float4 d4, float4 t4, uint4 hr,
-                                            DiffShade& out) {
-  shade_diff<true>(sc, env, P, theta, samples, r, o4, d4, t4, hr, out);
-}
+// A vertex record.  Its contribution is T S E, the next vertex's throughput
+// T P; dPa / dSa: derivatives of P / S by the same channel of the albedo, dPr /
+// dSr by the roughness; E: environment radiance, texel `tex` (-1: none).
+//   0: T, material (-1: none, -2: not a vertex, an alpha pass-through)
+//   1: P, dPa   2: dPr, dSa   3: S, -   4: dSr, tex   5: E, -
+constexpr int REC_SKIP = -2;
 
-// One path of pixel (px, py) with camera.wgsl's sample index `samples`: the
-// loop of k_batch (closest hit, shading, the shadow ray, the next bounce while
-// fewer than depth closest-hit rays were traced).  acc += its contributions in
-// the order the drop-in adds them; REC: V[0..nv) its vertices.
-template <bool REC>
-__device__ __forceinline__ void diff_path(const SceneDev& sc, const EnvDev& env, const CamState& cam,
-                                          const DiffParams& P, float theta, uint32_t W, uint32_t H, uint32_t px,
-                                          uint32_t py, int32_t samples, float acc[3], DVert* V, int& nv,
-                                          int (*sstack)[TRACE_THREADS], uint32_t* err, uint32_t& nrays) {
+struct ViewDev {
+  CamState cam;
+  float theta;
+  uint32_t W, H;
+  unsigned long long first;  // path index of the chunk's first path: sample * W * H + pixel
+};
+
+constexpr int PATH_THREADS = 128;
+
+__global__ void __launch_bounds__(PATH_THREADS) k_path_camera(PathDev D, ViewDev V, uint32_t sample_base) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) D.count->rays[0] = D.n;
+  if (i >= D.n) return;
+  const unsigned long long npix = (unsigned long long)V.W * V.H, p = V.first + i;
+  const uint32_t pix = (uint32_t)(p % npix), px = pix % V.W, py = pix / V.W;
   V3 org, dir;
-  camera_ray(cam, px, py, W, H, samples, org, dir);
-  float4 o4 = make_float4(org.x, org.y, org.z, 0.0f), d4 = make_float4(dir.x, dir.y, dir.z, 0.0f);
-  float4 t4 = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(py * W + px));
-  nv = 0;
-  for (int bounce = 0; bounce < P.depth; bounce++) {
-    float t;
-    int idx;
-    uint32_t bary;
-    if (REC) diff_trace_out(false, sc, o4, d4, t, idx, bary, sstack, err);
-    else diff_trace(false, sc, o4, d4, t, idx, bary, sstack, err);
-    nrays++;
-    if (idx < 0) {
-      int tex;
-      const V3 e = diff_env(P, theta, v3(d4.x, d4.y, d4.z), tex);
-      acc[0] = acc[0] + e.x * t4.x;
-      acc[1] = acc[1] + e.y * t4.y;
-      acc[2] = acc[2] + e.z * t4.z;
-      if (REC) {
-        DVert& R = V[nv++];
-        set3(R.T, t4.x, t4.y, t4.z);
-        set3(R.Q, e);
-        set3(R.QE, 1.0f, 1.0f, 1.0f);
-        set3(R.P, 0.0f, 0.0f, 0.0f); set3(R.dPa, 0.0f, 0.0f, 0.0f); set3(R.dPr, 0.0f, 0.0f, 0.0f);
-        set3(R.dQa, 0.0f, 0.0f, 0.0f); set3(R.dQr, 0.0f, 0.0f, 0.0f);
-        R.tex = tex;
-        R.mat = -1;
-      }
-      return;
-    }
-    DiffShade s;
-    const uint4 hr = make_uint4(__float_as_uint(t), (uint32_t)idx, bary, 0u);
-    if (REC) shade_diff_out(sc, env, P, theta, samples, (uint32_t)bounce, o4, d4, t4, hr, s);
-    else shade_diff<false>(sc, env, P, theta, samples, (uint32_t)bounce, o4, d4, t4, hr, s);
-    float cr = 0.0f, cg = 0.0f, cb = 0.0f;
-    if (s.emitted) { cr = s.em.x; cg = s.em.y; cb = s.em.z; }
-    int stex = -1;
-    V3 se = v3(0.0f, 0.0f, 0.0f);
-    if (s.es) {
-      float ts;
-      int is;
-      uint32_t sb;
-      if (REC) diff_trace_out(true, sc, s.so, s.sd, ts, is, sb, sstack, err);
-      else diff_trace(true, sc, s.so, s.sd, ts, is, sb, sstack, err);
-      nrays++;
-      if (is < 0) {
-        se = diff_env(P, theta, v3(s.sd.x, s.sd.y, s.sd.z), stex);
-        cr += se.x * s.st.x;
-        cg += se.y * s.st.y;
-        cb += se.z * s.st.z;
-      }
-    }
-    acc[0] = acc[0] + cr;
-    acc[1] = acc[1] + cg;
-    acc[2] = acc[2] + cb;
-    const bool next = s.eb && bounce + 1 < P.depth;
-    if (REC && !(s.pass && next)) {  // a pass-through that continues changes nothing: not recorded
-      DVert& R = V[nv++];
-      set3(R.T, t4.x, t4.y, t4.z);
-      if (next) {
-        set3(R.P, s.P); set3(R.dPa, s.dPa); set3(R.dPr, s.dPr);
+  camera_ray(V.cam, px, py, V.W, V.H, (int32_t)(sample_base + (uint32_t)(p / npix)), org, dir);
+  D.o[0][i] = make_float4(org.x, org.y, org.z, __uint_as_float(i));
+  D.d[0][i] = make_float4(dir.x, dir.y, dir.z, 0.0f);
+  D.t[0][i] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(pix));
+}
+
+__global__ void __launch_bounds__(TRACE_THREADS, LANES_BLOCKS) k_path_trace(SceneDev sc, PathDev D, int bounce) {
+  __shared__ int sstack[LANES_SMEM][TRACE_THREADS];
+  const int b = bounce & 1;
+  trace_lanes<false, true>(
+      sc, D.count->rays[bounce], D.count->ticket + bounce, &D.total->err, sstack,
+      [&](uint32_t j, float4& o, float4& d) {
+        o = D.o[b][j];
+        d = D.d[b][j];
+      },
+      [&](uint32_t j, float, float, float, float t, int i, uint32_t bary) {
+        __stcs(D.hit + j, make_uint4(__float_as_uint(t), (uint32_t)i, bary, 0u));
+      });
+}
+
+// shade_miss.wgsl or shade_hit.wgsl for every ray of the bounce.
+#ifndef PK_PATH_SHADE_BLOCKS
+#define PK_PATH_SHADE_BLOCKS 6
+#endif
+template <bool REC>
+__global__ void __launch_bounds__(PATH_THREADS, PK_PATH_SHADE_BLOCKS) k_path_shade(SceneDev sc, EnvDev env, DiffParams P,
+                                                                                  PathDev D, ViewDev V, int bounce) {
+  __shared__ uint32_t s_n[2], s_at[2];
+  const uint32_t n = D.count->rays[bounce];
+  const int b = bounce & 1;
+  const unsigned long long npix = (unsigned long long)V.W * V.H;
+  const uint32_t lane = threadIdx.x & 31u, ltmask = (1u << lane) - 1u;
+  for (uint32_t base = blockIdx.x * PATH_THREADS; base < n; base += gridDim.x * PATH_THREADS) {
+    const uint32_t j = base + threadIdx.x;
+    if (threadIdx.x < 2) s_n[threadIdx.x] = 0;
+    __syncthreads();
+    bool next = false, es = false;
+    float4 bo, bd, bt, so, sd, st;
+    if (j < n) {
+      const float4 o4 = __ldcs(D.o[b] + j), d4 = __ldcs(D.d[b] + j), t4 = __ldcs(D.t[b] + j);
+      const uint4 hr = __ldcs(D.hit + j);
+      const uint32_t path = __float_as_uint(o4.w);
+      const size_t at = (size_t)bounce * D.n + path;
+      D.lived[path] = (uint8_t)(bounce + 1);
+      if ((int)hr.y < 0) {
+        int tex;
+        const V3 e = diff_env(P, V.theta, v3(d4.x, d4.y, d4.z), tex);
+        if (REC) {
+          D.rec[0][at] = make_float4(t4.x, t4.y, t4.z, __int_as_float(-1));
+          D.rec[1][at] = make_float4(0.f, 0.f, 0.f, 0.f);
+          D.rec[2][at] = make_float4(0.f, 0.f, 0.f, 0.f);
+          D.rec[3][at] = make_float4(1.f, 1.f, 1.f, 0.f);
+          D.rec[4][at] = make_float4(0.f, 0.f, 0.f, __int_as_float(tex));
+          D.rec[5][at] = make_float4(e.x, e.y, e.z, 0.f);
+        } else {
+          D.add[at] = make_float4(e.x * t4.x, e.y * t4.y, e.z * t4.z, 0.0f);
+        }
       } else {
-        set3(R.P, 0.0f, 0.0f, 0.0f); set3(R.dPa, 0.0f, 0.0f, 0.0f); set3(R.dPr, 0.0f, 0.0f, 0.0f);
-      }
-      if (s.emitted) {
-        set3(R.Q, s.Qem);
-        set3(R.dQa, 0.0f, 0.0f, 0.0f); set3(R.dQr, 0.0f, 0.0f, 0.0f); set3(R.QE, 0.0f, 0.0f, 0.0f);
-        R.tex = -1;
-        R.mat = -1;
-      } else {
-        set3(R.Q, s.S.x * se.x, s.S.y * se.y, s.S.z * se.z);
-        set3(R.dQa, s.dSa.x * se.x, s.dSa.y * se.y, s.dSa.z * se.z);
-        set3(R.dQr, s.dSr.x * se.x, s.dSr.y * se.y, s.dSr.z * se.z);
-        set3(R.QE, s.S);
-        R.tex = stex;
-        R.mat = s.mat;
+        DiffShade s;
+        const int32_t samples = (int32_t)(P.sample_base + (uint32_t)((V.first + path) / npix));
+        shade_diff<REC>(sc, env, P, V.theta, samples, (uint32_t)bounce, o4, d4, t4, hr, s);
+        next = s.eb && bounce + 1 < P.depth;
+        es = s.es;
+        bo = make_float4(s.bo.x, s.bo.y, s.bo.z, o4.w); bd = s.bd; bt = s.bt;
+        so = make_float4(s.so.x, s.so.y, s.so.z, o4.w); sd = s.sd; st = s.st;
+        if (REC) {
+          if (s.pass && next) {  // changes nothing: not a vertex
+            D.rec[0][at] = make_float4(0.f, 0.f, 0.f, __int_as_float(REC_SKIP));
+          } else {
+            const V3 zero = v3(0.0f, 0.0f, 0.0f);
+            const V3 p = next ? s.P : zero, dpr = next ? s.dPr : zero;
+            const float dpa = next ? s.dPa.x : 0.0f;
+            const V3 q = s.emitted ? s.Qem : s.S;
+            D.rec[0][at] = make_float4(t4.x, t4.y, t4.z, __int_as_float(s.emitted ? -1 : s.mat));
+            D.rec[1][at] = make_float4(p.x, p.y, p.z, dpa);
+            D.rec[2][at] = make_float4(dpr.x, dpr.y, dpr.z, s.emitted ? 0.0f : s.dSa.x);
+            D.rec[3][at] = make_float4(q.x, q.y, q.z, 0.0f);
+            D.rec[4][at] = make_float4(s.dSr.x, s.dSr.y, s.dSr.z, __int_as_float(-1));
+            const float one = s.emitted ? 1.0f : 0.0f;  // a shadow ray that escapes writes its radiance
+            D.rec[5][at] = make_float4(one, one, one, 0.0f);
+          }
+        } else {
+          D.add[at] = s.emitted ? make_float4(s.em.x, s.em.y, s.em.z, 0.0f) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
       }
     }
-    if (!next) return;
-    o4 = s.bo;
-    d4 = s.bd;
-    t4 = s.bt;
+    // append: one counter update per block and queue
+    const uint32_t mb = __ballot_sync(0xffffffffu, next), ms = __ballot_sync(0xffffffffu, es);
+    uint32_t wb = 0, ws = 0;
+    if (lane == 0) {
+      if (mb) wb = atomicAdd(&s_n[0], (uint32_t)__popc(mb));
+      if (ms) ws = atomicAdd(&s_n[1], (uint32_t)__popc(ms));
+    }
+    wb = __shfl_sync(0xffffffffu, wb, 0);
+    ws = __shfl_sync(0xffffffffu, ws, 0);
+    __syncthreads();
+    if (threadIdx.x == 0 && s_n[0]) s_at[0] = atomicAdd(&D.count->rays[bounce + 1], s_n[0]);
+    if (threadIdx.x == 32 && s_n[1]) s_at[1] = atomicAdd(&D.count->shadow[bounce], s_n[1]);
+    __syncthreads();
+    if (next) {
+      const uint32_t k = s_at[0] + wb + (uint32_t)__popc(mb & ltmask);
+      __stcs(D.o[b ^ 1] + k, bo);
+      __stcs(D.d[b ^ 1] + k, bd);
+      __stcs(D.t[b ^ 1] + k, bt);
+    }
+    if (es) {
+      const uint32_t k = s_at[1] + ws + (uint32_t)__popc(ms & ltmask);
+      __stcs(D.so + k, so);
+      __stcs(D.sd + k, sd);
+      __stcs(D.st + k, st);
+    }
+    __syncthreads();
   }
 }
 
-__global__ void __launch_bounds__(DIFF_THREADS, PK_DIFF_FWD_BLOCKS) k_diff_forward(SceneDev sc, EnvDev env, CamState cam, DiffParams P,
-                                                               float theta, uint32_t W, uint32_t H,
-                                                               float4* __restrict__ image, uint32_t* err,
-                                                               unsigned long long* rays) {
-  __shared__ int sstack[DIFF_SSTACK][TRACE_THREADS];
+// trace_shadow.wgsl for the bounce's shadow rays; one that escapes adds the
+// environment's radiance to its vertex (each vertex has at most one).
+template <bool REC>
+__global__ void __launch_bounds__(TRACE_THREADS, LANES_BLOCKS) k_path_shadow(SceneDev sc, DiffParams P, PathDev D,
+                                                                             float theta, int bounce) {
+  __shared__ int sstack[LANES_SMEM][TRACE_THREADS];
+  trace_lanes<true, false>(
+      sc, D.count->shadow[bounce], D.count->shadow_ticket + bounce, &D.total->err, sstack,
+      [&](uint32_t j, float4& o, float4& d) {
+        o = D.so[j];
+        d = D.sd[j];
+      },
+      [&](uint32_t j, float dx, float dy, float dz, float, int i, uint32_t) {
+        if (i >= 0) return;
+        const size_t at = (size_t)bounce * D.n + __float_as_uint(D.so[j].w);
+        int tex;
+        const V3 e = diff_env(P, theta, v3(dx, dy, dz), tex);
+        if (REC) {
+          D.rec[4][at].w = __int_as_float(tex);
+          D.rec[5][at] = make_float4(e.x, e.y, e.z, 0.0f);
+        } else {
+          const float4 st = D.st[j];
+          float4 a = D.add[at];
+          a.x += e.x * st.x;
+          a.y += e.y * st.y;
+          a.z += e.z * st.z;
+          D.add[at] = a;
+        }
+      });
+}
+
+// Sums of the chunk's contributions, continuing image (the sums of the chunks
+// before; `last`: then the mean).
+__global__ void __launch_bounds__(PATH_THREADS) k_path_sum(PathDev D, unsigned long long first, uint32_t npix,
+                                                           float4* __restrict__ image, float inv, int last) {
   const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-  if (pix >= W * H) return;
-  const uint32_t px = pix % W, py = pix / W;
-  float acc[3] = {0.0f, 0.0f, 0.0f};
-  uint32_t nrays = 0;
-  for (int s = 0; s < P.spp; s++) {
-    int nv;
-    diff_path<false>(sc, env, cam, P, theta, W, H, px, py, (int32_t)(P.sample_base + (uint32_t)s), acc, nullptr, nv,
-                     sstack, err, nrays);
+  if (pix >= npix) return;
+  float4 acc = first ? image[pix] : make_float4(0.f, 0.f, 0.f, 0.f);
+  const uint32_t r = (uint32_t)(first % npix);
+  for (unsigned long long i = pix >= r ? pix - r : (unsigned long long)npix - r + pix; i < D.n; i += npix) {
+    const int nb = D.lived[i];
+    for (int b = 0; b < nb; b++) {
+      const float4 c = __ldcs(D.add + (size_t)b * D.n + i);
+      acc.x = acc.x + c.x;
+      acc.y = acc.y + c.y;
+      acc.z = acc.z + c.z;
+    }
   }
-  const float inv = 1.0f / (float)P.spp;
-  image[pix] = make_float4(acc[0] * inv, acc[1] * inv, acc[2] * inv, 0.0f);
-  atomicAdd(rays, (unsigned long long)nrays);
+  image[pix] = last ? make_float4(acc.x * inv, acc.y * inv, acc.z * inv, 0.0f) : acc;
 }
 
 // Sum of v over the lanes of `mask` holding the same key; the lowest such lane
 // receives it (others get 0).  Every lane of `mask` must call it.
-__device__ __forceinline__ float group_sum(unsigned mask, int key, float v, bool& leader) {
-  const unsigned peers = __match_any_sync(mask, key);
+__device__ __forceinline__ float group_sum(unsigned peers, float v) {
   float sum = 0.0f;
   for (unsigned m = peers; m; m &= m - 1u) sum += __shfl_sync(peers, v, __ffs(m) - 1);
-  leader = (int)(threadIdx.x & 31u) == __ffs(peers) - 1;
   return sum;
 }
 
-__global__ void __launch_bounds__(DIFF_THREADS, PK_DIFF_ADJ_BLOCKS) k_diff_adjoint(SceneDev sc, EnvDev env, CamState cam, DiffParams P,
-                                                               float theta, uint32_t W, uint32_t H,
-                                                               const float4* __restrict__ dimage,
-                                                               double* __restrict__ g_albedo,
-                                                               double* __restrict__ g_rough,
-                                                               double* __restrict__ g_env, uint32_t* err,
-                                                               unsigned long long* rays) {
-  __shared__ int sstack[DIFF_SSTACK][TRACE_THREADS];
+// The backward sweep of the chunk's paths: L_v = Q_v + P_v L_{v+1} from the last
+// vertex, gradients per vertex.  Material terms: warp-aggregated atomics into
+// per-block FP32 partials, flushed with FP64 atomics; environment terms:
+// warp-aggregated per texel, added in FP64.
+constexpr int SWEEP_THREADS = 256;
+constexpr int SWEEP_PATHS = 8;  // paths per thread: the partials of a block cover 2048
+__global__ void __launch_bounds__(SWEEP_THREADS) k_path_sweep(DiffParams P, PathDev D, unsigned long long first,
+                                                              uint32_t npix, const float4* __restrict__ dimage,
+                                                              double* __restrict__ g_albedo,
+                                                              double* __restrict__ g_rough,
+                                                              double* __restrict__ g_env) {
   extern __shared__ float spart[];  // n_mats x 4: albedo rgb, roughness
   for (uint32_t i = threadIdx.x; i < 4 * P.n_mats; i += blockDim.x) spart[i] = 0.0f;
   __syncthreads();
-  const uint32_t pix = blockIdx.x * blockDim.x + threadIdx.x;
-  const bool live = pix < W * H;  // every lane stays for the warp-wide reductions
-  const uint32_t px = live ? pix % W : 0u, py = live ? pix / W : 0u;
-  float g[3] = {0.0f, 0.0f, 0.0f};
-  if (live) {
-    const float4 dv = dimage[pix];
-    const float inv = 1.0f / (float)P.spp;
-    g[0] = dv.x * inv; g[1] = dv.y * inv; g[2] = dv.z * inv;
-  }
-  DVert V[DIFF_MAX_DEPTH];
-  uint32_t nrays = 0;
-  for (int s = 0; s < P.spp; s++) {
+  const float inv = 1.0f / (float)P.spp;
+  for (int q = 0; q < SWEEP_PATHS; q++) {
+    const uint32_t i = (blockIdx.x * SWEEP_PATHS + q) * SWEEP_THREADS + threadIdx.x;
+    float g[3] = {0.0f, 0.0f, 0.0f}, L[3] = {0.0f, 0.0f, 0.0f};
     int nv = 0;
-    float acc[3] = {0.0f, 0.0f, 0.0f};
-    if (live)
-      diff_path<true>(sc, env, cam, P, theta, W, H, px, py, (int32_t)(P.sample_base + (uint32_t)s), acc, V, nv,
-                      sstack, err, nrays);
-    // backward sweep
-    float L[3] = {0.0f, 0.0f, 0.0f};
-    for (int v = nv - 1; v >= 0; v--) {
-      DVert& R = V[v];
-      float dr = 0.0f;
-#pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const float gt = g[c] * R.T[c];
-        const float da = gt * (R.dQa[c] + R.dPa[c] * L[c]);
-        dr += gt * (R.dQr[c] + R.dPr[c] * L[c]);
-        R.QE[c] = gt * R.QE[c];
-        L[c] = R.Q[c] + R.P[c] * L[c];
-        R.dQa[c] = da;
-      }
-      R.dQr[0] = dr;
+    if (i < D.n) {
+      const float4 dv = dimage[(uint32_t)((first + i) % npix)];
+      g[0] = dv.x * inv; g[1] = dv.y * inv; g[2] = dv.z * inv;
+      nv = D.lived[i];
     }
-    // scatter, record by record across the warp
-    for (int v = 0; v < DIFF_MAX_DEPTH; v++) {
-      if (!__any_sync(0xffffffffu, v < nv)) break;
-      const bool on = v < nv;
-      const int mkey = on ? V[v].mat : -1;
-      bool lead;
-      const float s0 = group_sum(0xffffffffu, mkey, mkey >= 0 ? V[v].dQa[0] : 0.0f, lead);
-      const float s1 = group_sum(0xffffffffu, mkey, mkey >= 0 ? V[v].dQa[1] : 0.0f, lead);
-      const float s2 = group_sum(0xffffffffu, mkey, mkey >= 0 ? V[v].dQa[2] : 0.0f, lead);
-      const float s3 = group_sum(0xffffffffu, mkey, mkey >= 0 ? V[v].dQr[0] : 0.0f, lead);
-      if (lead && mkey >= 0) {
-        atomicAdd(&spart[4 * mkey + 0], s0);
-        atomicAdd(&spart[4 * mkey + 1], s1);
-        atomicAdd(&spart[4 * mkey + 2], s2);
-        atomicAdd(&spart[4 * mkey + 3], s3);
-      }
-      const int tkey = on ? V[v].tex : -1;
+    const int most = __reduce_max_sync(0xffffffffu, nv);
+    for (int v = most - 1; v >= 0; v--) {
+      int mkey = -1, tkey = -1;
+      float da[3] = {0.f, 0.f, 0.f}, dr = 0.0f, de[3] = {0.f, 0.f, 0.f};
+      if (v < nv) {
+        const size_t at = (size_t)v * D.n + i;
+        const float4 r0 = __ldcs(D.rec[0] + at);
+        if (__float_as_int(r0.w) != REC_SKIP) {
+          const float4 r1 = __ldcs(D.rec[1] + at), r2 = __ldcs(D.rec[2] + at), r3 = __ldcs(D.rec[3] + at),
+                       r4 = __ldcs(D.rec[4] + at), r5 = __ldcs(D.rec[5] + at);
+          mkey = __float_as_int(r0.w);
+          tkey = __float_as_int(r4.w);
+          const float T[3] = {r0.x, r0.y, r0.z}, Pv[3] = {r1.x, r1.y, r1.z}, dPr[3] = {r2.x, r2.y, r2.z},
+                      S[3] = {r3.x, r3.y, r3.z}, dSr[3] = {r4.x, r4.y, r4.z}, E[3] = {r5.x, r5.y, r5.z};
 #pragma unroll
-      for (int c = 0; c < 3; c++) {
-        const float se = group_sum(0xffffffffu, tkey, tkey >= 0 ? V[v].QE[c] : 0.0f, lead);
-        if (lead && tkey >= 0 && se != 0.0f) atomicAdd(g_env + 3 * (size_t)tkey + c, (double)se);
+          for (int c = 0; c < 3; c++) {
+            const float gt = g[c] * T[c];
+            da[c] = gt * (r2.w * E[c] + r1.w * L[c]);
+            dr += gt * (dSr[c] * E[c] + dPr[c] * L[c]);
+            de[c] = gt * S[c];
+            L[c] = S[c] * E[c] + Pv[c] * L[c];
+          }
+        }
       }
+      const uint32_t lane = threadIdx.x & 31u;
+      const unsigned mp = __match_any_sync(0xffffffffu, mkey);
+      if (mkey >= 0) {
+        const float s0 = group_sum(mp, da[0]), s1 = group_sum(mp, da[1]), s2 = group_sum(mp, da[2]),
+                    s3 = group_sum(mp, dr);
+        if ((int)lane == __ffs(mp) - 1) {
+          atomicAdd(&spart[4 * mkey + 0], s0);
+          atomicAdd(&spart[4 * mkey + 1], s1);
+          atomicAdd(&spart[4 * mkey + 2], s2);
+          atomicAdd(&spart[4 * mkey + 3], s3);
+        }
+      }
+      __syncwarp();
+      const unsigned tp = __match_any_sync(0xffffffffu, tkey);
+      if (tkey >= 0) {
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const float se = group_sum(tp, de[c]);
+          if ((int)lane == __ffs(tp) - 1 && se != 0.0f) atomicAdd(g_env + 3 * (size_t)tkey + c, (double)se);
+        }
+      }
+      __syncwarp();
     }
   }
   __syncthreads();
@@ -520,7 +579,16 @@ __global__ void __launch_bounds__(DIFF_THREADS, PK_DIFF_ADJ_BLOCKS) k_diff_adjoi
       else atomicAdd(g_albedo + 3 * (i >> 2) + (i & 3u), (double)v);
     }
   }
-  if (live) atomicAdd(rays, (unsigned long long)nrays);
+}
+
+// After a chunk: its rays.  After the last: status and ray count for the host.
+__global__ void k_path_end(PathCount* c, PathTotal* t, int depth, uint32_t* host) {
+  unsigned long long r = t->rays;
+  for (int b = 0; b < depth; b++) r += (unsigned long long)c->rays[b] + c->shadow[b];
+  t->rays = r;
+  host[0] = t->err;
+  host[1] = (uint32_t)(r & 0xffffffffu);
+  host[2] = (uint32_t)(r >> 32);
 }
 
 namespace {
@@ -554,22 +622,74 @@ EnvDev diff_env_dev(pk_ctx* c) {
                 (int)c->diff_env_nb, 1, nullptr};
 }
 
-// Runs the launch, waits, reads the error flag and the ray count.
-template <class F>
-int diff_run(pk_ctx* c, const char* what, F launch) {
-  DevBuf<uint32_t> err(1);
-  DevBuf<unsigned long long> rays(1);
-  check(cudaMemsetAsync(err.p, 0, 4, c->stream), "memset");
-  check(cudaMemsetAsync(rays.p, 0, 8, c->stream), "memset");
-  launch(err.p, rays.p);
-  check(cudaGetLastError(), what);
-  uint32_t herr = 0;
-  unsigned long long hr = 0;
-  check(cudaMemcpyAsync(&herr, err.p, 4, cudaMemcpyDeviceToHost, c->stream), "D2H");
-  check(cudaMemcpyAsync(&hr, rays.p, 8, cudaMemcpyDeviceToHost, c->stream), "D2H");
-  check(cudaStreamSynchronize(c->stream), "sync");
-  c->diff_rays = hr;
-  if (herr) {
+// Paths per chunk: enough to fill the GPU many times over (the tail of a
+// bounce's longest rays costs as much as some 10^5 rays), within PATH_SPACE
+// bytes of workspace that the context keeps.
+constexpr unsigned long long PATH_CHUNK = 1ull << 22;
+constexpr unsigned long long PATH_SPACE = 3ull << 30;
+
+// Renders every path (REC: recording vertices) chunk by chunk; after(D, first,
+// last) turns a chunk into its part of the result.
+template <bool REC, class F>
+int run_paths(pk_ctx* c, const char* what, const DiffParams& P, F after) {
+  const cudaStream_t st = c->stream;
+  const uint32_t npix = c->W * c->H;
+  const unsigned long long total = (unsigned long long)npix * (unsigned long long)P.spp;
+  const unsigned long long per = 9 * 16 + 16 + 4 + (unsigned long long)P.depth * 16 * (REC ? 6 : 1);
+  const unsigned long long chunk = std::min(std::min(total, PATH_CHUNK), PATH_SPACE / per);
+  const size_t n = (size_t)chunk, head = 512;
+  static_assert(sizeof(PathCount) + sizeof(PathTotal) <= 512, "header");
+  const size_t need = head + n * (size_t)per + 64;
+  if (c->diff_space.cap < need) c->diff_space.alloc(need);  // grows, at most to PATH_SPACE; goes with the context
+  unsigned char* at = c->diff_space.p;
+  auto take = [&](size_t bytes) {
+    unsigned char* p = at;
+    at += (bytes + 15) / 16 * 16;
+    return p;
+  };
+  PathDev D{};
+  D.total = reinterpret_cast<PathTotal*>(at);
+  D.count = reinterpret_cast<PathCount*>(at + sizeof(PathTotal));
+  at += head;
+  for (int b = 0; b < 2; b++) {
+    D.o[b] = reinterpret_cast<float4*>(take(16 * n));
+    D.d[b] = reinterpret_cast<float4*>(take(16 * n));
+    D.t[b] = reinterpret_cast<float4*>(take(16 * n));
+  }
+  D.so = reinterpret_cast<float4*>(take(16 * n));
+  D.sd = reinterpret_cast<float4*>(take(16 * n));
+  D.st = reinterpret_cast<float4*>(take(16 * n));
+  D.hit = reinterpret_cast<uint4*>(take(16 * n));
+  if (REC)
+    for (int k = 0; k < 6; k++) D.rec[k] = reinterpret_cast<float4*>(take(16 * n * (size_t)P.depth));
+  else
+    D.add = reinterpret_cast<float4*>(take(16 * n * (size_t)P.depth));
+  D.lived = take(n);
+  const SceneDev sc = c->dropin_scene();
+  const EnvDev env = diff_env_dev(c);
+  check(cudaMemsetAsync(D.total, 0, sizeof(PathTotal), st), "memset");
+  for (unsigned long long first = 0; first < total; first += chunk) {
+    D.n = (uint32_t)std::min(chunk, total - first);
+    const bool last = first + chunk >= total;
+    const ViewDev V{c->cam_host, c->theta_next, c->W, c->H, first};
+    check(cudaMemsetAsync(D.count, 0, sizeof(PathCount), st), "memset");
+    const unsigned blocks = (D.n + PATH_THREADS - 1) / PATH_THREADS;
+    const unsigned lanes = std::min((unsigned)c->sms * LANES_BLOCKS, blocks);
+    const unsigned shade = std::min((unsigned)c->sms * 4 * PK_PATH_SHADE_BLOCKS, blocks);
+    k_path_camera<<<blocks, PATH_THREADS, 0, st>>>(D, V, P.sample_base);
+    for (int b = 0; b < P.depth; b++) {
+      k_path_trace<<<lanes, TRACE_THREADS, 0, st>>>(sc, D, b);
+      k_path_shade<REC><<<shade, PATH_THREADS, 0, st>>>(sc, env, P, D, V, b);
+      k_path_shadow<REC><<<lanes, TRACE_THREADS, 0, st>>>(sc, P, D, V.theta, b);
+    }
+    after(D, first, last);
+    k_path_end<<<1, 1, 0, st>>>(D.count, D.total, P.depth, c->host_words_dev);
+    check(cudaGetLastError(), what);
+  }
+  check(cudaStreamSynchronize(st), "sync");
+  const volatile uint32_t* h = c->host_words;
+  c->diff_rays = (unsigned long long)h[1] | ((unsigned long long)h[2] << 32);
+  if (h[0]) {
     c->err = std::string(what) + ": device error flags (traversal stack)";
     return PK_ERR_DEVICE;
   }
@@ -639,11 +759,12 @@ extern "C" int pk_diff_render(pk_ctx* c, const pk_diff_params* p, float* image4)
     const int rc = diff_check(c, p, dp);
     if (rc != PK_OK) return rc;
     if (!image4) return diff_fail(c, PK_ERR_ARG, "pk_diff_render: null image");
-    const uint32_t n = c->W * c->H;
-    return diff_run(c, "pk_diff_render", [&](uint32_t* err, unsigned long long* rays) {
-      k_diff_forward<<<(n + DIFF_THREADS - 1) / DIFF_THREADS, DIFF_THREADS, 0, c->stream>>>(
-          c->dropin_scene(), diff_env_dev(c), c->cam_host, dp, c->theta_next, c->W, c->H,
-          reinterpret_cast<float4*>(image4), err, rays);
+    const uint32_t npix = c->W * c->H;
+    float4* image = reinterpret_cast<float4*>(image4);
+    const float inv = 1.0f / (float)dp.spp;
+    return run_paths<false>(c, "pk_diff_render", dp, [&](const PathDev& D, unsigned long long first, bool last) {
+      k_path_sum<<<(npix + PATH_THREADS - 1) / PATH_THREADS, PATH_THREADS, 0, c->stream>>>(D, first, npix, image, inv,
+                                                                                           last ? 1 : 0);
     });
   } catch (CudaError& e) {
     c->err = e.what();
@@ -661,14 +782,14 @@ extern "C" int pk_diff_backward(pk_ctx* c, const pk_diff_params* p, const float*
     if (rc != PK_OK) return rc;
     if (!d_image4 || !g_albedo3 || !g_roughness || !g_env_rgb)
       return diff_fail(c, PK_ERR_ARG, "pk_diff_backward: null buffer");
-    const uint32_t n = c->W * c->H;
+    const uint32_t npix = c->W * c->H;
     const size_t smem = 16 * (size_t)p->n_mats;
     if (smem > 48 * 1024)
-      check(cudaFuncSetAttribute(k_diff_adjoint, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "attr");
-    return diff_run(c, "pk_diff_backward", [&](uint32_t* err, unsigned long long* rays) {
-      k_diff_adjoint<<<(n + DIFF_THREADS - 1) / DIFF_THREADS, DIFF_THREADS, smem, c->stream>>>(
-          c->dropin_scene(), diff_env_dev(c), c->cam_host, dp, c->theta_next, c->W, c->H,
-          reinterpret_cast<const float4*>(d_image4), g_albedo3, g_roughness, g_env_rgb, err, rays);
+      check(cudaFuncSetAttribute(k_path_sweep, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "attr");
+    return run_paths<true>(c, "pk_diff_backward", dp, [&](const PathDev& D, unsigned long long first, bool) {
+      const unsigned per = SWEEP_THREADS * SWEEP_PATHS;
+      k_path_sweep<<<(D.n + per - 1) / per, SWEEP_THREADS, smem, c->stream>>>(
+          dp, D, first, npix, reinterpret_cast<const float4*>(d_image4), g_albedo3, g_roughness, g_env_rgb);
     });
   } catch (CudaError& e) {
     c->err = e.what();

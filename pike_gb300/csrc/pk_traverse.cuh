@@ -180,4 +180,113 @@ __device__ __forceinline__ void traverse(const SceneDev& sc, float ox, float oy,
                                     ntest);
 }
 
+// Persistent lanes over n rays, for kernels of TRACE_THREADS threads.  A lane
+// owns one ray at a time; when at least LANES_REFILL lanes of a warp are idle
+// they claim new rays together from `ticket` (zero at launch), and a lane takes
+// at most LANES_BUDGET inner steps before the warp meets again, so no lane
+// waits for the longest of a fixed group of 32 rays.  No speculation: each ray
+// visits the nodes and leaves of trace.wgsl's (trace_shadow.wgsl's) loop in its
+// order.  WHOLE: an any-hit ray tests the leaf it hits in to its end, for
+// callers that want the triangle; otherwise it stops at the first accepted one.
+// load(j, o, d) fetches ray j; done(j, d, t, triangle, barycentrics) takes the
+// result (triangle -1: none).
+// (Threshold, budget, stack split and leaf unroll as measured for the frame's
+// traversal, k_trace_dyn.)
+constexpr int LANES_REFILL = 16;
+constexpr int LANES_BUDGET = 8;
+constexpr int LANES_SMEM = 8;  // stack entries per lane in shared memory, the rest of 64 in local memory
+constexpr int LANES_LOCAL = 64 - LANES_SMEM;
+constexpr int LANES_BLOCKS = 10;  // resident blocks per SM (48 registers)
+
+template <bool ANY, bool WHOLE, class Load, class Done>
+__device__ __forceinline__ void trace_lanes(const SceneDev& sc, uint32_t n, uint32_t* __restrict__ ticket,
+                                            uint32_t* err, int (*sstack)[TRACE_THREADS], Load load, Done done) {
+  int lstack[LANES_LOCAL];
+  const int lane = threadIdx.x & 31, tid = threadIdx.x;
+  const uint32_t ltmask = (1u << lane) - 1u;
+  const float eps = ANY ? 1e-7f : 1e-8f;
+  uint32_t j = 0;
+  bool have = false, exhausted = false;
+  float ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f, ix = 0.f, iy = 0.f, iz = 0.f;
+  float best_t = MAX_T;
+  int best_i = -1;
+  uint32_t best_b = 0u;
+  int sp = 0, cur = 0;
+  for (;;) {
+    const uint32_t idle = __ballot_sync(0xffffffffu, !have && !exhausted);
+    const uint32_t busy = __ballot_sync(0xffffffffu, have);
+    if (idle && (__popc(idle) >= LANES_REFILL || busy == 0u)) {
+      const int leader = __ffs(idle) - 1;
+      uint32_t base = 0;
+      if (lane == leader) base = atomicAdd(ticket, (uint32_t)__popc(idle));
+      base = __shfl_sync(0xffffffffu, base, leader);
+      if (!have && !exhausted) {
+        j = base + (uint32_t)__popc(idle & ltmask);
+        if (j < n) {
+          float4 o, d;
+          load(j, o, d);
+          ox = o.x; oy = o.y; oz = o.z;
+          dx = d.x; dy = d.y; dz = d.z;
+          ix = 1.0f / dx; iy = 1.0f / dy; iz = 1.0f / dz;
+          best_t = MAX_T; best_i = -1; best_b = 0u;
+          sp = 0;
+          cur = sc.root;
+          have = true;
+        } else {
+          exhausted = true;
+        }
+      }
+    }
+    if (!__any_sync(0xffffffffu, have)) break;
+    if (!have) continue;
+    bool fin = false;
+    int budget = LANES_BUDGET;
+    while (cur >= 0 && budget-- > 0) {
+      float lh, rh;
+      int cl, cr;
+      inner_children(sc, cur, ox, oy, oz, ix, iy, iz, lh, rh, cl, cr);
+      const bool lok = lh < best_t, rok = rh < best_t;
+      if (lok && rok) {
+        int nearc, farc;
+        if (lh > rh) { nearc = cr; farc = cl; } else { nearc = cl; farc = cr; }
+        if (sp < LANES_SMEM) sstack[sp][tid] = farc;
+        else if (sp < LANES_SMEM + LANES_LOCAL) lstack[sp - LANES_SMEM] = farc;
+        else { atomicOr(err, ERR_STACK); fin = true; break; }
+        ++sp;
+        cur = nearc;
+        continue;
+      }
+      if (lok) { cur = cl; continue; }
+      if (rok) { cur = cr; continue; }
+      if (sp == 0) { fin = true; break; }
+      --sp;
+      cur = sp < LANES_SMEM ? sstack[sp][tid] : lstack[sp - LANES_SMEM];
+    }
+    while (!fin && cur < 0) {
+      const uint32_t word = (uint32_t)cur & 0x7fffffffu;
+      const int size = (int)(word >> 24);
+      const int base = (int)(word & 0x00ffffffu);
+#pragma unroll 4
+      for (int i = 0; i < size; i++) {
+        float res, u, v;
+        if (!mt_test(sc, base + i, ox, oy, oz, dx, dy, dz, eps, res, u, v)) continue;
+        if (res < best_t) {
+          best_t = res;
+          best_i = base + i;
+          best_b = pack_unorm16(u) | (pack_unorm16(v) << 16);
+        }
+        if (ANY && !WHOLE && best_i != -1) break;
+      }
+      if (ANY && best_i != -1) { fin = true; break; }
+      if (sp == 0) { fin = true; break; }
+      --sp;
+      cur = sp < LANES_SMEM ? sstack[sp][tid] : lstack[sp - LANES_SMEM];
+    }
+    if (fin) {
+      done(j, dx, dy, dz, best_t, best_i, best_b);
+      have = false;
+    }
+  }
+}
+
 }  // namespace pk
