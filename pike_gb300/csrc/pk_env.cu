@@ -1,13 +1,16 @@
 // pk_env.cu -- EnvironmentGenerator tables (render/env_sampler.js:43-157):
 // per-texel radiance, stable sort by descending radiance, equal-mass luminance
-// bins and the per-texel pdf; and PK_ENV_ALIAS's alias table.  The total
-// radiance (row-major sum) and the bin walk (a running sum reset at every bin)
-// are sequentially rounded double sums in the reference, so they are one
-// chain of dependent FP64 additions each.  On GB300 a chain of FP64 additions
-// on one GPU lane runs about a hundred times slower than on a Grace core
-// (2048x1024: 380 ms for the tables with both walks on one warp), so the two
-// walks run on the host over the radiance the GPU computed; the radiance, the
-// sort, the pdf texture and the coordinates stay on the GPU.
+// bins and the per-texel pdf; and PK_ENV_ALIAS's alias table.
+//
+// The total radiance (row-major sum) and the bin walk (a running sum reset at
+// every bin) are sequentially rounded double sums in the reference: one chain of
+// dependent FP64 additions each.  Their values never leave this file, only the
+// bins they decide, so the GPU decides them from prefix sums with a bound on how
+// far the sequential sums can lie from them (k_env_next); a map where a bin's
+// edge falls within the bound, or whose sums are not finite, takes the walks
+// themselves on the host (walk_bins), as every map did before (a constant map is
+// one).  2048x1024, upload and build: 12.7 ms with the walks, of which the kernels
+// were 0.5 ms; 1.04 ms without.
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -51,11 +54,85 @@ __global__ void k_env_radiance_f32(const float* __restrict__ rgb, uint32_t n, do
   vals[i] = i;
 }
 
+// ---- the luminance bins ------------------------------------------------------
+// Radiance is not negative, so the sum of m doubles added one after the other
+// lies within (m - 1) 2^-53 (relative) of their exact sum, and so do the prefix
+// sums below with their 64 additions or fewer each.  With P the prefix sums of
+// the sorted radiance, T the total, nb the number of bins and B = T / nb the bin
+// size, the sequential sum from position i to before position k lies within
+//   tol = 2^-53 T (4 (n + 4096) / nb + 512)
+// of P(k) - P(i) even after the reference's own error in B (each of the three
+// terms counted at least twice): the walk's bin that starts at i ends at the
+// first k with P(k) - P(i) >= B - tol, if that difference is also >= B + tol.
+struct EnvPlan {
+  double total, bin, tol;
+  uint32_t status;  // 0: decided; 1: the walk has to decide
+  uint32_t nb;      // bins made
+  uint32_t err, pad;
+};
+constexpr uint32_t ENV_MAX_BINS = 1024;
+
+// total: the sum of all (after the prefix sums); sorted[0]: complemented bits of the largest.
+__global__ void k_env_plan(const double* __restrict__ prefix, const unsigned long long* __restrict__ sorted, uint32_t n,
+                           EnvPlan* __restrict__ plan) {
+  const double u = 1.1102230246251565e-16;  // 2^-53
+  const double brightest = __longlong_as_double((long long)~sorted[0]);
+  const double total = prefix[n - 1] + __longlong_as_double((long long)~sorted[n - 1]);
+  const double rel = ((double)n + 256.0) * 2.0 * u;
+  plan->nb = 0;
+  plan->total = total;
+  plan->status = 1;
+  if (!(total > 0.0) || !isfinite(total) || !(brightest > 0.0)) return;
+  // numBins = min(256, max(32, 2 * ceil(total / brightest)))
+  const double lo = fmin(256.0, fmax(32.0, 2.0 * ceil(total * (1.0 - rel) / brightest)));
+  const double hi = fmin(256.0, fmax(32.0, 2.0 * ceil(total * (1.0 + rel) / brightest)));
+  if (lo != hi) return;
+  plan->bin = total / lo;
+  plan->tol = u * total * (4.0 * ((double)n + 4096.0) / lo + 512.0);
+  plan->status = 0;
+}
+
+// For every position i, where a bin that starts there ends: a binary search.
+// Bit 31: undecided.  n: the bin is the last.
+__global__ void k_env_next(const double* __restrict__ prefix, uint32_t n, const EnvPlan* __restrict__ plan,
+                           uint32_t* __restrict__ next) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n || plan->status) return;
+  const double from = prefix[i], want = plan->bin - plan->tol;
+  uint32_t lo = i + 1, hi = n;  // first k in (i, n) with P(k) - P(i) >= B - tol, else n
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (prefix[mid] - from >= want) hi = mid; else lo = mid + 1;
+  }
+  next[i] = lo < n && !(prefix[lo] - from >= plan->bin + plan->tol) ? lo | 0x80000000u : lo;
+}
+
+// createLuminanceHistogram (env_sampler.js:74-94): bin after bin.
+__global__ void k_env_chain(const uint32_t* __restrict__ next, uint32_t n, EnvPlan* __restrict__ plan,
+                            int2* __restrict__ bins) {
+  if (plan->status) return;
+  uint32_t i = 0, nb = 0;
+  while (i < n) {
+    const uint32_t k = next[i];
+    if ((k & 0x80000000u) || nb >= ENV_MAX_BINS) { plan->status = 1; return; }
+    bins[nb++] = make_int2((int)i, (int)k);
+    i = k;
+  }
+  plan->nb = nb;
+}
+
+// The doubles behind the sorted keys.
+__global__ void k_env_sorted(const unsigned long long* __restrict__ keys, uint32_t n, double* __restrict__ out) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < n) out[i] = __longlong_as_double((long long)~keys[i]);
+}
+
 // createPdfTexture / createEnvCoordBuffer (env_sampler.js:104-157).
 __global__ void k_env_pdf(const uint32_t* __restrict__ order, uint32_t n, uint32_t w, const int2* __restrict__ bins,
-                          uint32_t nb, int2* __restrict__ coords, float* __restrict__ pdf) {
+                          const EnvPlan* __restrict__ plan, int2* __restrict__ coords, float* __restrict__ pdf) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= n) return;
+  const uint32_t nb = plan->nb;
+  if (i >= n || nb == 0) return;
   uint32_t lo = 0, hi = nb;  // the bin holding sorted position i
   while (hi - lo > 1) {
     const uint32_t mid = (lo + hi) / 2;
@@ -234,26 +311,10 @@ double js_max(double a, double b) { return (a != a || b != b) ? NAN : (a > b ? a
 
 namespace {
 
-// The tables from per-texel radiance `rad` with sort keys and values already
-// set (the radiance kernels above).
-int build_from_radiance(const Scratch& sc, uint32_t w, uint32_t h, TmpBuf<double>& rad,
-                        TmpBuf<unsigned long long>& keys, TmpBuf<uint32_t>& vals, DevBuf<int2>& bins_out,
-                        uint32_t& nb_out, DevBuf<int2>& coords_out, DevBuf<float>& pdf_out, std::string& why) {
-  const cudaStream_t s = sc.s;
-  const uint32_t n = w * h;
-  TmpBuf<unsigned long long> keys_tmp(sc, n);
-  TmpBuf<uint32_t> vals_tmp(sc, n), err(sc, 1);
-  check(cudaMemsetAsync(err.p, 0, 4, s), "memset");
-  std::vector<double> r(n);
-  check(cudaMemcpyAsync(r.data(), rad.p, (size_t)n * 8, cudaMemcpyDeviceToHost, s), "D2H");
-  radix_sort_pairs_u64(sc, reinterpret_cast<uint64_t*>(keys.p), vals.p, reinterpret_cast<uint64_t*>(keys_tmp.p),
-                       vals_tmp.p, n, 1, err.p);
-  uint32_t herr = 0;
-  check(cudaMemcpyAsync(&herr, err.p, 4, cudaMemcpyDeviceToHost, s), "D2H");
-  std::vector<uint32_t> order(n);
-  check(cudaMemcpyAsync(order.data(), vals.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s), "D2H");
-  check(cudaStreamSynchronize(s), "sync");
-  if (herr) { why = "radix sort look-back timed out"; return 1; }
+// The reference's two sums on the host, for the maps the GPU leaves undecided.
+int walk_bins(const std::vector<double>& r, const std::vector<uint32_t>& order, std::vector<int2>& bins,
+              std::string& why) {
+  const uint32_t n = (uint32_t)r.size();
   // totalRadiance += rad (row-major) and brightestTexel = max(rad, brightest)
   double total = 0.0, brightest = 0.0;
   for (uint32_t i = 0; i < n; i++) {
@@ -266,7 +327,6 @@ int build_from_radiance(const Scratch& sc, uint32_t w, uint32_t h, TmpBuf<double
   const double bin_size = total / num_bins;
   // createLuminanceHistogram (env_sampler.js:74-94): walk the sorted texels,
   // closing a bin when the running sum reaches binSize, then resetting it.
-  std::vector<int2> bins;
   double current = 0.0;
   int32_t prev = 0;
   for (uint32_t k = 0; k < n; k++) {
@@ -278,17 +338,62 @@ int build_from_radiance(const Scratch& sc, uint32_t w, uint32_t h, TmpBuf<double
     current = current + r[order[k]];
   }
   bins.push_back(make_int2(prev, (int)n));
-  const uint32_t nbh = (uint32_t)bins.size();
-  if (nbh < 2) { why = "environment yields a single luminance bin"; return 1; }
-  if (nbh > 1024) { why = "too many luminance bins"; return 1; }
-  bins_out.alloc(nbh);
-  check(cudaMemcpyAsync(bins_out.p, bins.data(), (size_t)nbh * 8, cudaMemcpyHostToDevice, s), "H2D");
+  return 0;
+}
+
+// The tables from per-texel radiance `rad` with sort keys and values already
+// set (the radiance kernels above).
+int build_from_radiance(const Scratch& sc, uint32_t w, uint32_t h, TmpBuf<double>& rad,
+                        TmpBuf<unsigned long long>& keys, TmpBuf<uint32_t>& vals, DevBuf<int2>& bins_out,
+                        uint32_t& nb_out, DevBuf<int2>& coords_out, DevBuf<float>& pdf_out, std::string& why) {
+  const cudaStream_t s = sc.s;
+  const uint32_t n = w * h, grid = (n + 255) / 256;
+  TmpBuf<EnvPlan> plan(sc, 1);
+  check(cudaMemsetAsync(plan.p, 0, sizeof(EnvPlan), s), "memset");
+  {
+    TmpBuf<unsigned long long> keys_tmp(sc, n);
+    TmpBuf<uint32_t> vals_tmp(sc, n);
+    radix_sort_pairs_u64(sc, reinterpret_cast<uint64_t*>(keys.p), vals.p, reinterpret_cast<uint64_t*>(keys_tmp.p),
+                         vals_tmp.p, n, 1, &plan.p->err);
+  }
+  TmpBuf<int2> bins(sc, ENV_MAX_BINS);
+  {
+    TmpBuf<double> prefix(sc, n);
+    TmpBuf<uint32_t> next(sc, n);
+    k_env_sorted<<<grid, 256, 0, s>>>(keys.p, n, prefix.p);
+    scan_exclusive_f64(sc, prefix.p, prefix.p, n);
+    k_env_plan<<<1, 1, 0, s>>>(prefix.p, keys.p, n, plan.p);
+    k_env_next<<<grid, 256, 0, s>>>(prefix.p, n, plan.p, next.p);
+    k_env_chain<<<1, 1, 0, s>>>(next.p, n, plan.p, bins.p);
+  }
   coords_out.alloc(n);
   pdf_out.alloc(n);
-  k_env_pdf<<<(n + 255) / 256, 256, 0, s>>>(vals.p, n, w, bins_out.p, nbh, coords_out.p, pdf_out.p);
-  check(cudaGetLastError(), "env pdf");
-  check(cudaStreamSynchronize(s), "sync");  // the host vectors are freed on return
-  nb_out = nbh;
+  k_env_pdf<<<grid, 256, 0, s>>>(vals.p, n, w, bins.p, plan.p, coords_out.p, pdf_out.p);
+  check(cudaGetLastError(), "env tables");
+  EnvPlan host;
+  check(cudaMemcpyAsync(&host, plan.p, sizeof host, cudaMemcpyDeviceToHost, s), "D2H");
+  check(cudaStreamSynchronize(s), "sync");
+  if (host.err) { why = "radix sort look-back timed out"; return 1; }
+  if (host.status) {
+    std::vector<double> r(n);
+    std::vector<uint32_t> order(n);
+    std::vector<int2> walked;
+    check(cudaMemcpyAsync(r.data(), rad.p, (size_t)n * 8, cudaMemcpyDeviceToHost, s), "D2H");
+    check(cudaMemcpyAsync(order.data(), vals.p, (size_t)n * 4, cudaMemcpyDeviceToHost, s), "D2H");
+    check(cudaStreamSynchronize(s), "sync");
+    if (walk_bins(r, order, walked, why)) return 1;
+    host.nb = (uint32_t)walked.size();
+    if (host.nb > ENV_MAX_BINS) { why = "too many luminance bins"; return 1; }
+    check(cudaMemcpyAsync(bins.p, walked.data(), (size_t)host.nb * 8, cudaMemcpyHostToDevice, s), "H2D");
+    check(cudaMemcpyAsync(plan.p, &host, sizeof host, cudaMemcpyHostToDevice, s), "H2D");
+    k_env_pdf<<<grid, 256, 0, s>>>(vals.p, n, w, bins.p, plan.p, coords_out.p, pdf_out.p);
+    check(cudaGetLastError(), "env pdf");
+  }
+  if (host.nb < 2) { why = "environment yields a single luminance bin"; return 1; }
+  bins_out.alloc(host.nb);
+  check(cudaMemcpyAsync(bins_out.p, bins.p, (size_t)host.nb * 8, cudaMemcpyDeviceToDevice, s), "D2D");
+  check(cudaStreamSynchronize(s), "sync");
+  nb_out = host.nb;
   return 0;
 }
 

@@ -90,41 +90,45 @@ void scan_exclusive_u32(const Scratch& w, const uint32_t* in, uint32_t* out, uin
   check(cudaGetLastError(), "k_scan_u32");
 }
 
-// ---------------- exclusive scan of u64 values (three phases) ---------------
+// ---------------- exclusive scan of 64-bit values (three phases) -------------
 // Tiles of SCAN_TILE values: each block scans its tile and writes the tile's
 // sum; the tile sums are scanned recursively; a last pass adds each tile's
-// offset.  Integer sums, so the result does not depend on the grouping.
-__device__ __forceinline__ unsigned long long warp_scan_incl_u64(unsigned long long v) {
+// offset.  Integer sums do not depend on the grouping; a double prefix is the
+// result of at most 8 + 5 + 8 + 1 additions per level.
+template <class T>
+__device__ __forceinline__ T warp_scan_incl(T v) {
   const int lane = threadIdx.x & 31;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
-    const unsigned long long x = __shfl_up_sync(0xffffffffu, v, o);
+    const T x = __shfl_up_sync(0xffffffffu, v, o);
     if (lane >= o) v += x;
   }
   return v;
 }
 
-__global__ void __launch_bounds__(SCAN_THREADS) k_scan_u64_tiles(const unsigned long long* in,
-                                                                unsigned long long* out, size_t n,
-                                                                unsigned long long* __restrict__ tile_sums) {
-  __shared__ unsigned long long s_warp[SCAN_THREADS / 32];
+template <class T>
+__global__ void __launch_bounds__(SCAN_THREADS) k_scan64_tiles(const T* in, T* out, size_t n,
+                                                               T* __restrict__ tile_sums) {
+  __shared__ T s_warp[SCAN_THREADS / 32];
   const size_t base = (size_t)blockIdx.x * SCAN_TILE + (size_t)threadIdx.x * SCAN_ITEMS;
-  unsigned long long v[SCAN_ITEMS], sum = 0;
+  T v[SCAN_ITEMS], sum = 0;
 #pragma unroll
   for (int k = 0; k < SCAN_ITEMS; k++) {
-    v[k] = base + k < n ? in[base + k] : 0ull;
+    v[k] = base + k < n ? in[base + k] : (T)0;
     sum += v[k];
   }
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const unsigned long long incl = warp_scan_incl_u64(sum);
+  const T incl = warp_scan_incl(sum);
+  T excl = __shfl_up_sync(0xffffffffu, incl, 1);  // no subtraction: a double prefix stays a sum of what it covers
+  if (lane == 0) excl = 0;
   if (lane == 31) s_warp[warp] = incl;
   __syncthreads();
-  unsigned long long woff = 0, tot = 0;
+  T woff = 0, tot = 0;
   for (int k = 0; k < SCAN_THREADS / 32; k++) {
     if (k < warp) woff += s_warp[k];
     tot += s_warp[k];
   }
-  unsigned long long run = woff + incl - sum;
+  T run = woff + excl;
 #pragma unroll
   for (int k = 0; k < SCAN_ITEMS; k++) {
     if (base + k < n) out[base + k] = run;
@@ -133,23 +137,29 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_u64_tiles(const unsigned 
   if (threadIdx.x == 0) tile_sums[blockIdx.x] = tot;
 }
 
-__global__ void k_scan_u64_add(unsigned long long* out, size_t n, const unsigned long long* __restrict__ tile_offs) {
+template <class T>
+__global__ void k_scan64_add(T* out, size_t n, const T* __restrict__ tile_offs) {
   const size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (i < n) out[i] += tile_offs[i / SCAN_TILE];
 }
 
-void scan_exclusive_u64(const Scratch& w, const unsigned long long* in, unsigned long long* out, size_t n) {
+template <class T>
+static void scan64(const Scratch& w, const T* in, T* out, size_t n) {
   if (n == 0) return;
   const size_t ntiles = (n + SCAN_TILE - 1) / SCAN_TILE;
-  TmpBuf<unsigned long long> sums(w, ntiles);
-  k_scan_u64_tiles<<<(unsigned)ntiles, SCAN_THREADS, 0, w.s>>>(in, out, n, sums.p);
-  check(cudaGetLastError(), "k_scan_u64_tiles");
+  TmpBuf<T> sums(w, ntiles);
+  k_scan64_tiles<T><<<(unsigned)ntiles, SCAN_THREADS, 0, w.s>>>(in, out, n, sums.p);
+  check(cudaGetLastError(), "k_scan64_tiles");
   if (ntiles > 1) {
-    scan_exclusive_u64(w, sums.p, sums.p, ntiles);
-    k_scan_u64_add<<<(unsigned)((n + 255) / 256), 256, 0, w.s>>>(out, n, sums.p);
-    check(cudaGetLastError(), "k_scan_u64_add");
+    scan64<T>(w, sums.p, sums.p, ntiles);
+    k_scan64_add<T><<<(unsigned)((n + 255) / 256), 256, 0, w.s>>>(out, n, sums.p);
+    check(cudaGetLastError(), "k_scan64_add");
   }
 }
+void scan_exclusive_u64(const Scratch& w, const unsigned long long* in, unsigned long long* out, size_t n) {
+  scan64<unsigned long long>(w, in, out, n);
+}
+void scan_exclusive_f64(const Scratch& w, const double* in, double* out, size_t n) { scan64<double>(w, in, out, n); }
 
 // ---------------- stable LSD radix sort -------------------------------------
 // One kernel per 8-bit digit (after Adinets & Merrill, "Onesweep: A Faster

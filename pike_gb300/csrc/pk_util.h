@@ -110,6 +110,11 @@ void scan_exclusive_u32(const Scratch& w, const uint32_t* in, uint32_t* out, uin
 // Exclusive prefix sum of n u64 values (in may alias out); enqueues and returns.
 void scan_exclusive_u64(const Scratch& w, const unsigned long long* in, unsigned long long* out, size_t n);
 
+// Exclusive prefix sum of n doubles that are not negative (in may alias out);
+// enqueues and returns.  For n < 2^33 every prefix is the result of at most 64
+// additions, so it lies within 64 * 2^-53 (relative) of the exact sum.
+void scan_exclusive_f64(const Scratch& w, const double* in, double* out, size_t n);
+
 // Stable LSD radix sort of `segs` arrays of n (64-bit key, 32-bit value) pairs
 // each, array k at keys + k * n and vals + k * n, ascending, in place using
 // scratch arrays of the same size.  Enqueues and returns; errors as above.
