@@ -856,9 +856,9 @@ int pk_postprocess(pk_ctx* c) {
 // the next bounce's compaction; that bounce's closest-hit misses are parked
 // in their hit records and added by the compaction, so every pixel still
 // receives its contributions in the serial order (shadow of bounce b before
-// the miss of bounce b+1).  `tail`: accumulate, postprocess and the sample
-// count too (frames in flight issue those outside, ordered across slots).
-static void render_frame_launches(pk_ctx* c, int k, cudaStream_t st, uint32_t bounces, bool tail) {
+// the miss of bounce b+1).  What the frame starts from (state, counts, tickets,
+// look-back states) and its accumulation are launched outside.
+static void render_frame_launches(pk_ctx* c, int k, cudaStream_t st, uint32_t bounces) {
   FrameSlot& fs = c->slot[k];
   LaunchCtx L = c->launch(k, st);
   // PK_OVERLAP_AUTO: overlap when frames render one at a time or are small
@@ -888,13 +888,9 @@ static void render_frame_launches(pk_ctx* c, int k, cudaStream_t st, uint32_t bo
   // tick() renders W*H pixels in batches of BATCH_SIZE (pk_configure's batch;
   // pike.js:133-154), each with its own counters, camera offset and bounces.
   const uint32_t nbatch = (uint32_t)(((uint64_t)c->npix + c->B - 1) / c->B);
-  const uint64_t steps = (uint64_t)nbatch * bounces;
-  const uint32_t nb = (uint32_t)std::min<uint64_t>(steps, MAX_BOUNCES);
-  // RenderState.generateCommands + tick(): clear colour, hit/miss and ray counts
-  check(cudaMemsetAsync(fs.color.p, 0, fs.color.bytes(), st), "memset");
-  check(cudaMemsetAsync(&fs.ctr.p->num_hits, 0, 16, st), "memset");
-  check(cudaMemsetAsync(fs.tickets.p, 0, fs.tickets.bytes(), st), "memset");
-  check(cudaMemsetAsync(fs.tiles.p, 0, (size_t)std::max(nb, 1u) * (2 * c->ct + c->st) * 8, st), "memset");
+  // RenderState.generateCommands + tick(): the colour buffer is cleared by the
+  // camera pass of a single batch (its rays cover every pixel once)
+  if (nbatch > 1) check(cudaMemsetAsync(fs.color.p, 0, fs.color.bytes(), st), "memset");
   uint64_t seq = 0;  // (batch, bounce) steps so far: their ticket and tile slots
   for (uint32_t batch = 0; batch < nbatch; batch++) {
     if (batch) {
@@ -902,7 +898,7 @@ static void render_frame_launches(pk_ctx* c, int k, cudaStream_t st, uint32_t bo
       check(cudaMemsetAsync(&fs.ctr.p->num_hits, 0, 16, st), "memset");  // clearNumHitsAndMisses, clearNumRays
     }
     fs.cur = 0;
-    c->timed(K_CAMERA, [&]() { launch_camera(L, fs.R(0), c->cap, (int64_t)batch * c->B); });
+    c->timed(K_CAMERA, [&]() { launch_camera(L, fs.R(0), c->cap, (int64_t)batch * c->B, nbatch == 1); });
     for (uint32_t b = 0; b < bounces; b++, seq++) {
       const uint32_t slot = (uint32_t)(seq % MAX_BOUNCES);
       if (seq && slot == 0) {
@@ -940,11 +936,6 @@ static void render_frame_launches(pk_ctx* c, int k, cudaStream_t st, uint32_t bo
     }
   }
   join();
-  if (tail) {
-    c->timed(K_ACCUM, [&]() { launch_accumulate(L); });
-    c->timed(K_POST, [&]() { launch_postprocess(L, c->exposure, c->saturation); });
-    c->timed(K_OTHER, [&]() { launch_end_frame(L); });
-  }
   check(cudaGetLastError(), "render_frame");
 }
 
@@ -969,18 +960,24 @@ static void render_frame(pk_ctx* c, uint32_t bounces) {
     check(cudaStreamWaitEvent(st, c->ev_read, 0), "cudaStreamWaitEvent");
     c->read_pending = false;
   }
-  launch_set_state(st, fs.ctr.p, fs.cam.p, c->samples_next, c->theta_next, c->cam_host, true);
+  LaunchCtx L = c->launch(k, st);
+  const uint32_t nbatch = (uint32_t)(((uint64_t)c->npix + c->B - 1) / c->B);
+  const uint64_t steps = std::min<uint64_t>(std::max<uint64_t>((uint64_t)nbatch * bounces, 1), MAX_BOUNCES);
+  launch_frame_begin(L, fs.cam.p, c->samples_next, c->theta_next, c->cam_host, fs.tickets.p, (uint32_t)fs.tickets.n,
+                     fs.tiles.p, (uint32_t)(steps * (2 * c->ct + c->st)));
   if (c->timing) {
-    render_frame_launches(c, k, st, bounces, true);
+    render_frame_launches(c, k, st, bounces);
+    c->timed(K_ACCUM, [&]() { launch_accumulate(L); });
+    c->timed(K_POST, [&]() { launch_postprocess(L, c->exposure, c->saturation); });
+    c->timed(K_OTHER, [&]() { launch_end_frame(L); });
   } else {
-    const bool tail = !piped;
     if (!fs.graph || fs.graph_bounces != bounces || fs.graph_counting != c->counting ||
-        fs.graph_key != c->state_version || fs.graph_tail != tail) {
+        fs.graph_key != c->state_version) {
       fs.drop_graph();
       cudaGraph_t g = nullptr;
       check(cudaStreamBeginCapture(st, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
       try {
-        render_frame_launches(c, k, st, bounces, tail);
+        render_frame_launches(c, k, st, bounces);
       } catch (...) {
         cudaStreamEndCapture(st, &g);
         if (g) cudaGraphDestroy(g);
@@ -995,18 +992,16 @@ static void render_frame(pk_ctx* c, uint32_t bounces) {
       fs.graph_bounces = bounces;
       fs.graph_counting = c->counting;
       fs.graph_key = c->state_version;
-      fs.graph_tail = tail;
     }
     check(cudaGraphLaunch(fs.graph, st), "cudaGraphLaunch");
+    if (piped) {
+      if (c->tail_pending) check(cudaStreamWaitEvent(st, c->ev_tail, 0), "cudaStreamWaitEvent");
+      if (c->read_pending) check(cudaStreamWaitEvent(st, c->ev_read, 0), "cudaStreamWaitEvent");
+    }
+    launch_frame_end(L, c->samples_next, c->exposure, c->saturation);
   }
+  check(cudaGetLastError(), "render_frame");
   if (piped) {
-    LaunchCtx L = c->launch(k, st);
-    if (c->tail_pending) check(cudaStreamWaitEvent(st, c->ev_tail, 0), "cudaStreamWaitEvent");
-    launch_accumulate(L);
-    if (c->read_pending) check(cudaStreamWaitEvent(st, c->ev_read, 0), "cudaStreamWaitEvent");
-    launch_postprocess(L, c->exposure, c->saturation);
-    launch_end_frame(L);
-    check(cudaGetLastError(), "render_frame");
     check(cudaEventRecord(c->ev_tail, st), "cudaEventRecord");
     check(cudaEventRecord(fs.ev_done, st), "cudaEventRecord");
     c->tail_pending = true;

@@ -28,7 +28,7 @@ struct EventPair {
 // shared.  Slot 0 is also the state of the pass-by-pass API.
 struct FrameSlot {
   DevBuf<Counters> ctr;
-  DevBuf<CamState> cam;
+  DevBuf<CamDev> cam;
   DevBuf<float4> color;
   DevBuf<float4> rq[2][3], sq[3];
   DevBuf<uint4> hrec;
@@ -45,7 +45,7 @@ struct FrameSlot {
   // launch parameter changes.
   cudaGraphExec_t graph = nullptr;
   uint32_t graph_bounces = 0;
-  bool graph_counting = false, graph_tail = false;
+  bool graph_counting = false;
   unsigned long long graph_key = 0;
 
   RayQ R(int i) { return RayQ{rq[i][0].p, rq[i][1].p, rq[i][2].p}; }
@@ -68,6 +68,7 @@ struct pk_ctx {
   using LaunchCtx = pk::LaunchCtx;
   using Counters = pk::Counters;
   using CamState = pk::CamState;
+  using CamDev = pk::CamDev;
   template <class T>
   using DevBuf = pk::DevBuf<T>;
   using EventPair = pk::EventPair;
@@ -100,7 +101,7 @@ struct pk_ctx {
   CamState cam_host{};
   bool state_dirty = false;  // slot 0's device copy is stale
   DevBuf<Counters>& ctr = slot[0].ctr;
-  DevBuf<CamState>& cam = slot[0].cam;
+  DevBuf<CamDev>& cam = slot[0].cam;
   bool cam_set = false;
   float exposure = 1.0f, saturation = 1.0f;
   DevBuf<float4>& color = slot[0].color;

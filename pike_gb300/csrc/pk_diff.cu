@@ -319,13 +319,16 @@ struct ViewDev {
 constexpr int PATH_THREADS = 128;
 
 __global__ void __launch_bounds__(PATH_THREADS) k_path_camera(PathDev D, ViewDev V, uint32_t sample_base) {
+  __shared__ CamBasis s_basis;
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (threadIdx.x == 0) s_basis = camera_basis(V.cam);
   if (i == 0) D.count->rays[0] = D.n;
+  __syncthreads();
   if (i >= D.n) return;
   const unsigned long long npix = (unsigned long long)V.W * V.H, p = V.first + i;
   const uint32_t pix = (uint32_t)(p % npix), px = pix % V.W, py = pix / V.W;
   V3 org, dir;
-  camera_ray(V.cam, px, py, V.W, V.H, (int32_t)(sample_base + (uint32_t)(p / npix)), org, dir);
+  camera_ray(V.cam, s_basis, px, py, V.W, V.H, (int32_t)(sample_base + (uint32_t)(p / npix)), org, dir);
   D.o[0][i] = make_float4(org.x, org.y, org.z, __uint_as_float(i));
   D.d[0][i] = make_float4(dir.x, dir.y, dir.z, 0.0f);
   D.t[0][i] = make_float4(1.0f, 1.0f, 1.0f, __uint_as_float(pix));

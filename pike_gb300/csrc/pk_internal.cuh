@@ -43,6 +43,12 @@ struct CamState {
   uint32_t invocation_offset;
 };
 
+// CamState on the device with the screen axes derived from it (camera_basis).
+struct CamDev {
+  CamState c;
+  float bx[3], by[3];
+};
+
 // One ray queue in SoA form.  Together the three float4 are the reference's
 // 48-byte DeferredRay {origin, dir, throughput}; t.w holds the pixel index bits.
 struct RayQ {

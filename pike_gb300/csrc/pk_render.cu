@@ -19,17 +19,21 @@ namespace pk {
 
 // offset >= 0 replaces the camera's invocationOffset (tick()'s batch j passes
 // j * BATCH_SIZE, pike.js:146).
-__global__ void __launch_bounds__(128) k_camera(const CamState* __restrict__ camp, Counters* __restrict__ ctr,
-                                                RayQ R, uint32_t n_threads, uint32_t capacity, int64_t offset) {
+// clear: the colour buffer's pixels are zeroed here too (a frame of one batch).
+__global__ void __launch_bounds__(128) k_camera(const CamDev* __restrict__ camp, Counters* __restrict__ ctr,
+                                                RayQ R, uint32_t n_threads, uint32_t capacity, int64_t offset,
+                                                float4* __restrict__ clear, uint32_t npix) {
   const uint32_t gid = blockIdx.x * blockDim.x + threadIdx.x;
+  if (clear && gid < npix) clear[gid] = make_float4(0.f, 0.f, 0.f, 0.f);
   if (gid >= n_threads) return;
-  const CamState cam = *camp;
+  const CamState cam = camp->c;
+  const CamBasis basis{v3(camp->bx[0], camp->bx[1], camp->bx[2]), v3(camp->by[0], camp->by[1], camp->by[2])};
   const uint32_t W = cam.dims_mask >> 16, H = cam.dims_mask & 0xffffu;
   const uint32_t idx = gid + (offset >= 0 ? (uint32_t)offset : cam.invocation_offset);
   const uint32_t px = idx % W, py = idx / W;
   if (px >= W || py >= H) return;
   V3 org, dir;
-  camera_ray(cam, px, py, W, H, ctr->samples, org, dir);
+  camera_ray(cam, basis, px, py, W, H, ctr->samples, org, dir);
   if (gid < capacity) {
     R.o[gid] = make_float4(org.x, org.y, org.z, 0.0f);
     R.d[gid] = make_float4(dir.x, dir.y, dir.z, 0.0f);
@@ -210,6 +214,11 @@ __device__ __forceinline__ void inner_children_exact(const SceneDev& sc, int cur
   cr = ch.y;
 }
 
+// Rays a warp takes at least when there are too few to give every warp of the
+// full grid 32 (pass by pass, 640x360 in batches of 100,000: 32 1744-1758 us, 16
+// 1685-1699, 8 1665, 4 1642-1644; 256x256 and 853x479 frames within 1%).
+constexpr uint32_t TRACE_SPREAD = 4;
+
 // 10 resident blocks per SM (<= 48 registers): with several frames in
 // flight this beats the unconstrained 55 registers (2607-2611 vs 2579-2581
 // Mrays/s at 1080p, paired runs) and 12 blocks (2494).
@@ -237,7 +246,11 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_DYN_MINBLOCKS) k_trace_dyn(S
   }
   uint32_t nfetch = 0, ntest = 0, nhit = 0;
   uint32_t j = 0;
-  bool have = false, exhausted = false;
+  // Few rays are spread over all warps of the grid, at least TRACE_SPREAD to a
+  // warp: lanes of a warp wait for one another's nodes and leaves, and there
+  // are warps to spare.
+  const uint32_t warps = gridDim.x * (TRACE_THREADS / 32), share = (n + warps - 1) / warps;
+  bool have = false, exhausted = (uint32_t)lane >= max(TRACE_SPREAD, share);
   float ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f, ix = 0.f, iy = 0.f, iz = 0.f;
   WtRay wr{};  // EXACT: the watertight test's per-ray set-up
   float best_t = MAX_T;
@@ -866,31 +879,22 @@ __global__ void __launch_bounds__(128) k_shade_miss(EnvDev env, Counters* __rest
 
 // accumulate.wgsl:20-34 (pixels x < W only; the reference's `>` bound lets
 // invocation x == W alias pixel (0, y+1) in a race, which is not reproduced).
+__device__ __forceinline__ float4 accumulate_one(int32_t samples, float4 c, float4 a) {
+  const float s = (float)samples, s1 = (float)(samples + 1);
+  return make_float4((fmax_(c.x, 0.0f) + a.x * s) / s1, (fmax_(c.y, 0.0f) + a.y * s) / s1,
+                     (fmax_(c.z, 0.0f) + a.z * s) / s1, 1.0f);
+}
 __global__ void __launch_bounds__(256) k_accumulate(const Counters* __restrict__ ctr, const float4* __restrict__ color,
                                                     float4* __restrict__ accum, uint32_t npix) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= npix) return;
-  const float s = (float)ctr->samples, s1 = (float)(ctr->samples + 1);
-  const float4 c = color[i];
-  float4 a = accum[i];
-  a.x = (fmax_(c.x, 0.0f) + a.x * s) / s1;
-  a.y = (fmax_(c.y, 0.0f) + a.y * s) / s1;
-  a.z = (fmax_(c.z, 0.0f) + a.z * s) / s1;
-  a.w = 1.0f;
-  accum[i] = a;
+  if (i < npix) accum[i] = accumulate_one(ctr->samples, color[i], accum[i]);
 }
 
 // Compensated accumulation (precision form, not the reference's running
 // mean): Kahan sums of max(c, 0) per pixel; the accumulation buffer receives
 // sum / (n + 1) so postprocess and readback see the same mean.
-__global__ void __launch_bounds__(256) k_accumulate_kahan(const Counters* __restrict__ ctr,
-                                                          const float4* __restrict__ color, float4* __restrict__ sum,
-                                                          float4* __restrict__ comp, float4* __restrict__ accum,
-                                                          uint32_t npix) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= npix) return;
-  const int32_t n = ctr->samples;
-  const float4 c = color[i];
+__device__ __forceinline__ float4 accumulate_kahan_one(int32_t n, float4 c, float4* __restrict__ sum,
+                                                       float4* __restrict__ comp, uint32_t i) {
   float4 sv = n == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : sum[i];
   float4 cv = n == 0 ? make_float4(0.f, 0.f, 0.f, 0.f) : comp[i];
   const float in[3] = {fmax_(c.x, 0.0f), fmax_(c.y, 0.0f), fmax_(c.z, 0.0f)};
@@ -906,7 +910,14 @@ __global__ void __launch_bounds__(256) k_accumulate_kahan(const Counters* __rest
   sum[i] = sv;
   comp[i] = cv;
   const float s1 = (float)(n + 1);
-  accum[i] = make_float4(sv.x / s1, sv.y / s1, sv.z / s1, 1.0f);
+  return make_float4(sv.x / s1, sv.y / s1, sv.z / s1, 1.0f);
+}
+__global__ void __launch_bounds__(256) k_accumulate_kahan(const Counters* __restrict__ ctr,
+                                                          const float4* __restrict__ color, float4* __restrict__ sum,
+                                                          float4* __restrict__ comp, float4* __restrict__ accum,
+                                                          uint32_t npix) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < npix) accum[i] = accumulate_kahan_one(ctr->samples, color[i], sum, comp, i);
 }
 
 // postprocess.wgsl:36-99 frag_main as a compute kernel writing a headless buffer.
@@ -915,12 +926,8 @@ __device__ __forceinline__ float rrt(float v) {
   const float b = v * (0.983729f * v + 0.4329510f) + 0.238081f;
   return a / b;
 }
-__global__ void __launch_bounds__(256) k_postprocess(const float4* __restrict__ accum, float4* __restrict__ out,
-                                                     uchar4* __restrict__ out8, uint32_t npix, float exposure,
-                                                     float saturation) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= npix) return;
-  const float4 a4 = accum[i];
+__device__ __forceinline__ void postprocess_one(float4 a4, float4* __restrict__ out, uchar4* __restrict__ out8,
+                                                uint32_t i, float exposure, float saturation) {
   V3 cc = scale(v3(a4.x, a4.y, a4.z), exposure);
   V3 o = vecmat(cc, v3(0.59719f, 0.35458f, 0.04823f), v3(0.07600f, 0.90834f, 0.01566f), v3(0.02840f, 0.13383f, 0.83777f));
   o = v3(rrt(o.x), rrt(o.y), rrt(o.z));
@@ -947,13 +954,58 @@ __global__ void __launch_bounds__(256) k_postprocess(const float4* __restrict__ 
   q.w = 255;
   out8[i] = q;
 }
+__global__ void __launch_bounds__(256) k_postprocess(const float4* __restrict__ accum, float4* __restrict__ out,
+                                                     uchar4* __restrict__ out8, uint32_t npix, float exposure,
+                                                     float saturation) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i < npix) postprocess_one(accum[i], out, out8, i, exposure, saturation);
+}
+
+// A frame's beginning and end in one launch each (pk_render_frame): on small
+// frames a launch costs as much as its work, 3.4 us a node with eight 256x256
+// frames in flight.  Begin: the render state by value, the axes of the camera,
+// zeroed queue counts, tickets and look-back states.  End: accumulation,
+// postprocessing and the sample count.
+__device__ __forceinline__ void set_state(Counters* ctr, CamDev* cam, int32_t samples, float theta,
+                                          const CamState& cs, int with_cam) {
+  ctr->samples = samples;
+  ctr->env_theta = theta;
+  if (with_cam) {
+    const CamBasis b = camera_basis(cs);
+    cam->c = cs;
+    cam->bx[0] = b.bx.x; cam->bx[1] = b.bx.y; cam->bx[2] = b.bx.z;
+    cam->by[0] = b.by.x; cam->by[1] = b.by.y; cam->by[2] = b.by.z;
+  }
+}
+__global__ void __launch_bounds__(256) k_frame_begin(Counters* ctr, CamDev* cam, int32_t samples, float theta, CamState cs,
+                                                     uint32_t* __restrict__ tickets, uint32_t n_tickets,
+                                                     unsigned long long* __restrict__ tiles, uint32_t n_tiles) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) {
+    set_state(ctr, cam, samples, theta, cs, 1);
+    ctr->num_hits = ctr->num_misses = ctr->num_rays = ctr->num_shadow = 0u;
+  }
+  if (i < n_tickets) tickets[i] = 0u;
+  for (uint32_t k = i; k < n_tiles; k += gridDim.x * blockDim.x) tiles[k] = 0ull;
+}
+__global__ void __launch_bounds__(256) k_frame_end(Counters* ctr, int32_t samples, const float4* __restrict__ color,
+                                                   float4* __restrict__ sum, float4* __restrict__ comp,
+                                                   float4* __restrict__ accum, float4* __restrict__ out,
+                                                   uchar4* __restrict__ out8, uint32_t npix, float exposure,
+                                                   float saturation) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) ctr->samples = samples + 1;
+  if (i >= npix) return;
+  const float4 a = sum ? accumulate_kahan_one(samples, color[i], sum, comp, i)
+                       : accumulate_one(samples, color[i], accum[i]);
+  accum[i] = a;
+  postprocess_one(a, out, out8, i, exposure, saturation);
+}
 
 __global__ void k_end_frame(Counters* ctr) { ctr->samples += 1; }
 // The render state a frame starts from (RenderState + CameraPass uniforms).
-__global__ void k_set_state(Counters* ctr, CamState* cam, int32_t samples, float theta, CamState cs, int with_cam) {
-  ctr->samples = samples;
-  ctr->env_theta = theta;
-  if (with_cam) *cam = cs;
+__global__ void k_set_state(Counters* ctr, CamDev* cam, int32_t samples, float theta, CamState cs, int with_cam) {
+  set_state(ctr, cam, samples, theta, cs, with_cam);
 }
 
 // Elementwise math probes (same numbering as the oracle's or_math).
@@ -1027,7 +1079,7 @@ __device__ __noinline__ bool batch_shade(const SceneDev& sc, const EnvDev& env, 
 }
 __device__ __noinline__ void batch_camera(const CamState& cam, uint32_t px, uint32_t py, uint32_t W, uint32_t H,
                                           int32_t samples, V3& org, V3& dir) {
-  camera_ray(cam, px, py, W, H, samples, org, dir);
+  camera_ray(cam, camera_basis(cam), px, py, W, H, samples, org, dir);
 }
 
 // 40 resident warps per SM (48 registers, some spilled): the loop stalls
@@ -1215,13 +1267,15 @@ Grids kernel_grids(int sms, uint32_t capacity) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s, k_shade, SHADE_THREADS, 0);
   const unsigned n = (unsigned)sms;
   const unsigned rays = std::max(1u, ((capacity + 31u) / 32u + TRACE_THREADS / 32 - 1) / (TRACE_THREADS / 32));
-  return Grids{Grid{n * std::max(t, 1), rays}, Grid{n * std::max(c, 1), std::max(1u, compact_tiles(capacity))},
+  const unsigned spread = (capacity + TRACE_SPREAD * (TRACE_THREADS / 32) - 1) / (TRACE_SPREAD * (TRACE_THREADS / 32));
+  return Grids{Grid{n * std::max(t, 1), std::max(1u, spread)}, Grid{n * std::max(c, 1), std::max(1u, compact_tiles(capacity))},
                Grid{n * std::max(s, 1), std::max(1u, shade_tiles(capacity))}, Grid{n * std::max(w, 1), rays}};
 }
 
-void launch_camera(const LaunchCtx& L, RayQ R, uint32_t n_threads, int64_t offset) {
+void launch_camera(const LaunchCtx& L, RayQ R, uint32_t n_threads, int64_t offset, bool clear) {
   if (n_threads == 0) return;
-  k_camera<<<grid_for(n_threads, 128), 128, 0, L.stream>>>(L.cam, L.ctr, R, n_threads, L.capacity, offset);
+  k_camera<<<grid_for(n_threads, 128), 128, 0, L.stream>>>(L.cam, L.ctr, R, n_threads, L.capacity, offset,
+                                                           clear ? L.color : nullptr, L.npix);
 }
 
 void launch_trace(const LaunchCtx& L, bool any_hit, bool fused, bool count, const uint32_t* countp, RayQ R,
@@ -1326,7 +1380,16 @@ void launch_postprocess(const LaunchCtx& L, float exposure, float saturation) {
 }
 
 void launch_end_frame(const LaunchCtx& L) { k_end_frame<<<1, 1, 0, L.stream>>>(L.ctr); }
-void launch_set_state(cudaStream_t s, Counters* ctr, CamState* cam, int32_t samples, float theta, const CamState& cs,
+void launch_frame_begin(const LaunchCtx& L, CamDev* cam, int32_t samples, float theta, const CamState& cs,
+                        uint32_t* tickets, uint32_t n_tickets, unsigned long long* tiles, uint32_t n_tiles) {
+  const unsigned grid = std::max(1u, std::min(64u, grid_for(n_tiles, 1024)));
+  k_frame_begin<<<grid, 256, 0, L.stream>>>(L.ctr, cam, samples, theta, cs, tickets, n_tickets, tiles, n_tiles);
+}
+void launch_frame_end(const LaunchCtx& L, int32_t samples, float exposure, float saturation) {
+  k_frame_end<<<grid_for(L.npix, 256), 256, 0, L.stream>>>(L.ctr, samples, L.color, L.accum_sum, L.accum_comp, L.accum,
+                                                           L.display, L.display8, L.npix, exposure, saturation);
+}
+void launch_set_state(cudaStream_t s, Counters* ctr, CamDev* cam, int32_t samples, float theta, const CamState& cs,
                       bool with_cam) {
   k_set_state<<<1, 1, 0, s>>>(ctr, cam, samples, theta, cs, with_cam ? 1 : 0);
 }

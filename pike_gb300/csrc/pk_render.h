@@ -32,7 +32,7 @@ struct Grids {
 struct LaunchCtx {
   cudaStream_t stream;
   Counters* ctr;
-  const CamState* cam;
+  const CamDev* cam;
   SceneDev scene;
   EnvDev env;
   float4* color;
@@ -56,7 +56,8 @@ struct LaunchCtx {
 };
 
 // offset >= 0: invocation offset of the rays (else the camera state's own)
-void launch_camera(const LaunchCtx& L, RayQ R, uint32_t n_threads, int64_t offset = -1);
+// clear: zero the colour buffer as well
+void launch_camera(const LaunchCtx& L, RayQ R, uint32_t n_threads, int64_t offset = -1, bool clear = false);
 // Kernels that claim work through an atomic ticket take it as `ticket`; the
 // look-back kernels also take a zeroed tile-state array (one word per tile).
 // The persistent traversals set bits in `flags`, which must hold zeros; the
@@ -80,8 +81,13 @@ void launch_shade_miss(const LaunchCtx& L, RayQ M);
 void launch_accumulate(const LaunchCtx& L);
 void launch_postprocess(const LaunchCtx& L, float exposure, float saturation);
 void launch_end_frame(const LaunchCtx& L);
+// A frame's render state, zeroed counts, n_tickets tickets and n_tiles look-back
+// states; its accumulation, postprocessing and sample count.
+void launch_frame_begin(const LaunchCtx& L, CamDev* cam, int32_t samples, float theta, const CamState& cs,
+                        uint32_t* tickets, uint32_t n_tickets, unsigned long long* tiles, uint32_t n_tiles);
+void launch_frame_end(const LaunchCtx& L, int32_t samples, float exposure, float saturation);
 // Sets a frame's sample index, environment rotation and (with_cam) camera.
-void launch_set_state(cudaStream_t s, Counters* ctr, CamState* cam, int32_t samples, float theta, const CamState& cs,
+void launch_set_state(cudaStream_t s, Counters* ctr, CamDev* cam, int32_t samples, float theta, const CamState& cs,
                       bool with_cam);
 void launch_math(cudaStream_t s, int fn, const float* x, const float* y, float* out, uint32_t n);
 

@@ -14,9 +14,21 @@ constexpr float SHADE_EPS = 1e-7f;
 // =====================================================================
 // camera.wgsl:75-93 main + createPrimaryRay (:58-73)
 // =====================================================================
+// The camera's screen axes (camera.wgsl:58-66), the same for every ray.
+struct CamBasis {
+  V3 bx, by;
+};
+__device__ __forceinline__ CamBasis camera_basis(const CamState& cam) {
+  const V3 ed = v3(cam.dir[0], cam.dir[1], cam.dir[2]);
+  const float tf = tan_(cam.fov * 0.5f);
+  CamBasis b;
+  b.bx = scale(normalize(cross(ed, v3(0.0f, 1.0f, 0.0f))), tf);
+  b.by = scale(normalize(cross(b.bx, ed)), tf);
+  return b;
+}
 // camera.wgsl:54-76 createPrimaryRay for pixel (px, py) of a W x H image.
-__device__ __forceinline__ void camera_ray(const CamState& cam, uint32_t px, uint32_t py, uint32_t W, uint32_t H,
-                                           int32_t samples, V3& org, V3& dir) {
+__device__ __forceinline__ void camera_ray(const CamState& cam, const CamBasis& basis, uint32_t px, uint32_t py,
+                                           uint32_t W, uint32_t H, int32_t samples, V3& org, V3& dir) {
   Hash h;
   h.seed = (px * 1973u + py * 9277u + (uint32_t)samples * 26699u) | 1u;
   h.seed = h.next();
@@ -34,13 +46,20 @@ __device__ __forceinline__ void camera_ray(const CamState& cam, uint32_t px, uin
   uy = ru * ny;
   const V3 eo = v3(cam.pos[0], cam.pos[1], cam.pos[2]);
   const V3 ed = v3(cam.dir[0], cam.dir[1], cam.dir[2]);
-  const float tf = tan_(cam.fov * 0.5f);
-  const V3 bx = scale(normalize(cross(ed, v3(0.0f, 1.0f, 0.0f))), tf);
-  const V3 by = scale(normalize(cross(bx, ed)), tf);
+  const V3 screen = add(add(add(scale(basis.bx, ux), scale(basis.by, uy)), ed), eo);
+  // With a zero aperture the lens offset is a zero of some sign where its other
+  // factors are finite (bokeh > 0), and changes no sum here unless the eye has a -0.
+  const float axes = fabsf(basis.bx.x) + fabsf(basis.bx.y) + fabsf(basis.bx.z) + fabsf(basis.by.x) +
+                     fabsf(basis.by.y) + fabsf(basis.by.z);
+  if (cam.aperture == 0.0f && cam.bokeh > 0.0f && cam.bokeh < 1e30f && fabsf(cam.focal_depth) < 1e30f && axes < 1e30f && __float_as_uint(eo.x) != 0x80000000u &&
+      __float_as_uint(eo.y) != 0x80000000u && __float_as_uint(eo.z) != 0x80000000u) {
+    dir = normalize(sub(screen, eo));
+    org = eo;
+    return;
+  }
   const float theta = h.rand() * c::TAU;
   const float pw = pow_(h.rand(), cam.bokeh);
-  const V3 dof = scale(scale(add(scale(bx, cos_(theta)), scale(by, sin_(theta))), cam.aperture), pw);
-  const V3 screen = add(add(add(scale(bx, ux), scale(by, uy)), ed), eo);
+  const V3 dof = scale(scale(add(scale(basis.bx, cos_(theta)), scale(basis.by, sin_(theta))), cam.aperture), pw);
   dir = normalize(sub(add(screen, scale(dof, cam.focal_depth)), add(eo, dof)));
   org = add(dof, eo);
 }
