@@ -188,8 +188,9 @@ __device__ __forceinline__ void shade_diff(const SceneDev& sc, const EnvDev& env
   if (h.rand() > f) {
     const float lr = sqrtf(h.rand());
     const float lphi = c::TAU * h.rand();
-    const float x = lr * cos_(lphi);
-    const float y = lr * sin_(lphi);
+    const SinCos lp = sincos_(lphi);
+    const float x = lr * lp.c;
+    const float y = lr * lp.s;
     const float z = sqrtf(fmax_(0.0f, 1.0f - x * x - y * y));
     bs.wi = v3(x, y, z);
     bs.pdf = lambert_pdf(bs.wi);

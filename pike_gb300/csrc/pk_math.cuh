@@ -98,6 +98,19 @@ static __device__ __noinline__ float cos_(float x) {
   const float v = (q & 1) ? sin_poly(r) : cos_poly(r);
   return ((q + 1) & 2) ? -v : v;
 }
+// sin_ and cos_ of one angle: one reduction and one of each polynomial, where
+// two calls reduce twice and, in a warp with mixed quadrants, run all four.
+struct SinCos {
+  float s, c;
+};
+static __device__ __noinline__ SinCos sincos_(float x) {
+  if (!(fabsf(x) < 1.0e30f)) return SinCos{x - x, x - x};
+  int q;
+  const float r = reduce_pio2(x, q);
+  const float sp = sin_poly(r), cp = cos_poly(r);
+  const float s = (q & 1) ? cp : sp, c = (q & 1) ? sp : cp;
+  return SinCos{(q & 2) ? -s : s, ((q + 1) & 2) ? -c : c};
+}
 __device__ __forceinline__ float tan_(float x) { return sin_(x) / cos_(x); }
 
 __device__ __forceinline__ float atan01(float t) {
@@ -186,10 +199,27 @@ __device__ __forceinline__ float qdiv(float v, float d, float r) {
   const float q0 = __fmul_rn(v, r);
   return __fmaf_rn(__fmaf_rn(-q0, d, v), r, q0);
 }
-__device__ __forceinline__ float unorm16(uint32_t v) { return qdiv((float)v, 65535.0f, 0x1.0001p-16f); }
+// Small integers to float without the conversion instruction (a quarter of the
+// rate): 2^23 + v is the float with v in its low mantissa bits, and the
+// subtraction is exact.  byte_f: byte k of w; u16_f: v < 2^16.
+template <int K>
+__device__ __forceinline__ float byte_f(uint32_t w) {
+  return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u + K)) - 8388608.0f;
+}
+__device__ __forceinline__ float u16_f(uint32_t v) { return __uint_as_float(0x4b000000u | v) - 8388608.0f; }
+// Components of unpack4x8snorm: byte K of w, with w's bytes offset by 128
+// (w ^ 0x80808080); max(v, -127) / 127 is max(v / 127, -1).
+template <int K>
+__device__ __forceinline__ float snorm8_offset(uint32_t w) {
+  const float v = __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u + K)) - 8388736.0f;
+  return qdiv(fmaxf(v, -127.0f), 127.0f, 0x1.020408p-7f);
+}
+template <int K>
+__device__ __forceinline__ float unorm8_byte(uint32_t w) {
+  return qdiv(byte_f<K>(w), 255.0f, 0x1.010102p-8f);
+}
+__device__ __forceinline__ float unorm16(uint32_t v) { return qdiv(u16_f(v), 65535.0f, 0x1.0001p-16f); }  // v < 2^16
 __device__ __forceinline__ float snorm16(int v) { return fmax_(qdiv((float)v, 32767.0f, 0x1.0002p-15f), -1.0f); }
-__device__ __forceinline__ float snorm8(int v) { return fmax_(qdiv((float)v, 127.0f, 0x1.020408p-7f), -1.0f); }
-__device__ __forceinline__ float unorm8(uint32_t v) { return qdiv((float)v, 255.0f, 0x1.010102p-8f); }
 __device__ __forceinline__ uint32_t pack_unorm16(float e) {
   return (uint32_t)floorf(0.5f + 65535.0f * fmin_(1.0f, fmax_(0.0f, e)));
 }

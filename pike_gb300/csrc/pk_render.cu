@@ -750,8 +750,9 @@ __device__ __forceinline__ bool shade_one(const SceneDev& sc, const EnvDev& env,
     if (h.rand() > f) {
       const float lr = sqrtf(h.rand());
       const float lphi = c::TAU * h.rand();
-      const float x = lr * cos_(lphi);
-      const float y = lr * sin_(lphi);
+      const SinCos lp = sincos_(lphi);
+      const float x = lr * lp.c;
+      const float y = lr * lp.s;
       const float z = sqrtf(fmax_(0.0f, 1.0f - x * x - y * y));
       bs.wi = v3(x, y, z);
       bs.pdf = lambert_pdf(bs.wi);
@@ -1025,8 +1026,18 @@ __global__ void k_math(int fn, const float* __restrict__ x, const float* __restr
     case 6: r = log2_(a); break;
     case 7: r = pow_(a, b); break;
     case 8: r = snorm16_decode(__float_as_int(a)); break;
-    case 9: r = snorm8(__float_as_int(a)); break;     // integer inputs, bit-cast
-    case 10: r = unorm8((uint32_t)__float_as_int(a)); break;
+    case 9:  // integer inputs, bit-cast; every byte of a word in turn
+    case 10: {
+      const uint32_t v = (uint32_t)__float_as_int(a) & 0xffu, w = v << (8 * (i & 3u));
+      const uint32_t o = w ^ 0x80808080u;
+      switch (i & 3u) {
+        case 0: r = fn == 9 ? snorm8_offset<0>(o) : unorm8_byte<0>(w); break;
+        case 1: r = fn == 9 ? snorm8_offset<1>(o) : unorm8_byte<1>(w); break;
+        case 2: r = fn == 9 ? snorm8_offset<2>(o) : unorm8_byte<2>(w); break;
+        default: r = fn == 9 ? snorm8_offset<3>(o) : unorm8_byte<3>(w);
+      }
+      break;
+    }
     case 11: r = unorm16((uint32_t)__float_as_int(a)); break;
     case 12: r = snorm16(__float_as_int(a)); break;
     default: r = __int_as_float(0x7fc00000);

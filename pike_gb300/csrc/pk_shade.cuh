@@ -59,7 +59,8 @@ __device__ __forceinline__ void camera_ray(const CamState& cam, const CamBasis& 
   }
   const float theta = h.rand() * c::TAU;
   const float pw = pow_(h.rand(), cam.bokeh);
-  const V3 dof = scale(scale(add(scale(basis.bx, cos_(theta)), scale(basis.by, sin_(theta))), cam.aperture), pw);
+  const SinCos lens = sincos_(theta);
+  const V3 dof = scale(scale(add(scale(basis.bx, lens.c), scale(basis.by, lens.s)), cam.aperture), pw);
   dir = normalize(sub(add(screen, scale(dof, cam.focal_depth)), add(eo, dof)));
   org = add(dof, eo);
 }
@@ -73,8 +74,8 @@ __device__ __forceinline__ V3 env_color(const EnvDev& env, float theta, V3 dir) 
   int x = f2i(floorf(u * (float)env.w)), y = f2i(floorf(v * (float)env.h));
   x = ((x % env.w) + env.w) % env.w;
   y = ((y % env.h) + env.h) % env.h;
-  const uchar4 cc = env.rgbe[(size_t)y * env.w + x];
-  const float r = unorm8(cc.x), g = unorm8(cc.y), b = unorm8(cc.z), a = unorm8(cc.w);
+  const uint32_t cc = __ldg(reinterpret_cast<const uint32_t*>(env.rgbe) + ((size_t)y * env.w + x));
+  const float r = unorm8_byte<0>(cc), g = unorm8_byte<1>(cc), b = unorm8_byte<2>(cc), a = unorm8_byte<3>(cc);
   const float p = pow_(2.0f, a * 255.0f - 128.0f);
   return v3(r * p, g * p, b * p);
 }
@@ -94,8 +95,8 @@ __device__ __forceinline__ float4 texel_at(const SceneDev& sc, int l, int i, int
   const int R = sc.atlas_res;
   i = ((i % R) + R) % R;
   j = ((j % R) + R) % R;
-  const uchar4 t = __ldg(sc.layers + ((size_t)l * R + (size_t)j) * R + (size_t)i);
-  return make_float4(unorm8(t.x), unorm8(t.y), unorm8(t.z), unorm8(t.w));
+  const uint32_t t = __ldg(reinterpret_cast<const uint32_t*>(sc.layers) + ((size_t)l * R + (size_t)j) * R + (size_t)i);
+  return make_float4(unorm8_byte<0>(t), unorm8_byte<1>(t), unorm8_byte<2>(t), unorm8_byte<3>(t));
 }
 // textureSampleLevel(atlas, linear + repeat sampler, uv, layer, 0) on rgba8unorm
 // layers (shade_hit.wgsl:184-197): a 1x1 layer returns its texel; larger ones
@@ -103,7 +104,10 @@ __device__ __forceinline__ float4 texel_at(const SceneDev& sc, int l, int i, int
 __device__ __forceinline__ float4 texel(const SceneDev& sc, int layer, float u, float v) {
   const int l = layer < 0 ? 0 : (layer >= sc.n_layers ? sc.n_layers - 1 : layer);
   const int R = sc.atlas_res;
-  if (R == 1) return texel_at(sc, l, 0, 0);
+  if (R == 1) {
+    const uint32_t t = __ldg(reinterpret_cast<const uint32_t*>(sc.layers) + l);
+    return make_float4(unorm8_byte<0>(t), unorm8_byte<1>(t), unorm8_byte<2>(t), unorm8_byte<3>(t));
+  }
   const float x = u * (float)R - 0.5f, y = v * (float)R - 0.5f;
   const float x0 = floorf(x), y0 = floorf(y);
   const float fx = x - x0, fy = y - y0;
@@ -114,9 +118,10 @@ __device__ __forceinline__ float4 texel(const SceneDev& sc, int layer, float u, 
                      mix1(mix1(a.z, b.z, fx), mix1(c.z, d.z, fx), fy), mix1(mix1(a.w, b.w, fx), mix1(c.w, d.w, fx), fy));
 }
 __device__ __forceinline__ void unpack_snorm8x3(uint32_t w, V3& o) {
-  o.x = snorm8((int)(int8_t)(w & 0xffu));
-  o.y = snorm8((int)(int8_t)((w >> 8) & 0xffu));
-  o.z = snorm8((int)(int8_t)((w >> 16) & 0xffu));
+  w ^= 0x80808080u;
+  o.x = snorm8_offset<0>(w);
+  o.y = snorm8_offset<1>(w);
+  o.z = snorm8_offset<2>(w);
 }
 // branchlessONB (:166-177)
 __device__ __forceinline__ void onb(V3 n, V3& b1, V3& b2) {
@@ -142,11 +147,14 @@ __device__ __forceinline__ SI surface(const SceneDev& sc, V3 ro, V3 rd, float t,
   const V3 T = normalize(matvec(t0, t1, t2, bary));
   const V3 B = normalize(matvec(q0, q1, q2, bary));
   const V3 N = normalize(matvec(n0, n1, n2, bary));
-  // uvs * bary (mat3x2 * vec3)
-  const float tu = snorm16((int)(int16_t)(a0.w & 0xffffu)) * bary.x + snorm16((int)(int16_t)(a1.w & 0xffffu)) * bary.y +
-                   snorm16((int)(int16_t)(a2.w & 0xffffu)) * bary.z;
-  const float tv = snorm16((int)(int16_t)(a0.w >> 16)) * bary.x + snorm16((int)(int16_t)(a1.w >> 16)) * bary.y +
-                   snorm16((int)(int16_t)(a2.w >> 16)) * bary.z;
+  // uvs * bary (mat3x2 * vec3); a 1x1 layer has one texel wherever it is sampled
+  float tu = 0.0f, tv = 0.0f;
+  if (sc.atlas_res != 1) {
+    tu = snorm16((int)(int16_t)(a0.w & 0xffffu)) * bary.x + snorm16((int)(int16_t)(a1.w & 0xffffu)) * bary.y +
+         snorm16((int)(int16_t)(a2.w & 0xffffu)) * bary.z;
+    tv = snorm16((int)(int16_t)(a0.w >> 16)) * bary.x + snorm16((int)(int16_t)(a1.w >> 16)) * bary.y +
+         snorm16((int)(int16_t)(a2.w >> 16)) * bary.z;
+  }
   const int4 mat = __ldg(sc.mat4 + tri.w);
   const float4 nm = texel(sc, mat.z, tu, tv);
   const V3 map_normal = mul(sub(v3(nm.x, nm.y, nm.z), v3(0.5f, 0.5f, 0.0f)), v3(2.0f, 2.0f, 1.0f));
@@ -199,8 +207,9 @@ __device__ __forceinline__ Sample sample_env(const EnvDev& env, float theta, Has
   const float v = (0.5f + (float)cc.y) / (float)env.h;
   const float th = u * c::TAU;
   const float phi = v * c::PI;
-  const float sin_phi = sin_(phi);
-  const V3 dir = v3(cos_(th) * sin_phi, cos_(phi), sin_(th) * sin_phi);
+  const SinCos pt = sincos_(phi), tt = sincos_(th);
+  const float sin_phi = pt.s;
+  const V3 dir = v3(tt.c * sin_phi, pt.c, tt.s * sin_phi);
   Sample s;
   s.pdf = pdf_texel(env, cc.x, cc.y) / sin_phi;
   s.wi = vecmat(dir, si.b1, si.b2, si.n);
@@ -251,8 +260,9 @@ __device__ __forceinline__ V3 sample_ggx(Hash& h, const SI& si) {
   const V3 t2v = cross(vh, t1v);
   const float r = sqrtf(h.rand());
   const float phi = c::TAU * h.rand();
-  const float t1 = r * cos_(phi);
-  float t2 = r * sin_(phi);
+  const SinCos sp = sincos_(phi);
+  const float t1 = r * sp.c;
+  float t2 = r * sp.s;
   const float s = 0.5f * (1.0f + vh.z);
   t2 = (1.0f - s) * sqrtf(1.0f - t1 * t1) + s * t2;
   const V3 nh = add(add(scale(t1v, t1), scale(t2v, t2)), scale(vh, sqrtf(fmax_(0.0f, 1.0f - t1 * t1 - t2 * t2))));
