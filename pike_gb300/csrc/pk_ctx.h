@@ -221,7 +221,7 @@ struct pk_ctx {
   pk::SceneDev dropin_scene() {
     pk::SceneDev s = launch().scene;
     s.inner = inner.p;
-    s.inner32 = compact_nodes ? inner32.p : nullptr;
+    s.inner32 = nullptr;  // always the 64-byte records: the same boxes
     s.root = root;
     return s;
   }

@@ -68,7 +68,7 @@ __device__ __forceinline__ void fused_miss(float4* color, uint32_t npix, uint4* 
 // every slot goes to flags[slot / 32].  FUSED: a ray that reaches the
 // environment adds its shade_miss.wgsl contribution directly (the miss queue
 // is not materialised); otherwise the compaction kernel builds the miss queue.
-template <bool ANY, bool FUSED, bool COUNT>
+template <bool ANY, bool FUSED, bool COUNT, bool COMPACT>
 __global__ void __launch_bounds__(TRACE_THREADS) k_trace(SceneDev sc, EnvDev env, Counters* __restrict__ ctr,
                                                           const uint32_t* __restrict__ countp, RayQ R,
                                                           uint4* __restrict__ hrec, uint32_t* __restrict__ flags,
@@ -96,7 +96,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_trace(SceneDev sc, EnvDev env
       float bt;
       int bi;
       uint32_t bb;
-      traverse<ANY, COUNT>(sc, o.x, o.y, o.z, d.x, d.y, d.z, bt, bi, bb, sstack, &ctr->err, nfetch, ntest);
+      traverse<ANY, COUNT, TRACE_THREADS, STACK_SMEM, COMPACT>(sc, o.x, o.y, o.z, d.x, d.y, d.z, bt, bi, bb, sstack, &ctr->err, nfetch, ntest);
       hit = bi != -1;
       if (hit && !ANY) hrec[j] = make_uint4(__float_as_uint(bt), (uint32_t)bi, bb, 0u);
       if (!hit && FUSED) {
@@ -179,15 +179,11 @@ constexpr int DYN_LOCAL = 64 - DYN_SMEM;
 #define PK_ANY_BUDGET PK_INNER_BUDGET
 #endif
 constexpr int INNER_BUDGET = PK_INNER_BUDGET;
-// Unroll of the leaf loop (the compiler then issues the next triangle's loads
-// early).  1080p, three paired runs: unrolled by 4 3753-3769 Mrays/s and a
-// 0.357-0.359 ms closest-hit launch, not unrolled 3727-3747 and 0.364-0.366
-// ms, by 2 3726-3734, by 8 3663-3673.
-#ifndef PK_LEAF_UNROLL
-#define PK_LEAF_UNROLL 4
-#endif
-constexpr int LEAF_UNROLL = PK_LEAF_UNROLL;
-
+// The leaf loop is not unrolled: leaves hold few triangles, and the loop's code
+// is what the instruction cache has to hold beside the inner loop's.  Eight
+// 1080p frames 25.6 ms unrolled by 4 (what the compiler chooses by itself too),
+// 25.7 by 2, 24.75 not unrolled.  (An unroll by 4 paid before the two record
+// formats had kernels of their own.)
 constexpr int ANY_BUDGET = PK_ANY_BUDGET;
 
 // Box test of the exact binary records: like box_hit, with the far distance
@@ -226,7 +222,12 @@ constexpr uint32_t TRACE_SPREAD = 4;
 #ifndef PK_DYN_MINBLOCKS
 #define PK_DYN_MINBLOCKS 10
 #endif
-template <bool ANY, bool FUSED, bool COUNT, bool EXACT>
+// (with the code of one record format per kernel and packed slab tests: 10
+// blocks 24.16 ms for eight 1080p frames, 9 24.64)
+// Which inner records a kernel reads, a constant: choosing by the pointer in
+// every step put both formats' code into the loop (24.75 against 24.16 ms).
+constexpr int NODES_64 = 0, NODES_32 = 1, NODES_EXACT = 2;
+template <bool ANY, bool FUSED, bool COUNT, int NODES>
 __global__ void __launch_bounds__(TRACE_THREADS, PK_DYN_MINBLOCKS) k_trace_dyn(SceneDev sc, EnvDev env, Counters* __restrict__ ctr,
                                                               const uint32_t* __restrict__ countp, RayQ R,
                                                               uint4* __restrict__ hrec, uint32_t* __restrict__ flags,
@@ -252,6 +253,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_DYN_MINBLOCKS) k_trace_dyn(S
   const uint32_t warps = gridDim.x * (TRACE_THREADS / 32), share = (n + warps - 1) / warps;
   bool have = false, exhausted = (uint32_t)lane >= max(TRACE_SPREAD, share);
   float ox = 0.f, oy = 0.f, oz = 0.f, dx = 0.f, dy = 0.f, dz = 0.f, ix = 0.f, iy = 0.f, iz = 0.f;
+  constexpr bool EXACT = NODES == NODES_EXACT;
   WtRay wr{};  // EXACT: the watertight test's per-ray set-up
   float best_t = MAX_T;
   int best_i = -1;
@@ -304,7 +306,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_DYN_MINBLOCKS) k_trace_dyn(S
         lok = lh < MAX_T && lh <= lim;
         rok = rh < MAX_T && rh <= lim;
       } else {
-        inner_children(sc, cur, ox, oy, oz, ix, iy, iz, lh, rh, cl, cr);
+        inner_children<NODES == NODES_32>(sc, cur, ox, oy, oz, ix, iy, iz, lh, rh, cl, cr);
         lok = lh < best_t;
         rok = rh < best_t;
       }
@@ -330,9 +332,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_DYN_MINBLOCKS) k_trace_dyn(S
       const uint32_t word = (uint32_t)cur & 0x7fffffffu;
       const int size = (int)(word >> 24);
       const int base = (int)(word & 0x00ffffffu);
-#if PK_LEAF_UNROLL
-#pragma unroll LEAF_UNROLL
-#endif
+#pragma unroll 1
       for (int i = 0; i < size; i++) {
         if (COUNT) ntest += 1;
         if (EXACT) {  // the watertight test of form (1), min (t, slot)
@@ -364,8 +364,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_DYN_MINBLOCKS) k_trace_dyn(S
       cur = sp < DYN_SMEM ? sstack[sp][tid] : lstack[sp - DYN_SMEM];
     }
     if (fin) {
-      const bool hit = best_i != -1;
-      if (hit) {
+      if (best_i != -1) {
         if (!ANY) __stcs(hrec + j, make_uint4(__float_as_uint(best_t), (uint32_t)best_i, best_b, 0u));
         if (!(ANY && FUSED)) atomicOr(flags + (j >> 5), 1u << (j & 31u));
         if (COUNT) nhit += 1;
@@ -397,7 +396,10 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_DYN_MINBLOCKS) k_trace_dyn(S
 // triangles and this lane still has nodes to visit, push the triangle group
 // and test it later) cost more than it saved on the 1080p benchmark (p = 4:
 // 2669 Mrays/s, p = 8: 2569, without: 2939) and was removed.  Lanes take new rays as
-// in k_trace_dyn.  Unlike the binary traversal, letting a lane visit several
+// in k_trace_dyn, and hand in their results then, 16 or more together: the
+// environment lookup of a miss is 250 instructions (1280x720, 524,288-triangle
+// soup, four frames: 7.83 -> 7.60 ms; the binary traversal was slower so, 25.4
+// against 24.75 ms at 1080p).  Unlike the binary traversal, letting a lane visit several
 // nodes in a row before the warp meets again did not pay (1080p: one visit
 // 3102-3108 Mrays/s, up to two 2893-2900, up to four 1753-1767), and the
 // refill threshold of the binary traversal (16 idle lanes) is also best here
@@ -454,6 +456,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_CW_MINBLOCKS) k_trace_cw(Sce
   }
   uint32_t nfetch = 0, ntest = 0, nhit = 0;
   uint32_t j = 0;
+  bool pend = false;  // a result in hand, delivered when the warp takes new rays
   bool have = false, exhausted = false;
   float ox = 0.f, oy = 0.f, oz = 0.f, ix = 0.f, iy = 0.f, iz = 0.f;
   WtRay wr{};
@@ -463,10 +466,25 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_CW_MINBLOCKS) k_trace_cw(Sce
   uint32_t best_b = 0u;
   int sp = 0;
   uint2 G = make_uint2(0u, 0u), T = make_uint2(0u, 0u);
+  // The result of the lane's ray.
+  const auto deliver = [&]() {
+    if (best_i != -1) {
+      if (!ANY) __stcs(hrec + j, make_uint4(__float_as_uint(best_t), (uint32_t)best_i, best_b, 0u));
+      if (!(ANY && FUSED)) atomicOr(flags + (j >> 5), 1u << (j & 31u));
+      if (COUNT) nhit += 1;
+    } else if (FUSED) {
+      const float4 tpv = __ldcs(R.t + j), d = __ldcs(R.d + j);
+      const V3 e = env_color(env, theta, v3(d.x, d.y, d.z));
+      fused_miss<ANY>(color, npix, hrec, j, __float_as_uint(tpv.w) & 0x0fffffffu, e.x * tpv.x, e.y * tpv.y,
+                      e.z * tpv.z, defer, &ctr->err);
+    }
+  };
   for (;;) {
     const uint32_t idle = __ballot_sync(0xffffffffu, !have && !exhausted);
     const uint32_t busy = __ballot_sync(0xffffffffu, have);
     if (idle && (__popc(idle) >= REFILL_MIN || busy == 0u)) {
+      if (pend) deliver();
+      pend = false;
       const int leader = __ffs(idle) - 1;
       uint32_t base = 0;
       if (lane == leader) base = atomicAdd(ticket, (uint32_t)__popc(idle));
@@ -529,18 +547,8 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_CW_MINBLOCKS) k_trace_cw(Sce
       }
     }
     if (fin) {
-      const bool hit = best_i != -1;
-      if (hit) {
-        if (!ANY) __stcs(hrec + j, make_uint4(__float_as_uint(best_t), (uint32_t)best_i, best_b, 0u));
-        if (!(ANY && FUSED)) atomicOr(flags + (j >> 5), 1u << (j & 31u));
-        if (COUNT) nhit += 1;
-      } else if (FUSED) {
-        const float4 tpv = __ldcs(R.t + j), d = __ldcs(R.d + j);
-        const V3 e = env_color(env, theta, v3(d.x, d.y, d.z));
-        fused_miss<ANY>(color, npix, hrec, j, __float_as_uint(tpv.w) & 0x0fffffffu, e.x * tpv.x, e.y * tpv.y,
-                        e.z * tpv.z, defer, &ctr->err);
-      }
       have = false;
+      pend = true;
     }
   }
   if (COUNT) {
@@ -1272,7 +1280,7 @@ void launch_batch_next_frame(cudaStream_t s, uint32_t* frame) { k_batch_next_fra
 
 Grids kernel_grids(int sms, uint32_t capacity) {
   int t = 0, c = 0, s = 0, w = 0;
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t, k_trace_dyn<false, true, false, false>, TRACE_THREADS, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t, k_trace_dyn<false, true, false, NODES_64>, TRACE_THREADS, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&w, k_trace_cw<false, true, false>, TRACE_THREADS, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_compact<0, true, COMPACT_R_LARGE>, COMPACT_THREADS, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s, k_shade, SHADE_THREADS, 0);
@@ -1315,11 +1323,14 @@ void launch_trace(const LaunchCtx& L, bool any_hit, bool fused, bool count, cons
 #define PK_TRACED(A, F, C)                                                                                         \
   do {                                                                                                             \
     if (L.trace_mode & TRACE_EXACT)                                                                                \
-      k_trace_dyn<A, F, C, true><<<grid, block, 0, L.stream>>>(L.scene, L.env, L.ctr, countp, R, hrec, flags,       \
-                                                               L.color, L.npix, ticket, defer);                    \
+      k_trace_dyn<A, F, C, NODES_EXACT><<<grid, block, 0, L.stream>>>(L.scene, L.env, L.ctr, countp, R, hrec, flags, \
+                                                                      L.color, L.npix, ticket, defer);             \
+    else if (L.scene.inner32)                                                                                      \
+      k_trace_dyn<A, F, C, NODES_32><<<grid, block, 0, L.stream>>>(L.scene, L.env, L.ctr, countp, R, hrec, flags,   \
+                                                                   L.color, L.npix, ticket, defer);                \
     else                                                                                                           \
-      k_trace_dyn<A, F, C, false><<<grid, block, 0, L.stream>>>(L.scene, L.env, L.ctr, countp, R, hrec, flags,      \
-                                                                L.color, L.npix, ticket, defer);                   \
+      k_trace_dyn<A, F, C, NODES_64><<<grid, block, 0, L.stream>>>(L.scene, L.env, L.ctr, countp, R, hrec, flags,   \
+                                                                   L.color, L.npix, ticket, defer);                \
   } while (0)
     if (!any_hit) {
       if (fused) { if (count) PK_TRACED(false, true, true); else PK_TRACED(false, true, false); }
@@ -1332,7 +1343,14 @@ void launch_trace(const LaunchCtx& L, bool any_hit, bool fused, bool count, cons
     return;
   }
 #define PK_TRACE(A, F, C) \
-  k_trace<A, F, C><<<grid, block, 0, L.stream>>>(L.scene, L.env, L.ctr, countp, R, hrec, flags, L.color, L.npix, ticket)
+  do {                                                                                                               \
+    if (L.scene.inner32)                                                                                             \
+      k_trace<A, F, C, true><<<grid, block, 0, L.stream>>>(L.scene, L.env, L.ctr, countp, R, hrec, flags, L.color,   \
+                                                           L.npix, ticket);                                          \
+    else                                                                                                             \
+      k_trace<A, F, C, false><<<grid, block, 0, L.stream>>>(L.scene, L.env, L.ctr, countp, R, hrec, flags, L.color,  \
+                                                            L.npix, ticket);                                         \
+  } while (0)
   if (!any_hit) {
     if (fused) { if (count) PK_TRACE(false, true, true); else PK_TRACE(false, true, false); }
     else { if (count) PK_TRACE(false, false, true); else PK_TRACE(false, false, false); }

@@ -131,9 +131,10 @@ __global__ void k_inner_records(const int32_t* __restrict__ nodes5, uint32_t n, 
   decode_box(nodes5 + 5 * (size_t)l, lb);
   decode_box(nodes5 + 5 * (size_t)(l + 1), rb);
   float4* r = inner + 4 * (size_t)rank[i];
-  r[0] = make_float4(lb[0], lb[1], lb[2], lb[3]);
-  r[1] = make_float4(lb[4], lb[5], rb[0], rb[1]);
-  r[2] = make_float4(rb[2], rb[3], rb[4], rb[5]);
+  // the order of inner_children (pk_traverse.cuh)
+  r[0] = make_float4(lb[0], lb[2], lb[1], lb[3]);
+  r[1] = make_float4(lb[4], lb[5], rb[4], rb[5]);
+  r[2] = make_float4(rb[0], rb[2], rb[1], rb[3]);
   reinterpret_cast<int4*>(r)[3] = make_int4(child_code(nodes5, rank, (uint32_t)l, n_tris, err),
                                             child_code(nodes5, rank, (uint32_t)l + 1, n_tris, err), 0, 0);
 }

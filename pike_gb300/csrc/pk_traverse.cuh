@@ -10,18 +10,36 @@ constexpr float MAX_T = 100000.0f;
 // =====================================================================
 // trace.wgsl:83-189 / trace_shadow.wgsl:82-190: BVH traversal.
 // =====================================================================
-__device__ __forceinline__ float box_hit(float xa, float xb, float ya, float yb, float za, float zb, float ox,
-                                         float oy, float oz, float ix, float iy, float iz) {
-  // t1 uses the x_range.x bounds (quantised max), t2 the x_range.y bounds (min).
-  const float t1x = (xa - ox) * ix, t2x = (xb - ox) * ix;
-  const float t1y = (ya - oy) * iy, t2y = (yb - oy) * iy;
-  const float t1z = (za - oz) * iz, t2z = (zb - oz) * iz;
+// Both planes of the axes come as pairs {x, y} and {z, z} for the packed FP32
+// instructions, which round each half like the single ones and issue once for
+// two: 12 instead of 24 subtractions and multiplications per inner node.  The
+// traversals issue on half of the cycles and stall mostly on latency, so this
+// gives less than its share of the instructions (eight 1080p frames 25.8 ->
+// 25.4 ms, 16 batched requests 29.1 -> 28.4 ms; z apart, without the doubled
+// registers of {oz, oz} and {iz, iz}: 25.5 and 28.5).
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 pair_of(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+// (b - o) * i of both halves
+__device__ __forceinline__ float2 pair_dist(F2 b, F2 o, F2 i) {
+  float2 r;
+  asm("{\n\t.reg .b64 t;\n\tsub.rn.f32x2 t, %2, %3;\n\tmul.rn.f32x2 t, t, %4;\n\tmov.b64 {%0, %1}, t;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "l"(b), "l"(o), "l"(i));
+  return r;
+}
+// t1: distances {x, y} of the x_range.x, y_range.x bounds (quantised max), t2 of
+// the .y bounds (min), z both.
+__device__ __forceinline__ float box_entry(float2 t1, float2 t2, float2 z) {
   // fminf/fmaxf agree with minNum/maxNum except for the sign of a zero
   // result, which only ever feeds comparisons here.  (Three-input min/max
   // for the outer reductions measured no faster: 3709-3748 against
   // 3740-3745 Mrays/s.)
-  const float tmax = fminf(fminf(fmaxf(t1x, t2x), fmaxf(t1y, t2y)), fmaxf(t1z, t2z));
-  const float tmin = fmaxf(fmaxf(fminf(t1x, t2x), fminf(t1y, t2y)), fminf(t1z, t2z));
+  const float tmax = fminf(fminf(fmaxf(t1.x, t2.x), fmaxf(t1.y, t2.y)), fmaxf(z.x, z.y));
+  const float tmin = fmaxf(fmaxf(fminf(t1.x, t2.x), fminf(t1.y, t2.y)), fminf(z.x, z.y));
   return (tmax >= tmin && tmax > 0.0f) ? tmin : MAX_T;
 }
 
@@ -38,16 +56,6 @@ __device__ __forceinline__ float snorm16_decode(int s) {
 }
 __device__ __forceinline__ float snorm_lo(int m) { return snorm16_decode((int)(int16_t)(uint16_t)((uint32_t)m & 0xffffu)); }
 __device__ __forceinline__ float snorm_hi(int m) { return snorm16_decode((int)(int16_t)(uint16_t)((uint32_t)m >> 16)); }
-
-// One inner-node step: both children's entry distances and child codes.
-// 32-byte records keep the reference's snorm16 boxes {Lx, Ly, Lz, Rx}{Ry, Rz,
-// codeL, codeR}; 64-byte records (the default: fewer instructions per step,
-// which matters more than bytes here) hold the same boxes decoded.
-// (Prefetching both children's records into L1 while the boxes are tested
-// measured far slower at 1080p: 3188-3197 Mrays/s against 3738-3746, and
-// 2766-2769 with the leaves' first triangle too.)
-__device__ __forceinline__ void inner_children(const SceneDev& sc, int cur, float ox, float oy, float oz, float ix,
-                                               float iy, float iz, float& lh, float& rh, int& cl, int& cr);
 
 // trace.wgsl:97-114: Moller-Trumbore on one leaf-ordered triangle record
 // {v0.xyz, e1.x}{e1.yz, e2.xy}{e2.z}.  Returns false where the reference
@@ -77,42 +85,44 @@ constexpr int TRACE_THREADS = 128;
 constexpr int STACK_SMEM = 32;   // per-thread entries kept in shared memory
 // (traverse_rt keeps the remaining 64 - SSTACK entries in local memory)
 
+// One inner-node step: both children's entry distances and child codes.
+// COMPACT: 32-byte records keep the reference's snorm16 boxes {Lx, Ly, Lz, Rx}{Ry, Rz,
+// codeL, codeR}; 64-byte records (the default: fewer instructions per step,
+// which matters more than bytes here) hold the same boxes decoded.
+// (Prefetching both children's records into L1 while the boxes are tested
+// measured far slower at 1080p: 3188-3197 Mrays/s against 3738-3746, and
+// 2766-2769 with the leaves' first triangle too.)
+template <bool COMPACT>
 __device__ __forceinline__ void inner_children(const SceneDev& sc, int cur, float ox, float oy, float oz, float ix,
                                                float iy, float iz, float& lh, float& rh, int& cl, int& cr) {
-  if (sc.inner32) {
+  const F2 o = pair_of(ox, oy), i = pair_of(ix, iy), oo = pair_of(oz, oz), ii = pair_of(iz, iz);
+  if (COMPACT) {
     const int4* rec = sc.inner32 + 2 * (size_t)cur;
     const int4 q0 = __ldg(rec), q1 = __ldg(rec + 1);
-    lh = box_hit(snorm_lo(q0.x), snorm_hi(q0.x), snorm_lo(q0.y), snorm_hi(q0.y), snorm_lo(q0.z), snorm_hi(q0.z), ox,
-                 oy, oz, ix, iy, iz);
-    rh = box_hit(snorm_lo(q0.w), snorm_hi(q0.w), snorm_lo(q1.x), snorm_hi(q1.x), snorm_lo(q1.y), snorm_hi(q1.y), ox,
-                 oy, oz, ix, iy, iz);
+    lh = box_entry(pair_dist(pair_of(snorm_lo(q0.x), snorm_lo(q0.y)), o, i),
+                   pair_dist(pair_of(snorm_hi(q0.x), snorm_hi(q0.y)), o, i),
+                   pair_dist(pair_of(snorm_lo(q0.z), snorm_hi(q0.z)), oo, ii));
+    rh = box_entry(pair_dist(pair_of(snorm_lo(q0.w), snorm_lo(q1.x)), o, i),
+                   pair_dist(pair_of(snorm_hi(q0.w), snorm_hi(q1.x)), o, i),
+                   pair_dist(pair_of(snorm_lo(q1.y), snorm_hi(q1.y)), oo, ii));
     cl = q1.z;
     cr = q1.w;
-  } else {
-    const float4* rec = sc.inner + 4 * (size_t)cur;
-    const float4 a = __ldg(rec), b = __ldg(rec + 1), c4 = __ldg(rec + 2);
+  } else {  // {Lx0, Ly0, Lx1, Ly1}{Lz0, Lz1, Rz0, Rz1}{Rx0, Ry0, Rx1, Ry1}{codeL, codeR, -, -}
+    const ulonglong2* rec = reinterpret_cast<const ulonglong2*>(sc.inner + 4 * (size_t)cur);
+    const ulonglong2 a = __ldg(rec), b = __ldg(rec + 1), c = __ldg(rec + 2);
     const int4 ch = __ldg(reinterpret_cast<const int4*>(rec) + 3);
-    lh = box_hit(a.x, a.y, a.z, a.w, b.x, b.y, ox, oy, oz, ix, iy, iz);
-    rh = box_hit(b.z, b.w, c4.x, c4.y, c4.z, c4.w, ox, oy, oz, ix, iy, iz);
+    lh = box_entry(pair_dist(a.x, o, i), pair_dist(a.y, o, i), pair_dist(b.x, oo, ii));
+    rh = box_entry(pair_dist(c.x, o, i), pair_dist(c.y, o, i), pair_dist(b.y, oo, ii));
     cl = ch.x;
     cr = ch.y;
   }
 }
 
-// Leaf-loop unroll of this shared traversal: kept off, the code size costs
-// the megakernels that inline it (unrolled by 4: 64-request batch 530 against
-// 440 ms, form (3) forward 691-693 against 796-799 Mrays/s, adjoint 563
-// against 690-692).
-#ifndef PK_RT_LEAF_UNROLL
-#define PK_RT_LEAF_UNROLL 0
-#endif
-constexpr int RT_LEAF_UNROLL = PK_RT_LEAF_UNROLL;
-
 // BLOCK threads per block share `sstack` (SSTACK entries per thread in shared
 // memory, 64 - SSTACK more in local memory).  ANY: any hit (trace_shadow.wgsl)
 // rather than closest hit; a constant at every inlined call site, a run-time
 // value where one out-of-line copy serves both.
-template <bool COUNT, int BLOCK, int SSTACK>
+template <bool COUNT, int BLOCK, int SSTACK, bool COMPACT = false>
 __device__ __forceinline__ void traverse_rt(const bool ANY, const SceneDev& sc, float ox, float oy, float oz,
                                             float dx, float dy, float dz, float& best_t, int& best_i,
                                             uint32_t& best_b, int (*sstack)[BLOCK], uint32_t* err,
@@ -132,7 +142,7 @@ __device__ __forceinline__ void traverse_rt(const bool ANY, const SceneDev& sc, 
       if (COUNT) nfetch += 3;
       float lh, rh;
       int cl, cr;
-      inner_children(sc, cur, ox, oy, oz, ix, iy, iz, lh, rh, cl, cr);
+      inner_children<COMPACT>(sc, cur, ox, oy, oz, ix, iy, iz, lh, rh, cl, cr);
       const bool lok = lh < best_t, rok = rh < best_t;
       if (lok && rok) {
         int nearc, farc;
@@ -151,9 +161,6 @@ __device__ __forceinline__ void traverse_rt(const bool ANY, const SceneDev& sc, 
       const uint32_t word = (uint32_t)cur & 0x7fffffffu;
       const int size = (int)(word >> 24);
       const int base = (int)(word & 0x00ffffffu);
-#if PK_RT_LEAF_UNROLL
-#pragma unroll RT_LEAF_UNROLL
-#endif
       for (int i = 0; i < size; i++) {
         if (COUNT) ntest += 1;
         float res, u, v;
@@ -171,12 +178,12 @@ __device__ __forceinline__ void traverse_rt(const bool ANY, const SceneDev& sc, 
     cur = sp < SSTACK ? sstack[sp][tid] : lstack[sp - SSTACK];
   }
 }
-template <bool ANY, bool COUNT, int BLOCK = TRACE_THREADS, int SSTACK = STACK_SMEM>
+template <bool ANY, bool COUNT, int BLOCK = TRACE_THREADS, int SSTACK = STACK_SMEM, bool COMPACT = false>
 __device__ __forceinline__ void traverse(const SceneDev& sc, float ox, float oy, float oz, float dx, float dy,
                                          float dz, float& best_t, int& best_i, uint32_t& best_b,
                                          int (*sstack)[BLOCK], uint32_t* err, uint32_t& nfetch,
                                          uint32_t& ntest) {
-  traverse_rt<COUNT, BLOCK, SSTACK>(ANY, sc, ox, oy, oz, dx, dy, dz, best_t, best_i, best_b, sstack, err, nfetch,
+  traverse_rt<COUNT, BLOCK, SSTACK, COMPACT>(ANY, sc, ox, oy, oz, dx, dy, dz, best_t, best_i, best_b, sstack, err, nfetch,
                                     ntest);
 }
 
@@ -190,8 +197,10 @@ __device__ __forceinline__ void traverse(const SceneDev& sc, float ox, float oy,
 // callers that want the triangle; otherwise it stops at the first accepted one.
 // load(j, o, d) fetches ray j; done(j, d, t, triangle, barycentrics) takes the
 // result (triangle -1: none).
-// (Threshold, budget, stack split and leaf unroll as measured for the frame's
-// traversal, k_trace_dyn.)
+// (Threshold, budget, stack split and leaf loop as measured for the frame's
+// traversal, k_trace_dyn; 2,097,143 random rays: leaf loop unrolled by 4 476 us,
+// not unrolled 463, without the 32-byte records' code 450.  Handing results in
+// at the next refill instead of at once: 533.)
 constexpr int LANES_REFILL = 16;
 constexpr int LANES_BUDGET = 8;
 constexpr int LANES_SMEM = 8;  // stack entries per lane in shared memory, the rest of 64 in local memory
@@ -244,7 +253,7 @@ __device__ __forceinline__ void trace_lanes(const SceneDev& sc, uint32_t n, uint
     while (cur >= 0 && budget-- > 0) {
       float lh, rh;
       int cl, cr;
-      inner_children(sc, cur, ox, oy, oz, ix, iy, iz, lh, rh, cl, cr);
+      inner_children<false>(sc, cur, ox, oy, oz, ix, iy, iz, lh, rh, cl, cr);
       const bool lok = lh < best_t, rok = rh < best_t;
       if (lok && rok) {
         int nearc, farc;
@@ -266,7 +275,7 @@ __device__ __forceinline__ void trace_lanes(const SceneDev& sc, uint32_t n, uint
       const uint32_t word = (uint32_t)cur & 0x7fffffffu;
       const int size = (int)(word >> 24);
       const int base = (int)(word & 0x00ffffffu);
-#pragma unroll 4
+#pragma unroll 1
       for (int i = 0; i < size; i++) {
         float res, u, v;
         if (!mt_test(sc, base + i, ox, oy, oz, dx, dy, dz, eps, res, u, v)) continue;

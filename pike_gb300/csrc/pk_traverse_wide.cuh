@@ -9,6 +9,7 @@
 // oracle's brute force) return the same bits.
 #pragma once
 #include "pk_internal.cuh"
+#include "pk_traverse.cuh"
 
 namespace pk {
 
@@ -62,6 +63,21 @@ __device__ __forceinline__ WtRay wt_setup(float ox, float oy, float oz, float dx
   return w;
 }
 
+// A vertex relative to the origin, sheared along the ray: (x, y) - o - s * z.
+// The last subtraction stays single: a packed one after the packed product
+// came out fused with it, rounded once.  (The soup's frames: 7.95 ms with
+// single instructions, 7.92 with the packed subtraction, 7.83 with both.)
+__device__ __forceinline__ float2 wt_shear(float x, float y, F2 o, F2 s, float z) {
+  float2 t, u;
+  asm("{\n\t.reg .b64 t;\n\tsub.rn.f32x2 t, %2, %3;\n\tmov.b64 {%0, %1}, t;\n\t}"
+      : "=f"(t.x), "=f"(t.y)
+      : "l"(pair_of(x, y)), "l"(o));
+  asm("{\n\t.reg .b64 t;\n\tmul.rn.f32x2 t, %2, %3;\n\tmov.b64 {%0, %1}, t;\n\t}"
+      : "=f"(u.x), "=f"(u.y)
+      : "l"(s), "l"(pair_of(z, z)));
+  return make_float2(__fsub_rn(t.x, u.x), __fsub_rn(t.y, u.y));
+}
+
 // The watertight test on one triangle record {v0.xyz, v1.x}{v1.yz, v2.xy}
 // {v2.z, slot, -, -}: false when rejected; otherwise t = T/det (accepted when
 // t > eps, eps = the pass's EPSILON: 1e-8 closest, 1e-7 any hit) and the
@@ -73,16 +89,14 @@ __device__ __forceinline__ bool wt_test(const float4* __restrict__ tris, uint32_
                                         float& t, float& u, float& v, uint32_t& slot) {
   const float4* tp = tris + 3 * (size_t)rec;
   const float4 P = __ldg(tp), Q = __ldg(tp + 1), R = __ldg(tp + 2);
-  // A = v0 - o, B = v1 - o, C = v2 - o in the permuted frame
-  const float Akx = sel3(P.x, P.y, P.z, r.kx) - r.ox, Aky = sel3(P.x, P.y, P.z, r.ky) - r.oy,
-              Akz = sel3(P.x, P.y, P.z, r.kz) - r.oz;
-  const float Bkx = sel3(P.w, Q.x, Q.y, r.kx) - r.ox, Bky = sel3(P.w, Q.x, Q.y, r.ky) - r.oy,
-              Bkz = sel3(P.w, Q.x, Q.y, r.kz) - r.oz;
-  const float Ckx = sel3(Q.z, Q.w, R.x, r.kx) - r.ox, Cky = sel3(Q.z, Q.w, R.x, r.ky) - r.oy,
+  // A = v0 - o, B = v1 - o, C = v2 - o in the permuted frame, sheared
+  const F2 oxy = pair_of(r.ox, r.oy), sxy = pair_of(r.sx, r.sy);
+  const float Akz = sel3(P.x, P.y, P.z, r.kz) - r.oz, Bkz = sel3(P.w, Q.x, Q.y, r.kz) - r.oz,
               Ckz = sel3(Q.z, Q.w, R.x, r.kz) - r.oz;
-  const float Ax = Akx - r.sx * Akz, Ay = Aky - r.sy * Akz;
-  const float Bx = Bkx - r.sx * Bkz, By = Bky - r.sy * Bkz;
-  const float Cx = Ckx - r.sx * Ckz, Cy = Cky - r.sy * Ckz;
+  const float2 A = wt_shear(sel3(P.x, P.y, P.z, r.kx), sel3(P.x, P.y, P.z, r.ky), oxy, sxy, Akz);
+  const float2 B = wt_shear(sel3(P.w, Q.x, Q.y, r.kx), sel3(P.w, Q.x, Q.y, r.ky), oxy, sxy, Bkz);
+  const float2 C = wt_shear(sel3(Q.z, Q.w, R.x, r.kx), sel3(Q.z, Q.w, R.x, r.ky), oxy, sxy, Ckz);
+  const float Ax = A.x, Ay = A.y, Bx = B.x, By = B.y, Cx = C.x, Cy = C.y;
   float U = Cx * By - Cy * Bx;
   float V = Ax * Cy - Ay * Cx;
   float W = Bx * Ay - By * Ax;
@@ -104,10 +118,20 @@ __device__ __forceinline__ bool wt_test(const float4* __restrict__ tris, uint32_
   return true;
 }
 
-// Byte k of `word` as a float.  (Building the float 2^23 + byte by a byte
-// permute and subtracting 2^23, instead of the conversion instruction, was
-// measured no faster: 2966-2990 against 2980-2984 Mrays/s.)
-__device__ __forceinline__ float byte_float(uint32_t word, int k) { return (float)((word >> (8 * k)) & 0xffu); }
+// Entry and exit distances q * b + a of one axis of child k, q its near and far
+// byte.  The bytes become the floats 2^23 + q by a byte permute, and the exact
+// subtraction and the FMA are packed pairs: per pair 4 instructions and no
+// conversion unit (1280x720, 524,288-triangle soup, four frames: 8.10 ms with
+// conversions and single FMAs, 7.98 with conversions and packed FMAs, 7.95 so).
+__device__ __forceinline__ float2 cw_planes(uint32_t n, uint32_t f, int k, F2 b, F2 a) {
+  const F2 q = pair_of(__uint_as_float(__byte_perm(n, 0x4b000000u, 0x7440u | (unsigned)k)),
+                       __uint_as_float(__byte_perm(f, 0x4b000000u, 0x7440u | (unsigned)k)));
+  float2 r;
+  asm("{\n\t.reg .b64 t;\n\tadd.rn.f32x2 t, %2, %3;\n\tfma.rn.f32x2 t, t, %4, %5;\n\tmov.b64 {%0, %1}, t;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "l"(q), "l"(pair_of(-8388608.0f, -8388608.0f)), "l"(b), "l"(a));
+  return r;
+}
 
 // Child test of one compressed wide node (pk_wide.h).  Returns the node's
 // internal-child hit mask, with the child of slot s at bit (s ^ oct) (the
@@ -152,19 +176,18 @@ __device__ __forceinline__ void cw_node(const float4* __restrict__ nodes, uint32
   // per-child tests with the masks built inside the loop: 1080p frame
   // 3348-3352 against 3292-3301 Mrays/s, closest-hit launch 0.376 against
   // 0.385 ms.
+  const F2 axx = pair_of(ax, ax), ayy = pair_of(ay, ay), azz = pair_of(az, az);
+  const F2 bxx = pair_of(bx, bx), byy = pair_of(by, by), bzz = pair_of(bz, bz);
   uint32_t hb = 0u;
 #pragma unroll
   for (int k = 0; k < 8; k++) {
     const int kb = k & 3;
-    const float tnx = __fmaf_rn(byte_float(k < 4 ? nx0 : nx1, kb), bx, ax);
-    const float tny = __fmaf_rn(byte_float(k < 4 ? ny0 : ny1, kb), by, ay);
-    const float tnz = __fmaf_rn(byte_float(k < 4 ? nz0 : nz1, kb), bz, az);
-    const float tfx = __fmaf_rn(byte_float(k < 4 ? fx0 : fx1, kb), bx, ax);
-    const float tfy = __fmaf_rn(byte_float(k < 4 ? fy0 : fy1, kb), by, ay);
-    const float tfz = __fmaf_rn(byte_float(k < 4 ? fz0 : fz1, kb), bz, az);
-    const float tmax = min3f(tfx, tfy, tfz);
+    const float2 tx = cw_planes(k < 4 ? nx0 : nx1, k < 4 ? fx0 : fx1, kb, bxx, axx);
+    const float2 ty = cw_planes(k < 4 ? ny0 : ny1, k < 4 ? fy0 : fy1, kb, byy, ayy);
+    const float2 tz = cw_planes(k < 4 ? nz0 : nz1, k < 4 ? fz0 : fz1, kb, bzz, azz);
+    const float tmax = min3f(tx.y, ty.y, tz.y);
     const float hi = fminf(__fmaf_rn(fabsf(tmax), WIDE_SLACK, tmax), cull_s);
-    if (fmaxf(max3f(tnx, tny, tnz), 0.0f) <= hi) hb |= 1u << k;
+    if (fmaxf(max3f(tx.x, ty.x, tz.x), 0.0f) <= hi) hb |= 1u << k;
   }
   // internal children: slot k -> visiting position k ^ oct
   uint32_t x = hb & imask;
