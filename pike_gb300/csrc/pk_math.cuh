@@ -189,37 +189,62 @@ __device__ __forceinline__ float log2_(float x) {
 __device__ __forceinline__ float pow_(float x, float y) { return exp2_(y * log2_(x)); }
 
 // ---- WGSL data packing ---------------------------------------------------
-// v / d for an integer-valued v by a constant d: the product with r = RN(1/d)
-// corrected by one FMA with the exact residual v - q0 d.  For the domains
-// used below (v in [-128, 127] by 127, [0, 255] by 255, [0, 65535] by 65535,
-// [-32768, 32767] by 32767) this equals the IEEE quotient for every input
-// (the GPU tests check each domain exhaustively); it replaces an IEEE division
-// (a longer inline sequence with a slow-path call) at some 45 sites per hit.
-__device__ __forceinline__ float qdiv(float v, float d, float r) {
-  const float q0 = __fmul_rn(v, r);
-  return __fmaf_rn(__fmaf_rn(-q0, d, v), r, q0);
+// v / d for an integer-valued v by a constant d: v times 1/d held as the sum of
+// two floats, R + R2, one rounding at the end.  For the domains used below (v
+// in [-127, 127] by 127, [0, 255] by 255, [0, 65535] by 65535, [-32767, 32767]
+// by 32767) this equals the IEEE quotient for every input (the GPU tests check
+// each domain exhaustively); it replaces an IEEE division (a longer inline
+// sequence with a slow-path call) at some 45 sites per hit.
+struct Recip {
+  float r, r2;
+};
+constexpr Recip R127 = {0x1.020408p-7f, 0x1.020408p-35f}, R255 = {0x1.010102p-8f, -0x1.fdfdfep-33f},
+                R65535 = {0x1.0001p-16f, 0x1.0001p-48f}, R32767 = {0x1.0002p-15f, 0x1.0002p-45f};
+__device__ __forceinline__ float qdiv(float v, Recip d) { return __fmaf_rn(v, d.r, __fmul_rn(v, d.r2)); }
+// Packed FP32: two binary32 operations in one instruction, each rounded like the
+// single one.
+using F2 = unsigned long long;
+__device__ __forceinline__ F2 pair_of(float x, float y) {
+  F2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 pair_qdiv(float x, float y, Recip d) {
+  float2 r;
+  asm("{\n\t.reg .b64 t;\n\tmul.rn.f32x2 t, %2, %4;\n\tfma.rn.f32x2 t, %2, %3, t;\n\tmov.b64 {%0, %1}, t;\n\t}"
+      : "=f"(r.x), "=f"(r.y)
+      : "l"(pair_of(x, y)), "l"(pair_of(d.r, d.r)), "l"(pair_of(d.r2, d.r2)));
+  return r;
 }
 // Small integers to float without the conversion instruction (a quarter of the
 // rate): 2^23 + v is the float with v in its low mantissa bits, and the
 // subtraction is exact.  byte_f: byte k of w; u16_f: v < 2^16.
 template <int K>
-__device__ __forceinline__ float byte_f(uint32_t w) {
-  return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u + K)) - 8388608.0f;
+__device__ __forceinline__ float byte_magic(uint32_t w) {
+  return __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u + K));
 }
+template <int K>
+__device__ __forceinline__ float byte_f(uint32_t w) { return byte_magic<K>(w) - 8388608.0f; }
 __device__ __forceinline__ float u16_f(uint32_t v) { return __uint_as_float(0x4b000000u | v) - 8388608.0f; }
 // Components of unpack4x8snorm: byte K of w, with w's bytes offset by 128
 // (w ^ 0x80808080); max(v, -127) / 127 is max(v / 127, -1).
 template <int K>
 __device__ __forceinline__ float snorm8_offset(uint32_t w) {
-  const float v = __uint_as_float(__byte_perm(w, 0x4b000000u, 0x7440u + K)) - 8388736.0f;
-  return qdiv(fmaxf(v, -127.0f), 127.0f, 0x1.020408p-7f);
+  return qdiv(fmaxf(byte_magic<K>(w) - 8388736.0f, -127.0f), R127);
+}
+// Bytes KA of wa and KB of wb: 7 instructions for two instead of 10.
+template <int KA, int KB>
+__device__ __forceinline__ float2 snorm8_pair(uint32_t wa, uint32_t wb) {
+  float2 v;
+  asm("{\n\t.reg .b64 t;\n\tadd.rn.f32x2 t, %2, %3;\n\tmov.b64 {%0, %1}, t;\n\t}"
+      : "=f"(v.x), "=f"(v.y)
+      : "l"(pair_of(byte_magic<KA>(wa), byte_magic<KB>(wb))), "l"(pair_of(-8388736.0f, -8388736.0f)));
+  return pair_qdiv(fmaxf(v.x, -127.0f), fmaxf(v.y, -127.0f), R127);
 }
 template <int K>
-__device__ __forceinline__ float unorm8_byte(uint32_t w) {
-  return qdiv(byte_f<K>(w), 255.0f, 0x1.010102p-8f);
-}
-__device__ __forceinline__ float unorm16(uint32_t v) { return qdiv(u16_f(v), 65535.0f, 0x1.0001p-16f); }  // v < 2^16
-__device__ __forceinline__ float snorm16(int v) { return fmax_(qdiv((float)v, 32767.0f, 0x1.0002p-15f), -1.0f); }
+__device__ __forceinline__ float unorm8_byte(uint32_t w) { return qdiv(byte_f<K>(w), R255); }
+__device__ __forceinline__ float unorm16(uint32_t v) { return qdiv(u16_f(v), R65535); }  // v < 2^16
+__device__ __forceinline__ float snorm16(int v) { return fmax_(qdiv((float)v, R32767), -1.0f); }
 __device__ __forceinline__ uint32_t pack_unorm16(float e) {
   return (uint32_t)floorf(0.5f + 65535.0f * fmin_(1.0f, fmax_(0.0f, e)));
 }

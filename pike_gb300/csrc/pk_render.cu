@@ -768,7 +768,7 @@ __device__ __forceinline__ bool shade_one(const SceneDev& sc, const EnvDev& env,
     } else {
       bs.wi = reflect(neg(si.wo), m);
       bs.pdf = specular_pdf(si, m);
-      bsdf = eval_specular(si, bs);
+      bsdf = eval_specular(si, bs, normalize(add(si.wo, bs.wi)));
     }
     if (bs.wi.z > 0.0f) {
       const V3 dir = matvec(si.b1, si.b2, si.n, bs.wi);
@@ -787,7 +787,7 @@ __device__ __forceinline__ bool shade_one(const SceneDev& sc, const EnvDev& env,
         V3 scv = scale(v3((1.0f - f) * el.x, (1.0f - f) * el.y, (1.0f - f) * el.z), lw);
         const V3 hv = normalize(add(si.wo, es_.wi));
         const float sw = power_heuristic(es_.pdf, specular_pdf(si, hv));
-        const V3 ev = eval_specular(si, es_);
+        const V3 ev = eval_specular(si, es_, hv);
         scv = add(scv, scale(v3(f * ev.x, f * ev.y, f * ev.z), sw));
         const V3 sdir = matvec(si.b1, si.b2, si.n, es_.wi);
         es = true;
@@ -1039,8 +1039,8 @@ __global__ void k_math(int fn, const float* __restrict__ x, const float* __restr
       const uint32_t v = (uint32_t)__float_as_int(a) & 0xffu, w = v << (8 * (i & 3u));
       const uint32_t o = w ^ 0x80808080u;
       switch (i & 3u) {
-        case 0: r = fn == 9 ? snorm8_offset<0>(o) : unorm8_byte<0>(w); break;
-        case 1: r = fn == 9 ? snorm8_offset<1>(o) : unorm8_byte<1>(w); break;
+        case 0: r = fn == 9 ? snorm8_pair<0, 1>(o, o).x : unorm8_byte<0>(w); break;
+        case 1: r = fn == 9 ? snorm8_pair<0, 1>(o, o).y : unorm8_byte<1>(w); break;
         case 2: r = fn == 9 ? snorm8_offset<2>(o) : unorm8_byte<2>(w); break;
         default: r = fn == 9 ? snorm8_offset<3>(o) : unorm8_byte<3>(w);
       }

@@ -68,12 +68,22 @@ __device__ __forceinline__ void camera_ray(const CamState& cam, const CamBasis& 
 // =====================================================================
 // shade_miss.wgsl:37-43 envColor: nearest texel with repeat addressing.
 // =====================================================================
+// floor(f) modulo n, as ((i % n) + n) % n of i = f2i(floor(f)): the two integer
+// divisions by a run-time n are some 50 instructions, one quotient estimate (off
+// by at most one) and an exact remainder in floats are nine.
+__device__ __forceinline__ int wrap_floor(float f, int n) {
+  const float g = floorf(f), fn = (float)n;
+  if (fabsf(g) < 4194304.0f && n < 4194304) {
+    const float r = __fmaf_rn(-floorf(g * __fdividef(1.0f, fn)), fn, g);
+    return (int)(r < 0.0f ? r + fn : (r >= fn ? r - fn : r));
+  }
+  const int i = f2i(g);
+  return ((i % n) + n) % n;
+}
 __device__ __forceinline__ V3 env_color(const EnvDev& env, float theta, V3 dir) {
   const float u = theta + atan2_(dir.z, dir.x) / c::TAU;
   const float v = acos_(dir.y) * c::INV_PI;
-  int x = f2i(floorf(u * (float)env.w)), y = f2i(floorf(v * (float)env.h));
-  x = ((x % env.w) + env.w) % env.w;
-  y = ((y % env.h) + env.h) % env.h;
+  const int x = wrap_floor(u * (float)env.w, env.w), y = wrap_floor(v * (float)env.h, env.h);
   const uint32_t cc = __ldg(reinterpret_cast<const uint32_t*>(env.rgbe) + ((size_t)y * env.w + x));
   const float r = unorm8_byte<0>(cc), g = unorm8_byte<1>(cc), b = unorm8_byte<2>(cc), a = unorm8_byte<3>(cc);
   const float p = pow_(2.0f, a * 255.0f - 128.0f);
@@ -117,11 +127,14 @@ __device__ __forceinline__ float4 texel(const SceneDev& sc, int layer, float u, 
   return make_float4(mix1(mix1(a.x, b.x, fx), mix1(c.x, d.x, fx), fy), mix1(mix1(a.y, b.y, fx), mix1(c.y, d.y, fx), fy),
                      mix1(mix1(a.z, b.z, fx), mix1(c.z, d.z, fx), fy), mix1(mix1(a.w, b.w, fx), mix1(c.w, d.w, fx), fy));
 }
-__device__ __forceinline__ void unpack_snorm8x3(uint32_t w, V3& o) {
-  w ^= 0x80808080u;
-  o.x = snorm8_offset<0>(w);
-  o.y = snorm8_offset<1>(w);
-  o.z = snorm8_offset<2>(w);
+// Tangent, bitangent and normal of a vertex (three snorm8 each).
+__device__ __forceinline__ void unpack_frame(uint4 a, V3& t, V3& b, V3& n) {
+  const uint32_t wt = a.x ^ 0x80808080u, wb = a.y ^ 0x80808080u, wn = a.z ^ 0x80808080u;
+  const float2 txy = snorm8_pair<0, 1>(wt, wt), bxy = snorm8_pair<0, 1>(wb, wb), nxy = snorm8_pair<0, 1>(wn, wn);
+  const float2 tbz = snorm8_pair<2, 2>(wt, wb);
+  t = v3(txy.x, txy.y, tbz.x);
+  b = v3(bxy.x, bxy.y, tbz.y);
+  n = v3(nxy.x, nxy.y, snorm8_offset<2>(wn));
 }
 // branchlessONB (:166-177)
 __device__ __forceinline__ void onb(V3 n, V3& b1, V3& b2) {
@@ -141,9 +154,9 @@ __device__ __forceinline__ SI surface(const SceneDev& sc, V3 ro, V3 rd, float t,
   const V3 bary = v3(1.0f - u - v, u, v);
   const uint4 a0 = __ldg(sc.attrs + tri.x), a1 = __ldg(sc.attrs + tri.y), a2 = __ldg(sc.attrs + tri.z);
   V3 t0, t1, t2, q0, q1, q2, n0, n1, n2;
-  unpack_snorm8x3(a0.x, t0); unpack_snorm8x3(a1.x, t1); unpack_snorm8x3(a2.x, t2);
-  unpack_snorm8x3(a0.y, q0); unpack_snorm8x3(a1.y, q1); unpack_snorm8x3(a2.y, q2);
-  unpack_snorm8x3(a0.z, n0); unpack_snorm8x3(a1.z, n1); unpack_snorm8x3(a2.z, n2);
+  unpack_frame(a0, t0, q0, n0);
+  unpack_frame(a1, t1, q1, n1);
+  unpack_frame(a2, t2, q2, n2);
   const V3 T = normalize(matvec(t0, t1, t2, bary));
   const V3 B = normalize(matvec(q0, q1, q2, bary));
   const V3 N = normalize(matvec(n0, n1, n2, bary));
@@ -239,9 +252,11 @@ __device__ __forceinline__ float specular_pdf(const SI& si, V3 m) {
   const float a = si.alpha;
   return fmax_(SHADE_EPS, ggx_d(m, a, a) * ggx_g1(si.wo, m, a, a) / (4.0f * si.wo.z));
 }
-__device__ __forceinline__ V3 eval_specular(const SI& si, const Sample& s) {
+// hv: normalize(wo + wi), which the caller's specular_pdf of an environment
+// sample needs too (the compiler does not merge calls, so D and G1 of wo came
+// twice with it).
+__device__ __forceinline__ V3 eval_specular(const SI& si, const Sample& s, V3 hv) {
   const float a = si.alpha;
-  const V3 hv = normalize(add(si.wo, s.wi));
   const float D = ggx_d(hv, a, a);
   const float G = ggx_g1(s.wi, hv, a, a) * ggx_g1(si.wo, hv, a, a);
   const float k = fmax_(D * G / (4.0f * si.wo.z * s.pdf), 0.0f);

@@ -17,12 +17,6 @@ constexpr float MAX_T = 100000.0f;
 // gives less than its share of the instructions (eight 1080p frames 25.8 ->
 // 25.4 ms, 16 batched requests 29.1 -> 28.4 ms; z apart, without the doubled
 // registers of {oz, oz} and {iz, iz}: 25.5 and 28.5).
-using F2 = unsigned long long;
-__device__ __forceinline__ F2 pair_of(float x, float y) {
-  F2 r;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
-  return r;
-}
 // (b - o) * i of both halves
 __device__ __forceinline__ float2 pair_dist(F2 b, F2 o, F2 i) {
   float2 r;
@@ -43,17 +37,9 @@ __device__ __forceinline__ float box_entry(float2 t1, float2 t2, float2 z) {
   return (tmax >= tmin && tmax > 0.0f) ? tmin : MAX_T;
 }
 
-// unpack2x16snorm component: max(s / 32767, -1).  For integer s in
-// [-32768, 32767] the product with RN(1/32767) corrected by two FMAs equals the
-// IEEE quotient for every input (the tests check all 65536), so this is the
-// same value the reference decode and the 64-byte records hold.
-__device__ __forceinline__ float snorm16_decode(int s) {
-  const float sf = (float)s;
-  const float r = 0x1.0002p-15f;
-  const float q0 = sf * r;
-  const float e = __fmaf_rn(-q0, 32767.0f, sf);
-  return fmax_(__fmaf_rn(e, r, q0), -1.0f);
-}
+// unpack2x16snorm component: max(s / 32767, -1), the value the reference decode
+// and the 64-byte records hold (the tests check all 65536).
+__device__ __forceinline__ float snorm16_decode(int s) { return snorm16(s); }
 __device__ __forceinline__ float snorm_lo(int m) { return snorm16_decode((int)(int16_t)(uint16_t)((uint32_t)m & 0xffffu)); }
 __device__ __forceinline__ float snorm_hi(int m) { return snorm16_decode((int)(int16_t)(uint16_t)((uint32_t)m >> 16)); }
 
