@@ -164,6 +164,6 @@ class Batch:
 
     def image(self, i: int) -> np.ndarray:
         r = self.requests[i]
-        out = np.zeros((r.height, r.width, 4), np.float32)
+        out = np.empty((r.height, r.width, 4), np.float32)
         self._call("pk_batch_read", i, ptr(out))
         return out

@@ -320,11 +320,17 @@ int pk_scene_upload(pk_ctx* c, const int32_t* tri4, uint32_t n_tris, const doubl
   });
 }
 
+// Enqueues a copy into a caller's buffer.
+static void to_host(pk_ctx* c, void* dst, const void* src, size_t bytes) {
+  touch_pages(dst, bytes);
+  check(cudaMemcpyAsync(dst, src, bytes, cudaMemcpyDeviceToHost, c->stream), "D2H");
+}
+
 int pk_scene_download(pk_ctx* c, double* pos3, uint32_t* attr4) {
   return guarded(c, [&]() {
     if (!c->attrs.p) return fail(c, PK_ERR_STATE, "no scene");
-    if (pos3) check(cudaMemcpyAsync(pos3, c->pos.p, c->pos.bytes(), cudaMemcpyDeviceToHost, c->stream), "D2H");
-    if (attr4) check(cudaMemcpyAsync(attr4, c->attrs.p, c->attrs.bytes(), cudaMemcpyDeviceToHost, c->stream), "D2H");
+    if (pos3) to_host(c, pos3, c->pos.p, c->pos.bytes());
+    if (attr4) to_host(c, attr4, c->attrs.p, c->attrs.bytes());
     check(cudaStreamSynchronize(c->stream), "sync");
     return PK_OK;
   });
@@ -378,9 +384,9 @@ int pk_materials_download(pk_ctx* c, uint32_t* n_mats, uint32_t* n_layers, int32
   return guarded(c, [&]() {
     if (n_mats) *n_mats = c->n_mats;
     if (n_layers) *n_layers = c->n_layers;
-    if (mat4 && c->n_mats) check(cudaMemcpyAsync(mat4, c->mat4.p, c->mat4.bytes(), cudaMemcpyDeviceToHost, c->stream), "D2H");
+    if (mat4 && c->n_mats) to_host(c, mat4, c->mat4.p, c->mat4.bytes());
     if (layers && c->n_layers && c->atlas_res == 1)
-      check(cudaMemcpyAsync(layers, c->layers.p, c->layers.bytes(), cudaMemcpyDeviceToHost, c->stream), "D2H");
+      to_host(c, layers, c->layers.p, c->layers.bytes());
     check(cudaStreamSynchronize(c->stream), "sync");
     return PK_OK;
   });
@@ -465,9 +471,10 @@ int pk_wide_download(pk_ctx* c, float* nodes20, float* tris12) {
   return guarded(c, [&]() {
     if (!c->wide_ready) return fail(c, PK_ERR_STATE, "no wide BVH");
     if (!nodes20) return fail(c, PK_ERR_ARG, "null output");
-    check(cudaMemcpy(nodes20, c->wide.p, 80 * (size_t)c->wide_nodes, cudaMemcpyDeviceToHost), "D2H");
+    to_host(c, nodes20, c->wide.p, 80 * (size_t)c->wide_nodes);
     if (tris12 && c->n_leaf_tris)
-      check(cudaMemcpy(tris12, c->wide_tris.p, 48 * (size_t)c->n_leaf_tris, cudaMemcpyDeviceToHost), "D2H");
+      to_host(c, tris12, c->wide_tris.p, 48 * (size_t)c->n_leaf_tris);
+    check(cudaStreamSynchronize(c->stream), "sync");
     return PK_OK;
   });
 }
@@ -476,9 +483,10 @@ int pk_exact_download(pk_ctx* c, float* records16, float* tris12, int32_t* root_
   return guarded(c, [&]() {
     if (!c->exact_ready) return fail(c, PK_ERR_STATE, "no FP32 binary records: set PK_TRACE_EXACT after building a BVH");
     if (!records16 || !root_code) return fail(c, PK_ERR_ARG, "null output");
-    check(cudaMemcpy(records16, c->exact.p, c->exact.bytes(), cudaMemcpyDeviceToHost), "D2H");
+    to_host(c, records16, c->exact.p, c->exact.bytes());
     if (tris12 && c->n_leaf_tris)
-      check(cudaMemcpy(tris12, c->exact_tris.p, 48 * (size_t)c->n_leaf_tris, cudaMemcpyDeviceToHost), "D2H");
+      to_host(c, tris12, c->exact_tris.p, 48 * (size_t)c->n_leaf_tris);
+    check(cudaStreamSynchronize(c->stream), "sync");
     *root_code = c->exact_root;
     return PK_OK;
   });
@@ -535,10 +543,10 @@ int pk_bvh_info(pk_ctx* c, uint32_t* n_nodes, uint32_t* n_leaf_tris, double norm
 int pk_bvh_download(pk_ctx* c, int32_t* nodes5, int32_t* tri4_leaf, float* verts4) {
   return guarded(c, [&]() {
     if (!c->bvh_ready) return fail(c, PK_ERR_STATE, "no BVH");
-    if (nodes5) check(cudaMemcpyAsync(nodes5, c->nodes5.p, c->nodes5.bytes(), cudaMemcpyDeviceToHost, c->stream), "D2H");
+    if (nodes5) to_host(c, nodes5, c->nodes5.p, c->nodes5.bytes());
     if (tri4_leaf && c->n_leaf_tris)
-      check(cudaMemcpyAsync(tri4_leaf, c->tri4_leaf.p, c->tri4_leaf.bytes(), cudaMemcpyDeviceToHost, c->stream), "D2H");
-    if (verts4) check(cudaMemcpyAsync(verts4, c->verts4.p, c->verts4.bytes(), cudaMemcpyDeviceToHost, c->stream), "D2H");
+      to_host(c, tri4_leaf, c->tri4_leaf.p, c->tri4_leaf.bytes());
+    if (verts4) to_host(c, verts4, c->verts4.p, c->verts4.bytes());
     check(cudaStreamSynchronize(c->stream), "sync");
     return PK_OK;
   });
@@ -609,8 +617,8 @@ int pk_env_alias_download(pk_ctx* c, uint32_t* table2, float* pdf) {
   return guarded(c, [&]() {
     if (!c->alias_ready) return fail(c, PK_ERR_STATE, "no alias table: set PK_ENV_ALIAS first");
     const size_t N = (size_t)c->env_w * c->env_h;
-    if (table2) check(cudaMemcpyAsync(table2, c->env_alias.p, 8 * N, cudaMemcpyDeviceToHost, c->stream), "D2H");
-    if (pdf) check(cudaMemcpyAsync(pdf, c->alias_pdf.p, 4 * N, cudaMemcpyDeviceToHost, c->stream), "D2H");
+    if (table2) to_host(c, table2, c->env_alias.p, 8 * N);
+    if (pdf) to_host(c, pdf, c->alias_pdf.p, 4 * N);
     check(cudaStreamSynchronize(c->stream), "sync");
     return PK_OK;
   });
@@ -643,9 +651,9 @@ int pk_env_info(pk_ctx* c, uint32_t* w, uint32_t* h, uint32_t* nb) {
 int pk_env_download(pk_ctx* c, int32_t* bins2, int32_t* coords2, float* pdf) {
   return guarded(c, [&]() {
     if (!c->env_ready) return fail(c, PK_ERR_STATE, "no environment");
-    if (bins2) check(cudaMemcpyAsync(bins2, c->bins.p, c->bins.bytes(), cudaMemcpyDeviceToHost, c->stream), "D2H");
-    if (coords2) check(cudaMemcpyAsync(coords2, c->coords.p, c->coords.bytes(), cudaMemcpyDeviceToHost, c->stream), "D2H");
-    if (pdf) check(cudaMemcpyAsync(pdf, c->pdf.p, c->pdf.bytes(), cudaMemcpyDeviceToHost, c->stream), "D2H");
+    if (bins2) to_host(c, bins2, c->bins.p, c->bins.bytes());
+    if (coords2) to_host(c, coords2, c->coords.p, c->coords.bytes());
+    if (pdf) to_host(c, pdf, c->pdf.p, c->pdf.bytes());
     check(cudaStreamSynchronize(c->stream), "sync");
     return PK_OK;
   });
@@ -1127,8 +1135,8 @@ static int read_px(pk_ctx* c, const void* src, void* dst, size_t bytes) {
   return guarded(c, [&]() {
     require_config(c);
     if (!dst) return fail(c, PK_ERR_ARG, "null output");
+    to_host(c, dst, src, bytes);
     check(cudaStreamSynchronize(c->stream), "sync");
-    check(cudaMemcpy(dst, src, bytes, cudaMemcpyDeviceToHost), "D2H");
     return PK_OK;
   });
 }
@@ -1148,9 +1156,9 @@ int pk_write_accum(pk_ctx* c, const float* in) {
 int pk_read_display(pk_ctx* c, float* out, uint8_t* out8) {
   return guarded(c, [&]() {
     require_config(c);
+    if (out) to_host(c, out, c->display.p, c->display.bytes());
+    if (out8) to_host(c, out8, c->display8.p, c->display8.bytes());
     check(cudaStreamSynchronize(c->stream), "sync");
-    if (out) check(cudaMemcpy(out, c->display.p, c->display.bytes(), cudaMemcpyDeviceToHost), "D2H");
-    if (out8) check(cudaMemcpy(out8, c->display8.p, c->display8.bytes(), cudaMemcpyDeviceToHost), "D2H");
     return PK_OK;
   });
 }

@@ -27,6 +27,7 @@ struct pk_batch {
   DevBuf<BatchScene> d_scenes;
   DevBuf<BatchReq> d_reqs;
   DevBuf<float4> accum;
+  DevBuf<float4> mean;  // staging of pk_batch_read
   DevBuf<unsigned long long> counter;
   DevBuf<uint32_t> frame, errflag;
   DevBuf<unsigned long long> remaining, remaining_init, done_ns;  // per request; done_ns[n] = launch start
@@ -81,6 +82,16 @@ void enqueue_frame(pk_batch* b, const BatchConfig& c, unsigned grid, unsigned lo
   check(cudaGetLastError(), "k_batch");
   launch_batch_next_frame(b->stream, b->frame.p);
 }
+
+// Means of n accumulated pixels.
+__global__ void __launch_bounds__(256) k_batch_mean(const float4* __restrict__ sum, float4* __restrict__ out,
+                                                    uint32_t n, float inv) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i >= n) return;
+  const float4 s = sum[i];
+  out[i] = make_float4(s.x * inv, s.y * inv, s.z * inv, s.w * inv);
+}
+constexpr size_t MEAN_PIXELS = 1u << 20;  // staged at a time (16 MB)
 
 void reset_accum(pk_batch* b) {
   if (b->accum.p) check(cudaMemsetAsync(b->accum.p, 0, b->accum.bytes(), b->stream), "memset");
@@ -140,6 +151,7 @@ int pk_batch_destroy(pk_batch* b) {
   b->d_scenes.release();
   b->d_reqs.release();
   b->accum.release();
+  b->mean.release();
   b->counter.release();
   b->frame.release();
   b->errflag.release();
@@ -293,12 +305,30 @@ int pk_batch_read(pk_batch* b, uint32_t req, float* rgba_mean) {
   return bguard(b, [&]() {
     if (req >= b->reqs.size() || !rgba_mean) return bfail(b, PK_ERR_ARG, "bad request index or null output");
     const BatchReq& q = b->reqs[req];
-    const size_t n = (size_t)q.W * q.H;
-    check(cudaMemcpyAsync(rgba_mean, b->accum.p + q.out_offset, n * 16, cudaMemcpyDeviceToHost, b->stream), "D2H");
-    check(cudaStreamSynchronize(b->stream), "sync");
+    // Scaled on the GPU (49 MB of 16 requests, into pages in use: 3.7 ms with the
+    // host's multiplications, 0.65 so), copied into pages this thread has touched.
+    const size_t n = (size_t)q.W * q.H, part = std::min(n, MEAN_PIXELS);
     const float inv = b->frames ? 1.0f / ((float)b->frames * (float)q.spp) : 0.0f;
-    for (size_t i = 0; i < 4 * n; i++) rgba_mean[i] *= inv;
-    return PK_OK;
+    touch_pages(rgba_mean, n * 16);
+    if (b->mean.n < part) {
+      try {
+        b->mean.alloc(part);
+      } catch (CudaError&) {  // no memory for it: scaled on the host
+        cudaGetLastError();
+        check(cudaMemcpyAsync(rgba_mean, b->accum.p + q.out_offset, n * 16, cudaMemcpyDeviceToHost, b->stream), "D2H");
+        check(cudaStreamSynchronize(b->stream), "sync");
+        for (size_t i = 0; i < 4 * n; i++) rgba_mean[i] *= inv;
+        return (int)PK_OK;
+      }
+    }
+    for (size_t i = 0; i < n; i += part) {
+      const uint32_t m = (uint32_t)std::min(part, n - i);
+      k_batch_mean<<<(m + 255) / 256, 256, 0, b->stream>>>(b->accum.p + q.out_offset + i, b->mean.p, m, inv);
+      check(cudaGetLastError(), "k_batch_mean");
+      check(cudaMemcpyAsync(rgba_mean + 4 * i, b->mean.p, (size_t)m * 16, cudaMemcpyDeviceToHost, b->stream), "D2H");
+    }
+    check(cudaStreamSynchronize(b->stream), "sync");
+    return (int)PK_OK;
   });
 }
 

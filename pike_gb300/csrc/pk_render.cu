@@ -1103,8 +1103,9 @@ __device__ __noinline__ void batch_camera(const CamState& cam, uint32_t px, uint
 
 // 40 resident warps per SM (48 registers, some spilled): the loop stalls
 // mostly on instruction fetch and memory latency, and more warps hide both
-// (64-request batch with the current shading code: 481 ms at 32 warps, 425 at
-// 40, 434 at 48, 489 at 64).
+// (64-request batch: 481 ms at 32 warps, 425 at 40, 434 at 48, 489 at 64;
+// 16 requests with packed slab tests and decodes: 22.06 ms at 32, 22.6 at 36,
+// 22.05 at 40, 24.5 at 44).
 // A lane traces a path's closest-hit ray and then, when shading emitted one,
 // its shadow ray within the same step.  (Carrying the shadow ray to the next
 // step, so that every lane runs one traversal per step, measured slower:

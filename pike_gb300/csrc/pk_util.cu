@@ -2,6 +2,7 @@
 // a stable LSD radix sort of 64-bit keys and the level lists of a binary tree,
 // used by the BVH and env builders.
 #include <cuda_runtime.h>
+#include <unistd.h>
 
 #include <algorithm>
 #include <string>
@@ -12,6 +13,13 @@
 #include "pk_util.h"
 
 namespace pk {
+
+void touch_pages(void* p, size_t bytes) {
+  static const size_t page = (size_t)std::max(4096l, sysconf(_SC_PAGESIZE));
+  volatile char* b = static_cast<volatile char*>(p);
+  for (size_t i = 0; i < bytes; i += page) b[i] = b[i];
+  if (bytes) b[bytes - 1] = b[bytes - 1];
+}
 
 cudaMemPool_t create_scratch_pool(int device) {
   cudaMemPoolProps props = {};
