@@ -306,9 +306,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_DYN_MINBLOCKS) k_trace_dyn(S
         lok = lh < MAX_T && lh <= lim;
         rok = rh < MAX_T && rh <= lim;
       } else {
-        inner_children<NODES == NODES_32>(sc, cur, ox, oy, oz, ix, iy, iz, lh, rh, cl, cr);
-        lok = lh < best_t;
-        rok = rh < best_t;
+        inner_children<NODES == NODES_32>(sc, cur, ox, oy, oz, ix, iy, iz, best_t, lok, rok, lh, rh, cl, cr);
       }
       if (lok && rok) {
         int nearc, farc;
@@ -474,7 +472,7 @@ __global__ void __launch_bounds__(TRACE_THREADS, PK_CW_MINBLOCKS) k_trace_cw(Sce
       if (COUNT) nhit += 1;
     } else if (FUSED) {
       const float4 tpv = __ldcs(R.t + j), d = __ldcs(R.d + j);
-      const V3 e = env_color(env, theta, v3(d.x, d.y, d.z));
+      const V3 e = env_color_call(env, theta, v3(d.x, d.y, d.z));
       fused_miss<ANY>(color, npix, hrec, j, __float_as_uint(tpv.w) & 0x0fffffffu, e.x * tpv.x, e.y * tpv.y,
                       e.z * tpv.z, defer, &ctr->err);
     }

@@ -89,6 +89,18 @@ __device__ __forceinline__ V3 env_color(const EnvDev& env, float theta, V3 dir) 
   const float p = pow_(2.0f, a * 255.0f - 128.0f);
   return v3(r * p, g * p, b * p);
 }
+// env_color as a call, for loops whose code has to stay small (the wide
+// traversal: 7.51 -> 7.38 ms for four 1280x720 soup frames; the binary one: none).
+static __device__ __noinline__ V3 env_color_at(const uchar4* rgbe, int w, int h, float theta, V3 dir) {
+  EnvDev e{};
+  e.rgbe = rgbe;
+  e.w = w;
+  e.h = h;
+  return env_color(e, theta, dir);
+}
+__device__ __forceinline__ V3 env_color_call(const EnvDev& env, float theta, V3 dir) {
+  return env_color_at(env.rgbe, env.w, env.h, theta, dir);
+}
 // =====================================================================
 // shade_hit.wgsl:153-483
 // =====================================================================
