@@ -28,7 +28,8 @@
 // launch; the old build ran every one of its 26 levels over all triangles in
 // memory.  A node's BFS index and a leaf's first triangle then follow from
 // per-level counts of the subtrees, summed from left to right (k_columns).
-//   1,310,730 triangles: 33.6 ms -> see the table in k_subtree's comment.
+//   1,310,730 triangles, whole build: 41.1 ms level by level, 8.0 in two phases,
+// 7.5 with the subtrees' scans in one copy (k_subtree).
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -842,10 +843,16 @@ __global__ void __launch_bounds__(NEXT_THREADS) k_lv_next(Level L, int b, uint32
 // triangles in shared memory, level by level over all nodes of the level at
 // once: segmented scans of the rounded boxes along the three lists, binary32
 // costs, the near ones again in double, a stable partition.
-// Bound by instruction issue and barrier latency; SUB = 512 with 128 threads
-// (4 positions each) keeps 4 blocks (45 KB) on an SM.
+// Bound by barrier and instruction-fetch latency (29% of issue slots with the six
+// scans of a level inlined one after the other, so the three lists share one copy
+// of their two scans and keep their costs in shared memory); 256 threads of two
+// positions each, 4 blocks (51 KB, 64 registers) on an SM.  Whole build of
+// 1,310,730 triangles: six scans inlined, 128 threads 8.02 ms; one copy, 128
+// threads 7.77 (96 registers: 4 blocks), 256 threads 7.53 (3 blocks 7.70), 512
+// threads of one position 8.45.
 // =====================================================================
-constexpr int ST_THREADS = 128;
+constexpr int ST_THREADS = 256;
+constexpr int ST_BLOCKS = 4;
 constexpr int ST_PER = (int)SUB / ST_THREADS;
 constexpr int ST_WARPS = ST_THREADS / 32;
 constexpr uint16_t NO_NODE = 0xffff;
@@ -888,18 +895,21 @@ struct StShared {
   uint32_t pre[SUB];     // left triangles before a position: 10 bits per list
   uint32_t near_[3][SUB / 32];
   uint8_t left[SUB];
-  FBox wbox[6][ST_WARPS];
-  uint32_t wflag[6][ST_WARPS];
+  float cost[3][SUB];
+  FBox wbox[2][ST_WARPS];
+  uint32_t wflag[2][ST_WARPS];
   uint32_t warp[ST_WARPS + 1][2];
   KBox kwarp[ST_WARPS];
   uint32_t lvbase[SUB + 1];
   uint32_t n_todo;
 };
 
-// Segmented running areas along one list; SLOT: the shared words of this scan.
-template <bool REV, int SLOT>
+// Segmented running areas along one list, forwards or backwards (each direction
+// has its shared words); emit(j, box, area) for the running box at position j.
+template <bool REV, class Emit>
 __device__ __forceinline__ void seg_areas(StShared& S, const uint16_t* lst, const uint16_t (&sg)[ST_PER],
-                                          uint32_t edge, float (&area)[ST_PER], FBox (*full)) {
+                                          uint32_t edge, float (&area)[ST_PER], Emit emit) {
+  constexpr int SLOT = REV ? 1 : 0;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   FBox bx[ST_PER];
   FBox inc = fbox_empty();
@@ -947,7 +957,7 @@ __device__ __forceinline__ void seg_areas(StShared& S, const uint16_t* lst, cons
     if ((edge >> j) & 1u) run = bx[j];
     else fbox_add(run, bx[j]);
     area[j] = fbox_sa(run);
-    if (full) full[j] = run;
+    emit(j, run, area[j]);
   }
 }
 
@@ -971,7 +981,7 @@ __device__ __forceinline__ double exact_cost(const StShared& S, const KBox* kbox
   return sweep_cost(kbox_sa(f), kbox_sa(g), psa, i, n);
 }
 
-__global__ void __launch_bounds__(ST_THREADS) k_subtree(Subtrees W) {
+__global__ void __launch_bounds__(ST_THREADS, ST_BLOCKS) k_subtree(Subtrees W) {
   extern __shared__ __align__(16) unsigned char st_raw[];
   StShared& S = *reinterpret_cast<StShared*>(st_raw);
   const SmallTask task = W.task[blockIdx.x];
@@ -1037,22 +1047,30 @@ __global__ void __launch_bounds__(ST_THREADS) k_subtree(Subtrees W) {
         if (p == st[j] + cn[j] - 1) tail |= 1u << j;
       }
     }
-    float f[3][ST_PER], g[3][ST_PER];
-    {
-      FBox full[ST_PER];
-      seg_areas<false, 0>(S, S.lst[b][0], sg, head, f[0], full);
+    // one copy of the scans for the three lists
+    uint32_t c3[ST_PER];
 #pragma unroll
-      for (int j = 0; j < ST_PER; j++)
-        if (sg[j] != NO_NODE && ((tail >> j) & 1u)) {  // the node's box
-          S.bound[sg[j]] = cost_bound(full[j], cn[j], fr.ok);
-          S.inv[sg[j]] = 1.0f / f[0][j];
+    for (int j = 0; j < ST_PER; j++) c3[j] = 0xffffffffu;
+#pragma unroll 1
+    for (int a = 0; a < 3; a++) {
+      const uint16_t* lst = S.lst[b][a];
+      float f[ST_PER], g[ST_PER];
+      seg_areas<false>(S, lst, sg, head, f, [&](int j, const FBox& run, float area) {
+        if (a == 0 && sg[j] != NO_NODE && ((tail >> j) & 1u)) {  // the node's box
+          S.bound[sg[j]] = cost_bound(run, cn[j], fr.ok);
+          S.inv[sg[j]] = 1.0f / area;
         }
+      });
+      seg_areas<true>(S, lst, sg, tail, g, [](int, const FBox&, float) {});
+#pragma unroll
+      for (int j = 0; j < ST_PER; j++) {
+        if (sg[j] == NO_NODE) continue;
+        const uint32_t i = tid * ST_PER + j - st[j];
+        const float cost = 0.5f + (f[j] * (float)(i + 1) + g[j] * (float)(cn[j] - 1 - i)) * S.inv[sg[j]];
+        S.cost[a][tid * ST_PER + j] = cost;
+        c3[j] = min(c3[j], __float_as_uint(cost));
+      }
     }
-    seg_areas<true, 1>(S, S.lst[b][0], sg, tail, g[0], nullptr);
-    seg_areas<false, 2>(S, S.lst[b][1], sg, head, f[1], nullptr);
-    seg_areas<true, 3>(S, S.lst[b][1], sg, tail, g[1], nullptr);
-    seg_areas<false, 4>(S, S.lst[b][2], sg, head, f[2], nullptr);
-    seg_areas<true, 5>(S, S.lst[b][2], sg, tail, g[2], nullptr);
     // a warp inside one node (its range is contiguous) combines its costs before the shared atomic
     const int s_first = sg[0], s_last = sg[ST_PER - 1], s_lane0 = __shfl_sync(0xffffffffu, s_first, 0);
     const bool one = __all_sync(0xffffffffu, s_first != NO_NODE && s_first == s_last && s_first == s_lane0);
@@ -1060,16 +1078,8 @@ __global__ void __launch_bounds__(ST_THREADS) k_subtree(Subtrees W) {
 #pragma unroll
     for (int j = 0; j < ST_PER; j++) {
       if (sg[j] == NO_NODE) continue;
-      const uint32_t i = tid * ST_PER + j - st[j];
-      const float inv = S.inv[sg[j]];
-      uint32_t c3 = 0xffffffffu;
-#pragma unroll
-      for (int a = 0; a < 3; a++) {
-        f[a][j] = 0.5f + (f[a][j] * (float)(i + 1) + g[a][j] * (float)(cn[j] - 1 - i)) * inv;
-        c3 = min(c3, __float_as_uint(f[a][j]));
-      }
-      if (one) low = min(low, c3);
-      else atomicMin(&S.nmin[sg[j]], c3);
+      if (one) low = min(low, c3[j]);
+      else atomicMin(&S.nmin[sg[j]], c3[j]);
     }
     if (one) {
       low = __reduce_min_sync(0xffffffffu, low);
@@ -1084,7 +1094,7 @@ __global__ void __launch_bounds__(ST_THREADS) k_subtree(Subtrees W) {
       const float limit = __uint_as_float(S.nmin[sg[j]]) + 2.0f * S.bound[sg[j]];
 #pragma unroll
       for (int a = 0; a < 3; a++)
-        if (!(f[a][j] > limit)) {
+        if (!(S.cost[a][p] > limit)) {
           atomicOr(&S.near_[a][p >> 5], 1u << (p & 31u));
           atomicMin(&S.first[sg[j]], a * cn[j] + (p - st[j]));
         }
