@@ -800,10 +800,14 @@ __device__ __forceinline__ bool shade_one(const SceneDev& sc, const EnvDev& env,
 
 // Resident blocks per SM (at 128 threads, warp-wide look-back, 1080p: 10
 // blocks 3342-3359 Mrays/s, 12: 3394-3396, 14: 3392-3407, 16: 3384-3392).
-#ifndef PK_SHADE_BLOCKS
-#define PK_SHADE_BLOCKS (1536 / SHADE_THREADS)
-#endif
-__global__ void __launch_bounds__(SHADE_THREADS, PK_SHADE_BLOCKS) k_shade(SceneDev sc, EnvDev env, Counters* __restrict__ ctr,
+// Queues of fewer than SHADE_MANY rays: 2 blocks of 512 threads (64 registers, few
+// spills) instead of 3 (40): there are not enough tiles for the third to cover
+// latency (256x256 frames 399 -> 387 us, 853x479 1037 -> 1020; the other way round
+// at 1280x720, 7.37 -> 7.48 ms, and 1080p, 23.7 -> 24.6).
+constexpr int SHADE_BLOCKS = 1536 / SHADE_THREADS, SHADE_BLOCKS_FEW = 1024 / SHADE_THREADS;
+constexpr uint32_t SHADE_MANY = 1u << 19;
+template <int BLOCKS>
+__global__ void __launch_bounds__(SHADE_THREADS, BLOCKS) k_shade(SceneDev sc, EnvDev env, Counters* __restrict__ ctr,
                                                           const uint32_t* __restrict__ hit_list,
                                                           const uint4* __restrict__ hrec, RayQ Rin, RayQ Rout,
                                                           RayQ S, uint32_t capacity, float4* __restrict__ color,
@@ -1282,7 +1286,8 @@ Grids kernel_grids(int sms, uint32_t capacity) {
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&t, k_trace_dyn<false, true, false, NODES_64>, TRACE_THREADS, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&w, k_trace_cw<false, true, false>, TRACE_THREADS, 0);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&c, k_compact<0, true, COMPACT_R_LARGE>, COMPACT_THREADS, 0);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&s, k_shade, SHADE_THREADS, 0);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(
+      &s, capacity >= SHADE_MANY ? k_shade<SHADE_BLOCKS> : k_shade<SHADE_BLOCKS_FEW>, SHADE_THREADS, 0);
   const unsigned n = (unsigned)sms;
   const unsigned rays = std::max(1u, ((capacity + 31u) / 32u + TRACE_THREADS / 32 - 1) / (TRACE_THREADS / 32));
   const unsigned spread = (capacity + TRACE_SPREAD * (TRACE_THREADS / 32) - 1) / (TRACE_SPREAD * (TRACE_THREADS / 32));
@@ -1386,8 +1391,11 @@ void launch_compact_shadow(const LaunchCtx& L, uint32_t* flags, RayQ S, RayQ M, 
 
 void launch_shade(const LaunchCtx& L, const uint32_t* hit_list, const uint4* hrec, RayQ Rin, RayQ Rout, RayQ S,
                   uint32_t* ticket, unsigned long long* tiles) {
-  k_shade<<<L.grids.shade.at(L.shade_tenths), SHADE_THREADS, 0, L.stream>>>(L.scene, L.env, L.ctr, hit_list, hrec, Rin, Rout, S,
-                                                                          L.capacity, L.color, L.npix, ticket, tiles);
+#define PK_SHADE(B)                                                                                             \
+  k_shade<B><<<L.grids.shade.at(L.shade_tenths), SHADE_THREADS, 0, L.stream>>>(                                  \
+      L.scene, L.env, L.ctr, hit_list, hrec, Rin, Rout, S, L.capacity, L.color, L.npix, ticket, tiles)
+  if (L.capacity >= SHADE_MANY) PK_SHADE(SHADE_BLOCKS); else PK_SHADE(SHADE_BLOCKS_FEW);
+#undef PK_SHADE
 }
 
 void launch_shade_miss(const LaunchCtx& L, RayQ M) {

@@ -9,7 +9,7 @@ import pytest
 from pike_gb300 import _lib, synth
 from pike_gb300._lib import Context, ptr
 
-from helpers import Pair, assert_bits_equal
+from helpers import Pair, assert_bits_equal, assert_bits_equal_nan, camera_struct
 
 pytestmark = pytest.mark.gpu
 
@@ -188,3 +188,91 @@ def test_paths_in_chunks(pk_built):
     for name, a, b0, b1 in zip(("albedo", "rough", "env"), g, *h):
         b = b0 + b1
         assert (a - b).abs().max() <= 1e-4 * b.abs().max(), name
+
+
+@pytest.mark.parametrize("change", [
+    dict(), dict(apertureSize=0.05), dict(bokeh=-1.0), dict(bokeh=0.0), dict(focalDepth=float("inf")),
+    dict(pos=[-0.0, 1.5, 4.0]), dict(pos=[0.0, -0.0, 4.0], apertureSize=0.0), dict(dir=[0.0, 1.0, 0.0]),
+    dict(fov=3.0, distortion=0.4)], ids=str)
+def test_camera_rays_with_and_without_a_lens(oracle, pk_built, change):
+    """A zero aperture leaves the lens out where that changes no bit, and only there."""
+    src = synth.small_scene(width=33, height=17)
+    pair = Pair(src, oracle)
+    pair.set_camera(dict(src.camera_state(), **change))
+    pair.set_render_state(3)
+    P = pair.P.r
+    for name in ("clear_color", "clear_hits_misses", "clear_rays"):
+        pair.ctx.call("pk_" + name)
+    P.begin_frame()
+    pair.ctx.call("pk_camera")
+    P.camera()
+    n = P.counters()["num_rays"]
+    assert_bits_equal_nan(pair.rays(_lib.PK_QUEUE_RAYS, 0, n), P.rays(0, n), "camera rays")
+
+
+@pytest.mark.parametrize("theta", [0.0, -0.5, -3.9, 2.7, 1.0e4, 3.0e6])
+def test_environment_lookup_wraps(oracle, pk_built, theta):
+    """Repeat addressing of the rotated map: inside it, some turns away on both
+    sides, and beyond 2^22 texels, where the integer remainder takes over."""
+    src = synth.displaced_sphere_scene(subdivisions=3, width=64, height=40, env_size=(67, 31))
+    pair = Pair(src, oracle)
+    pair.set_render_state(0, theta)
+    P = pair.P.r
+    for name in ("clear_color", "clear_hits_misses", "clear_rays"):
+        pair.ctx.call("pk_" + name)
+    P.begin_frame()
+    for name in ("camera", "trace", "shade_hit", "trace_shadow", "shade_miss", "accumulate"):
+        pair.ctx.call("pk_" + name)
+        getattr(P, name)()
+    want = P.accum()
+    assert_bits_equal(pair.image("accum"), want, "pass by pass")
+    pair.ctx.call("pk_set_render_state", 0, theta)
+    pair.ctx.call("pk_render_frame", 1)
+    pair.ctx.call("pk_sync")
+    assert_bits_equal(pair.image("accum"), want, "fused")
+
+
+@pytest.mark.parametrize("capacity", [(1 << 19) - 128, 1 << 19, 1 << 20])
+def test_queue_capacity_changes_no_bit(oracle, pk_built, capacity):
+    """The same 2046 rays in queues on both sides of the lines where shading and compaction change form."""
+    src = synth.small_scene(width=66, height=31)
+    pair = Pair(src, oracle)
+    pair.set_render_state(0)
+    pair.P.r.tick(4)
+    want = pair.P.r.accum()
+    pair.ctx.call("pk_configure", src.width, src.height, capacity)
+    pair.ctx.call("pk_set_camera", C.byref(camera_struct(src.camera_state())))
+    pair.ctx.call("pk_set_render_state", 0, 0.0)
+    pair.ctx.call("pk_render_frame", 4)
+    pair.ctx.call("pk_sync")
+    assert_bits_equal(pair.image("accum"), want, "fused")
+
+
+def test_batch_readback_in_parts(pk_built):
+    """A request of more than the 2^20 pixels that are read back at a time: the
+    pixels whose camera ray misses have the drop-in's bits (shading seeds differ)."""
+    from pike_gb300.batch import Batch, Request, scene_context
+    w, h = 1100, 1000
+    src = synth.small_scene(width=w, height=h)
+    ctx, cam = scene_context(src), dict(src.camera_state(), dir=[0.0, 0.4, 0.9165151])  # up: sky below as well
+    batch = Batch([ctx])
+    batch.set_requests([Request(scene=0, width=w, height=h, spp=1, depth=1, camera=cam)])
+    batch.render(1)
+    got = batch.image(0)
+    ctx.call("pk_configure", w, h, w * h)
+    ctx.call("pk_set_camera", C.byref(camera_struct(cam)))
+    ctx.call("pk_set_render_state", 0, 0.0)
+    want = np.zeros((h, w, 4), np.float32)
+    for name in ("clear_color", "clear_hits_misses", "clear_rays", "camera", "trace"):
+        ctx.call("pk_" + name)
+    n = np.zeros(8, np.uint32)
+    ctx.call("pk_read_counters", ptr(n))
+    hits = np.zeros((int(n[1]), 16), np.uint32)
+    ctx.call("pk_read_hits", 0, hits.shape[0], ptr(hits))
+    ctx.call("pk_set_render_state", 0, 0.0)
+    ctx.call("pk_render_frame", 1)
+    ctx.call("pk_read_accum", ptr(want))
+    miss = np.ones(w * h, bool)
+    miss[hits[:, 15] & 0x0FFFFFFF] = False
+    assert miss[: 1 << 20].any() and miss[1 << 20:].any()
+    assert np.array_equal(got.reshape(-1, 4)[miss, :3].view(np.uint32), want.reshape(-1, 4)[miss, :3].view(np.uint32))
