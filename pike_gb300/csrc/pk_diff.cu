@@ -34,8 +34,8 @@
 // smooth function of theta (paths do not move), so its exact derivative is
 // what central differences with common random numbers measure.
 //
-// Adjoint.  k_diff_adjoint replays every path from its seed (nothing is
-// stored between the passes) and records per vertex the throughput T that
+// Adjoint.  The backward pass replays every path from its seed (nothing is
+// stored between the passes; k_path_*<true>) and records per vertex the throughput T that
 // reaches it, the factor P to the next vertex's throughput, the contribution
 // factor Q of the vertex (next-event estimate, emission, or the environment
 // when the ray leaves) and their derivatives; a backward sweep with

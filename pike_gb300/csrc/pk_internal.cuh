@@ -112,45 +112,15 @@ __device__ __forceinline__ unsigned long long pack2(uint32_t a, uint32_t b) {
 __device__ __forceinline__ uint32_t unpack_a(unsigned long long v) { return (uint32_t)(v & 0x7fffffffull); }
 __device__ __forceinline__ uint32_t unpack_b(unsigned long long v) { return (uint32_t)((v >> 31) & 0x7fffffffull); }
 
-// Exclusive prefix of this tile's two counts over all earlier tiles.  Called by
-// one thread.  Tiles are numbered in the order blocks claim them (an atomic
-// ticket), so every earlier tile belongs to a block that is already running;
-// waits are bounded and report ERR_LOOKBACK instead of hanging.
-__device__ __forceinline__ unsigned long long lookback2(unsigned long long* tiles, uint32_t tile,
-                                                        unsigned long long agg, uint32_t* err) {
-  if (tile == 0) {
-    st_release(&tiles[0], TILE_PRE | agg);
-    return 0ull;
-  }
-  st_release(&tiles[tile], TILE_AGG | agg);
-  unsigned long long excl = 0;
-  int i = (int)tile - 1;
-  while (i >= 0) {
-    unsigned long long v = ld_acquire(&tiles[i]);
-    int spins = 0;
-    while ((v & ~TILE_VAL) == 0) {
-      if (++spins > LOOKBACK_SPIN_LIMIT) {
-        atomicOr(err, ERR_LOOKBACK);
-        v = TILE_PRE;
-        break;
-      }
-      __nanosleep(64);
-      v = ld_acquire(&tiles[i]);
-    }
-    excl += v & TILE_VAL;
-    if ((v & ~TILE_VAL) == TILE_PRE) break;
-    --i;
-  }
-  st_release(&tiles[tile], TILE_PRE | (excl + agg));
-  return excl;
-}
-
-// The same prefix computed by one whole warp (every lane calls it; all get
-// the result): each round reads a window of 32 earlier tiles at once, waits
-// (bounded) until each has published, and sums the aggregates from the tile
-// before this one back to the nearest tile holding an inclusive prefix, which
-// ends the walk.  A walk over n unfinished predecessors takes n / 32 rounds
-// of memory latency instead of n.
+// Exclusive prefix of this tile's two counts over all earlier tiles, by one
+// whole warp (every lane calls it; all get the result).  Tiles are numbered in
+// the order blocks claim them (an atomic ticket), so every earlier tile belongs
+// to a block that is already running; waits are bounded and report ERR_LOOKBACK
+// instead of hanging.  Each round reads a window of 32 earlier tiles at once,
+// waits until each has published, and sums the aggregates from the tile before
+// this one back to the nearest tile holding an inclusive prefix, which ends the
+// walk.  A walk over n unfinished predecessors takes n / 32 rounds of memory
+// latency instead of n.
 __device__ __forceinline__ unsigned long long lookback2_warp(unsigned long long* tiles, uint32_t tile,
                                                              unsigned long long agg, uint32_t* err) {
   const int lane = (int)(threadIdx.x & 31u);

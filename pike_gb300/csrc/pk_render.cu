@@ -186,7 +186,7 @@ constexpr int INNER_BUDGET = PK_INNER_BUDGET;
 // formats had kernels of their own.)
 constexpr int ANY_BUDGET = PK_ANY_BUDGET;
 
-// Box test of the exact binary records: like box_hit, with the far distance
+// Box test of the exact binary records: the drop-in's, with the far distance
 // widened by WIDE_SLACK (relative) so that rounding never drops a box.
 __device__ __forceinline__ float box_hit_exact(float xa, float xb, float ya, float yb, float za, float zb, float ox,
                                                float oy, float oz, float ix, float iy, float iz) {
