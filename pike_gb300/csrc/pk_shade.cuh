@@ -73,7 +73,7 @@ __device__ __forceinline__ void camera_ray(const CamState& cam, const CamBasis& 
 // by at most one) and an exact remainder in floats are nine.
 __device__ __forceinline__ int wrap_floor(float f, int n) {
   const float g = floorf(f), fn = (float)n;
-  if (fabsf(g) < 4194304.0f && n < 4194304) {
+  if (fabsf(g) < 1048576.0f && n < 1048576) {
     const float r = __fmaf_rn(-floorf(g * __fdividef(1.0f, fn)), fn, g);
     return (int)(r < 0.0f ? r + fn : (r >= fn ? r - fn : r));
   }

@@ -15,6 +15,12 @@
 namespace pk {
 
 void touch_pages(void* p, size_t bytes) {
+  cudaPointerAttributes a;
+  if (cudaPointerGetAttributes(&a, p) != cudaSuccess) {
+    cudaGetLastError();
+    return;
+  }
+  if (a.type != cudaMemoryTypeUnregistered) return;  // pinned, or not the host's to touch
   static const size_t page = (size_t)std::max(4096l, sysconf(_SC_PAGESIZE));
   volatile char* b = static_cast<volatile char*>(p);
   for (size_t i = 0; i < bytes; i += page) b[i] = b[i];

@@ -22,7 +22,7 @@ inline void check(cudaError_t e, const char* what) {
 // has when the new size fits it and fills at least half of it: a scene that is
 // rebuilt at about its old size then costs no cudaMalloc and no cudaFree (which
 // waits for the whole device).
-// Makes the pages of a caller's buffer resident, its contents kept, before the GPU
+// Makes the pages of a caller's pageable buffer resident, its contents kept, before the GPU
 // copies into it: where the GPU reaches pageable memory through the host's page
 // tables, the copy engine faulted fresh pages in one by one (49 MB in 16 buffers:
 // 30-52 ms, touched by this thread first 17 ms, by eight threads 20 ms).

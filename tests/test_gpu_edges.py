@@ -213,7 +213,7 @@ def test_camera_rays_with_and_without_a_lens(oracle, pk_built, change):
 @pytest.mark.parametrize("theta", [0.0, -0.5, -3.9, 2.7, 1.0e4, 3.0e6])
 def test_environment_lookup_wraps(oracle, pk_built, theta):
     """Repeat addressing of the rotated map: inside it, some turns away on both
-    sides, and beyond 2^22 texels, where the integer remainder takes over."""
+    sides, and beyond 2^20 texels, where the integer remainder takes over."""
     src = synth.displaced_sphere_scene(subdivisions=3, width=64, height=40, env_size=(67, 31))
     pair = Pair(src, oracle)
     pair.set_render_state(0, theta)
