@@ -186,8 +186,9 @@ void scan_exclusive_f64(const Scratch& w, const double* in, double* out, size_t 
 // (blockIdx.y).
 constexpr int SORT_THREADS = 256;
 constexpr int SORT_WARPS = SORT_THREADS / 32;
-constexpr int SORT_ROUNDS = 12;                       // rounds of 32 keys per warp
-constexpr int SORT_TILE = SORT_THREADS * SORT_ROUNDS; // 3072 keys per block: 36 KB of pairs in shared memory
+// rounds of 32 keys per warp (2048x1024 map's tables: 6 929 us, 8 915, 10 925, 12 948)
+constexpr int SORT_ROUNDS = 8;
+constexpr int SORT_TILE = SORT_THREADS * SORT_ROUNDS;  // 2048 keys per block: 24 KB of pairs in shared memory
 constexpr int RADIX = 256;
 constexpr int SORT_PASSES = 8;
 constexpr uint32_t SORT_BACK = 4;  // tiles a look-back reads at once (2048x1024 map: 1 958 us, 4 948, 8 953, 16 965)

@@ -86,10 +86,11 @@ def test_sweep_build_refuses_a_point(ctx):
     ctx.call("pk_bvh_build", _lib.PK_BVH_SWEEP)
 
 
-@pytest.mark.parametrize("w,h,kind", [(2, 1, "log"), (3071, 1, "log"), (3072, 1, "log"), (1, 3073, "log"),
+@pytest.mark.parametrize("w,h,kind", [(2, 1, "log"), (2047, 1, "log"), (2048, 1, "log"), (1, 2049, "log"),
+                                      (128, 96, "log"), (3071, 1, "log"), (3072, 1, "log"), (1, 3073, "log"),
                                       (97, 64, "log"), (64, 64, "two"), (128, 64, "steep"), (96, 64, "constant")])
 def test_env_tables_at_sort_tiles_and_bin_edges(ctx, oracle, w, h, kind):
-    """Tiles of 3072 keys; maps whose bin edges fall on ties (decided by the sequential walk)."""
+    """Tiles of 2048 keys, 1 to 6 of them (a look-back reads 4); maps whose bin edges fall on ties (decided by the sequential walk)."""
     rng = np.random.default_rng(w * h)
     lum = {"log": lambda: np.exp(1.5 * rng.standard_normal((h, w))), "two": lambda: rng.integers(1, 3, (h, w)) * 1.0,
            "steep": lambda: 2.0 ** -rng.uniform(0, 60, (h, w)), "constant": lambda: np.ones((h, w))}[kind]()
