@@ -65,9 +65,11 @@ __device__ __forceinline__ void fused_miss(float4* color, uint32_t npix, uint4* 
 
 // trace.wgsl:191-213 main (closest hit) and trace_shadow.wgsl:192-207 main (any
 // hit).  Warps claim 32 consecutive queue slots at a time; the outcome bit of
-// every slot goes to flags[slot / 32].  FUSED: a ray that reaches the
-// environment adds its shade_miss.wgsl contribution directly (the miss queue
-// is not materialised); otherwise the compaction kernel builds the miss queue.
+// every slot goes to flags[slot / 32], for the compaction that reads and clears
+// it (a fused any-hit traversal has none after it and writes no flags).  FUSED: a
+// ray that reaches the environment adds its shade_miss.wgsl contribution directly
+// (the miss queue is not materialised); otherwise the compaction kernel builds
+// the miss queue.
 template <bool ANY, bool FUSED, bool COUNT, bool COMPACT>
 __global__ void __launch_bounds__(TRACE_THREADS) k_trace(SceneDev sc, EnvDev env, Counters* __restrict__ ctr,
                                                           const uint32_t* __restrict__ countp, RayQ R,
@@ -107,7 +109,7 @@ __global__ void __launch_bounds__(TRACE_THREADS) k_trace(SceneDev sc, EnvDev env
       }
     }
     const uint32_t m = __ballot_sync(0xffffffffu, hit);
-    if (lane == 0) flags[base >> 5] = m;
+    if (!(ANY && FUSED) && lane == 0) flags[base >> 5] = m;
     if (COUNT && lane == 0) nhit += (uint32_t)__popc(m);
   }
   if (COUNT) {
