@@ -138,6 +138,8 @@ void require_config(pk_ctx* c) {
 void require_render(pk_ctx* c) {
   require_config(c);
   if (!c->bvh_ready) throw std::runtime_error("no BVH: call pk_bvh_build or pk_bvh_upload");
+  if (((c->trace_mode & TRACE_WIDE) && !c->wide_ready) || ((c->trace_mode & TRACE_EXACT) && !c->exact_ready))
+    throw std::runtime_error("this BVH has no records for the trace mode: its build failed");
   if (!c->n_mats || !c->n_layers) throw std::runtime_error("no materials: call pk_materials_set/upload");
   if (!c->attrs.p) throw std::runtime_error("no scene attributes: call pk_scene_flatten/upload");
   if (c->bvh_verts > c->n_verts) throw std::runtime_error("BVH vertices exceed the scene's vertex attributes");
@@ -224,6 +226,28 @@ int pk_destroy(pk_ctx* c) {
 
 const char* pk_last_error(const pk_ctx* c) { return c ? c->err.c_str() : "null context"; }
 
+// The buffers of a configuration whose sizes are set.
+static void configure_buffers(pk_ctx* c) {
+  if (c->kahan) {
+    c->accum_sum.alloc(c->npix);
+    c->accum_comp.alloc(c->npix);
+  }
+  c->ct = compact_tiles(c->cap);
+  c->st = shade_tiles(c->cap);
+  c->grids = kernel_grids(c->sms, c->cap);
+  for (int i = 0; i < 3; i++) c->mq[i].alloc(2 * (size_t)c->cap);
+  alloc_slot(c, 0);
+  for (int k = 1; k < MAX_IN_FLIGHT; k++) release_slot(c->slot[k]);  // sized again on first use
+  c->next_slot = c->last_slot = 0;
+  c->accum.alloc(c->npix);
+  c->display.alloc(c->npix);
+  c->display8.alloc(c->npix);
+  check(cudaMemsetAsync(c->accum.p, 0, c->accum.bytes(), c->stream), "memset");
+  check(cudaMemsetAsync(c->display.p, 0, c->display.bytes(), c->stream), "memset");
+  check(cudaMemsetAsync(c->display8.p, 0, c->display8.bytes(), c->stream), "memset");
+  check(cudaStreamSynchronize(c->stream), "sync");
+}
+
 int pk_configure(pk_ctx* c, uint32_t width, uint32_t height, uint32_t batch) {
   return guarded(c, [&]() {
     c->invalidate_graph();
@@ -233,30 +257,29 @@ int pk_configure(pk_ctx* c, uint32_t width, uint32_t height, uint32_t batch) {
     c->W = width; c->H = height; c->B = batch;
     c->cap = (batch + 127u) / 128u * 128u;
     c->npix = width * height;
-    if (c->kahan) {
-      c->accum_sum.alloc(c->npix);
-      c->accum_comp.alloc(c->npix);
+    try {
+      configure_buffers(c);
+    } catch (...) {
+      c->cap = 0;  // not configured: some buffers still have their old sizes
+      throw;
     }
-    c->ct = compact_tiles(c->cap);
-    c->st = shade_tiles(c->cap);
-    c->grids = kernel_grids(c->sms, c->cap);
-    for (int i = 0; i < 3; i++) c->mq[i].alloc(2 * (size_t)c->cap);
-    alloc_slot(c, 0);
-    for (int k = 1; k < MAX_IN_FLIGHT; k++) release_slot(c->slot[k]);  // sized again on first use
-    c->next_slot = c->last_slot = 0;
-    c->accum.alloc(c->npix);
-    c->display.alloc(c->npix);
-    c->display8.alloc(c->npix);
-    check(cudaMemsetAsync(c->accum.p, 0, c->accum.bytes(), c->stream), "memset");
-    check(cudaMemsetAsync(c->display.p, 0, c->display.bytes(), c->stream), "memset");
-    check(cudaMemsetAsync(c->display8.p, 0, c->display8.bytes(), c->stream), "memset");
-    check(cudaStreamSynchronize(c->stream), "sync");
     return PK_OK;
   });
 }
 
 // ---------------- scene ----------------
 namespace {
+// Before buffers are replaced: when one of the copies or allocations fails, no
+// later call and no captured frame may find the old sizes with the new buffers.
+void drop_scene(pk_ctx* c) {
+  c->n_verts = c->n_tris = 0;
+  c->bvh_ready = false;
+  c->invalidate_graph();
+}
+void drop_materials(pk_ctx* c) {
+  c->n_mats = c->n_layers = 0;
+  c->invalidate_graph();
+}
 int flatten_impl(pk_ctx* c, const double* pos3, const double* nrm3, const double* tan4, const double* bn3,
                  const double* bt4, const double* uv2, uint32_t n_verts, const int32_t* tri4, uint32_t n_tris,
                  double scale, const double translate[3]) {
@@ -272,6 +295,7 @@ int flatten_impl(pk_ctx* c, const double* pos3, const double* nrm3, const double
     upload(u, uv2, 2 * (size_t)n_verts, c->stream);
     if (bn3) upload(bn, bn3, 3 * (size_t)n_verts, c->stream);
     if (bt4) upload(bt, bt4, 4 * (size_t)n_verts, c->stream);
+    drop_scene(c);
     c->pos.alloc(3 * (size_t)n_verts);
     c->attrs.alloc(n_verts);
     const double tr[3] = {translate ? translate[0] : 0.0, translate ? translate[1] : 0.0, translate ? translate[2] : 0.0};
@@ -282,8 +306,6 @@ int flatten_impl(pk_ctx* c, const double* pos3, const double* nrm3, const double
     check(cudaStreamSynchronize(c->stream), "sync");
     c->n_verts = n_verts;
     c->n_tris = n_tris;
-    c->bvh_ready = false;
-    c->invalidate_graph();
     return PK_OK;
   });
 }
@@ -308,14 +330,13 @@ int pk_scene_upload(pk_ctx* c, const int32_t* tri4, uint32_t n_tris, const doubl
     for (uint32_t t = 0; t < n_tris; t++)
       for (int k = 0; k < 3; k++)
         if (tri4[4 * t + k] < 0 || (uint32_t)tri4[4 * t + k] >= n_verts) return fail(c, PK_ERR_ARG, "vertex index out of range");
+    drop_scene(c);
     upload(c->tri4, tri4, n_tris, c->stream);
     upload(c->pos, pos3, 3 * (size_t)n_verts, c->stream);
     upload(c->attrs, attr4, n_verts, c->stream);
     check(cudaStreamSynchronize(c->stream), "sync");
     c->n_verts = n_verts;
     c->n_tris = n_tris;
-    c->bvh_ready = false;
-    c->invalidate_graph();
     return PK_OK;
   });
 }
@@ -342,6 +363,7 @@ int pk_materials_set(pk_ctx* c, const double* mats9, uint32_t n_mats) {
     std::vector<int32_t> index4;
     std::vector<uint8_t> layers;
     build_material_layers(mats9, n_mats, index4, layers);
+    drop_materials(c);
     upload(c->mat4, index4.data(), n_mats, c->stream);
     upload(c->layers, layers.data(), layers.size() / 4, c->stream);
     check(cudaStreamSynchronize(c->stream), "sync");
@@ -356,6 +378,7 @@ int pk_materials_set(pk_ctx* c, const double* mats9, uint32_t n_mats) {
 int pk_materials_upload(pk_ctx* c, const int32_t* mat4, uint32_t n_mats, const uint8_t* layers, uint32_t n_layers) {
   return guarded(c, [&]() {
     if (!mat4 || !layers || !n_mats || !n_layers) return fail(c, PK_ERR_ARG, "no materials");
+    drop_materials(c);
     upload(c->mat4, mat4, n_mats, c->stream);
     upload(c->layers, layers, n_layers, c->stream);
     check(cudaStreamSynchronize(c->stream), "sync");
@@ -371,6 +394,8 @@ int pk_atlas_upload(pk_ctx* c, const uint8_t* layers, uint32_t res, uint32_t n_l
   return guarded(c, [&]() {
     if (!layers || !res || !n_layers || res > 16384) return fail(c, PK_ERR_ARG, "bad atlas");
     if ((uint64_t)res * res * n_layers >= (1ull << 32)) return fail(c, PK_ERR_ARG, "atlas too large");
+    c->n_layers = 0;
+    c->invalidate_graph();
     upload(c->layers, layers, (size_t)res * res * n_layers, c->stream);
     check(cudaStreamSynchronize(c->stream), "sync");
     c->n_layers = n_layers;
@@ -421,7 +446,17 @@ static int build_exact(pk_ctx* c) {
   return PK_OK;
 }
 
+// The BVH's arrays are about to be replaced: no call and no captured frame may
+// use them until finish_bvh has accepted the new ones.
+static void drop_bvh(pk_ctx* c) {
+  c->bvh_ready = false;
+  c->invalidate_graph();
+}
+
+// The traversal records of the BVH's new arrays.  A tree that the drop-in's
+// records hold but a set trace mode's do not stays usable in the other modes.
 static int finish_bvh(pk_ctx* c) {
+  drop_bvh(c);
   c->wide_ready = false;
   c->exact_ready = false;
   if (!(c->trace_mode & TRACE_WIDE)) {
@@ -496,6 +531,7 @@ int pk_bvh_upload(pk_ctx* c, const int32_t* nodes5, uint32_t n_nodes, const int3
                   const float* verts4, uint32_t n_verts) {
   return guarded(c, [&]() {
     if (!nodes5 || !n_nodes || !verts4 || !n_verts) return fail(c, PK_ERR_ARG, "empty BVH");
+    drop_bvh(c);
     upload(c->nodes5, nodes5, 5 * (size_t)n_nodes, c->stream);
     c->node_box_d.release();
     upload(c->tri4_leaf, tri4_leaf, n_leaf_tris, c->stream);
@@ -568,8 +604,15 @@ static int env_changed(pk_ctx* c) {
   return c->env_sampling == PK_ENV_ALIAS ? build_alias(c) : PK_OK;
 }
 
+// Before its buffers are replaced (as drop_scene).
+static void drop_env(pk_ctx* c) {
+  c->env_ready = false;
+  c->invalidate_graph();
+}
+
 static int env_set(pk_ctx* c, const uint8_t* rgbe, uint32_t w, uint32_t h, const int32_t* bins2, uint32_t nb,
                    const int32_t* coords2, const float* pdf) {
+  drop_env(c);
   upload(c->rgbe, rgbe, (size_t)w * h, c->stream);
   upload(c->bins, bins2, nb, c->stream);
   upload(c->coords, coords2, (size_t)w * h, c->stream);
@@ -585,13 +628,12 @@ int pk_env_build(pk_ctx* c, const uint8_t* rgbe, uint32_t w, uint32_t h) {
   return guarded(c, [&]() {
     if (!rgbe || !w || !h) return fail(c, PK_ERR_ARG, "empty environment");
     if ((uint64_t)w * h >= (1ull << 31)) return fail(c, PK_ERR_ARG, "environment too large");
+    drop_env(c);
     upload(c->rgbe, rgbe, (size_t)w * h, c->stream);
     std::string why;
     uint32_t nb = 0;
-    if (build_env_tables_gpu(c->scratch(), c->rgbe.p, w, h, c->bins, nb, c->coords, c->pdf, why)) {
-      c->env_ready = false;
+    if (build_env_tables_gpu(c->scratch(), c->rgbe.p, w, h, c->bins, nb, c->coords, c->pdf, why))
       return fail(c, PK_ERR_ARG, "pk_env_build: " + why);
-    }
     c->env_w = w; c->env_h = h; c->env_nb = nb;
     c->env_ready = true;
     c->invalidate_graph();

@@ -1,7 +1,9 @@
 """What one call leaves behind for the next on the same context."""
+import numpy as np
 import pytest
 
 from pike_gb300 import _lib, synth
+from pike_gb300._lib import ptr
 
 from helpers import Pair, assert_bits_equal
 
@@ -32,3 +34,72 @@ def test_passes_after_a_frame_of_the_chunked_schedule(oracle, pk_built, mode):
     for p in (used, fresh):
         p.ctx.call("pk_set_trace_mode", mode)
     assert_bits_equal(pass_by_pass(used, 4), pass_by_pass(fresh, 4), f"mode {mode}")
+
+
+def cast(ctx, n=64):
+    torch = pytest.importorskip("torch")
+    o, d = torch.zeros((n, 4), device="cuda"), torch.ones((n, 4), device="cuda")
+    hits = torch.zeros((n, 4), dtype=torch.int32, device="cuda")
+    idx, cnt = torch.zeros(n, dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    for call in ("pk_cast_rays", "pk_cast_rays_noalloc"):
+        ctx.call(call, o.data_ptr(), d.data_ptr(), n, 0, hits.data_ptr(), idx.data_ptr(), cnt.data_ptr())
+
+
+def upload_bvh(ctx, nodes, tris, verts):
+    ctx.call("pk_bvh_upload", ptr(nodes), nodes.shape[0], ptr(tris), tris.shape[0], ptr(verts), verts.shape[0])
+
+
+def frame(pair, bounces=4):
+    pair.ctx.call("pk_set_render_state", 0, 0.0)
+    pair.ctx.call("pk_render_frame", bounces)
+    pair.ctx.call("pk_sync")
+    return pair.image("accum")
+
+
+@pytest.mark.parametrize("mode", [_lib.PK_TRACE_PERSISTENT, _lib.PK_TRACE_PERSISTENT | _lib.PK_TRACE_WIDE,
+                                  _lib.PK_TRACE_PERSISTENT | _lib.PK_TRACE_EXACT])
+def test_refused_bvh_leaves_nothing_to_traverse(oracle, pk_built, mode):
+    """A malformed upload over a BVH in use, with a captured frame: every traversal
+    is refused until a sound BVH is there, and then gives the first image again."""
+    src = synth.small_scene(width=64, height=48)
+    pair = Pair(src, oracle)
+    c, b = pair.ctx, pair.P.bvh
+    c.call("pk_set_trace_mode", mode)
+    want = frame(pair)
+    bad = np.ascontiguousarray(b.nodes[:5]).copy()
+    bad[0, :2] = (7, -1)  # a child outside the tree
+    with pytest.raises(_lib.PikeError):
+        upload_bvh(c, bad, np.ascontiguousarray(b.tris[:3]), b.verts)
+    for call in (lambda: frame(pair), lambda: cast(c), lambda: c.call("pk_trace")):
+        with pytest.raises(_lib.PikeError):
+            call()
+    upload_bvh(c, b.nodes, b.tris, b.verts)
+    cast(c)
+    assert_bits_equal(frame(pair), want, "after a sound upload")
+    c.call("pk_bvh_build", _lib.PK_BVH_SWEEP)
+    assert_bits_equal(frame(pair), want, "after a build")
+
+
+@pytest.mark.parametrize("mode", [_lib.PK_TRACE_WIDE, _lib.PK_TRACE_EXACT])
+def test_bvh_that_only_the_drop_in_records_hold(oracle, pk_built, mode):
+    """Two parents of one pair of leaves: the drop-in's records hold that, a tree
+    with each node reached once is needed for the others.  Refused there, usable here."""
+    src = synth.small_scene(width=64, height=48)
+    pair = Pair(src, oracle)
+    c, b = pair.ctx, pair.P.bvh
+    box = b.nodes[0, 2:]
+    nodes = np.array([[1, -1, *box], [3, -1, *box], [3, -1, *box], [-1, (2 << 24) | 0, *box], [-1, (1 << 24) | 2, *box]],
+                     np.int32)
+    tris = np.ascontiguousarray(b.tris[:3])
+    c.call("pk_set_trace_mode", _lib.PK_TRACE_PERSISTENT | mode)
+    frame(pair)
+    with pytest.raises(_lib.PikeError):
+        upload_bvh(c, nodes, tris, b.verts)
+    with pytest.raises(_lib.PikeError):
+        frame(pair)
+    cast(c)
+    c.call("pk_set_trace_mode", _lib.PK_TRACE_PERSISTENT)
+    got = frame(pair)
+    c.call("pk_set_trace_mode", _lib.PK_TRACE_CHUNKED)
+    assert_bits_equal(frame(pair), got, "the drop-in's records")
