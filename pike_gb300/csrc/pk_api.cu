@@ -137,12 +137,9 @@ void require_config(pk_ctx* c) {
 }
 void require_render(pk_ctx* c) {
   require_config(c);
-  if (!c->bvh_ready) throw std::runtime_error("no BVH: call pk_bvh_build or pk_bvh_upload");
+  if (const char* gap = c->scene_gap()) throw std::runtime_error(gap);
   if (((c->trace_mode & TRACE_WIDE) && !c->wide_ready) || ((c->trace_mode & TRACE_EXACT) && !c->exact_ready))
     throw std::runtime_error("this BVH has no records for the trace mode: its build failed");
-  if (!c->n_mats || !c->n_layers) throw std::runtime_error("no materials: call pk_materials_set/upload");
-  if (!c->attrs.p) throw std::runtime_error("no scene attributes: call pk_scene_flatten/upload");
-  if (c->bvh_verts > c->n_verts) throw std::runtime_error("BVH vertices exceed the scene's vertex attributes");
   if (!c->cam_set) throw std::runtime_error("no camera: call pk_set_camera");
 }
 

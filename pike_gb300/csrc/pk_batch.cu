@@ -112,7 +112,7 @@ int pk_batch_create(pk_batch** out, pk_ctx* const* scenes, uint32_t n_scenes) {
     for (uint32_t i = 0; i < n_scenes; i++) {
       pk_ctx* c = scenes[i];
       if (!c || c->device != b->device) return bfail(b, PK_ERR_ARG, "scenes must be contexts on one device");
-      if (!c->bvh_ready || !c->env_ready || !c->attrs.p || !c->mat4.p)
+      if (c->scene_gap() || !c->env_ready)
         return bfail(b, PK_ERR_STATE, "every scene needs a BVH, materials and an environment");
       const LaunchCtx L = c->launch();
       b->ctxs.push_back(c);

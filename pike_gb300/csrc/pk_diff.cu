@@ -607,7 +607,7 @@ int diff_fail(pk_ctx* c, int code, const char* msg) {
 }
 
 int diff_check(pk_ctx* c, const pk_diff_params* p, DiffParams& dp) {
-  if (!c->bvh_ready) return diff_fail(c, PK_ERR_STATE, "pk_diff: no BVH");
+  if (const char* gap = c->scene_gap()) return diff_fail(c, PK_ERR_STATE, gap);
   if (!c->W || !c->H) return diff_fail(c, PK_ERR_STATE, "pk_diff: call pk_configure first");
   if (!c->cam_set) return diff_fail(c, PK_ERR_STATE, "pk_diff: call pk_set_camera first");
   if (!c->diff_env_ready) return diff_fail(c, PK_ERR_STATE, "pk_diff: call pk_diff_set_env_sampling first");

@@ -1,11 +1,13 @@
 """What one call leaves behind for the next on the same context."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
 from pike_gb300 import _lib, synth
-from pike_gb300._lib import ptr
+from pike_gb300._lib import Context, ptr
 
-from helpers import Pair, assert_bits_equal
+from helpers import Pair, assert_bits_equal, camera_struct
 
 pytestmark = pytest.mark.gpu
 
@@ -103,3 +105,41 @@ def test_bvh_that_only_the_drop_in_records_hold(oracle, pk_built, mode):
     got = frame(pair)
     c.call("pk_set_trace_mode", _lib.PK_TRACE_CHUNKED)
     assert_bits_equal(frame(pair), got, "the drop-in's records")
+
+
+@pytest.mark.parametrize("lacks", ["materials", "attributes", "vertices"])
+def test_paths_need_the_whole_scene(pk_built, lacks):
+    """Differentiable and batched rendering refuse what frames refuse: a BVH
+    without materials, without vertex attributes, or with more vertices than those."""
+    torch = pytest.importorskip("torch")
+    from pike_gb300.batch import Batch, scene_context
+    from pike_gb300.diff import DiffScene
+    src = synth.small_scene(width=32, height=24)
+    whole = DiffScene(src, 32, 24, spp=1, depth=2)
+    params = whole.source_params(env_size=(32, 16))
+    whole.render(*params)
+    donor = scene_context(src)
+    n, k = C.c_uint32(), C.c_uint32()
+    donor.call("pk_bvh_info", C.byref(n), C.byref(k), None)
+    nodes, tris = np.zeros((n.value, 5), np.int32), np.zeros((k.value, 4), np.int32)
+    verts = np.zeros((src.pos.shape[0], 4), np.float32)
+    donor.call("pk_bvh_download", ptr(nodes), ptr(tris), ptr(verts))
+    ctx = Context(0)
+    ctx.call("pk_configure", 32, 24, 32 * 24)
+    if lacks != "materials":
+        ctx.call("pk_materials_set", ptr(np.ascontiguousarray(src.materials, np.float64)), src.materials.shape[0])
+    if lacks != "attributes":
+        m = 3 if lacks == "vertices" else src.pos.shape[0]
+        ctx.call("pk_scene_upload", ptr(np.array([[0, 1, 2, 0]], np.int32)), 1,
+                 ptr(np.ascontiguousarray(src.pos[:m], np.float64)), ptr(np.zeros((m, 4), np.uint32)), m)
+    upload_bvh(ctx, nodes, tris, verts)
+    ctx.call("pk_env_build", ptr(src.env_rgbe), src.env_rgbe.shape[1], src.env_rgbe.shape[0])
+    with pytest.raises(_lib.PikeError):
+        Batch([ctx])
+    part = DiffScene.__new__(DiffScene)
+    part.__dict__.update(whole.__dict__, ctx=ctx, env_shape=None)
+    ctx.call("pk_set_camera", C.byref(camera_struct(whole.camera_state)))
+    with pytest.raises(_lib.PikeError):
+        part.render(*params)
+    with pytest.raises(_lib.PikeError):
+        part.backward(*params, torch.ones((24, 32, 4), device="cuda"))
