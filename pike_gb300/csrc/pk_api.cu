@@ -138,6 +138,7 @@ void require_config(pk_ctx* c) {
 void require_render(pk_ctx* c) {
   require_config(c);
   if (const char* gap = c->scene_gap()) throw std::runtime_error(gap);
+  if (c->bvh_verts > c->n_verts) throw std::runtime_error("BVH vertices exceed the scene's vertex attributes");
   if (((c->trace_mode & TRACE_WIDE) && !c->wide_ready) || ((c->trace_mode & TRACE_EXACT) && !c->exact_ready))
     throw std::runtime_error("this BVH has no records for the trace mode: its build failed");
   if (!c->cam_set) throw std::runtime_error("no camera: call pk_set_camera");

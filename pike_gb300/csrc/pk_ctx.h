@@ -218,7 +218,6 @@ struct pk_ctx {
     if (!bvh_ready) return "no BVH: call pk_bvh_build or pk_bvh_upload";
     if (!n_mats || !n_layers) return "no materials: call pk_materials_set/upload";
     if (!attrs.p) return "no scene attributes: call pk_scene_flatten/upload";
-    if (bvh_verts > n_verts) return "BVH vertices exceed the scene's vertex attributes";
     return nullptr;
   }
   // The drop-in's traversal records (the reference's snorm16 boxes and root),

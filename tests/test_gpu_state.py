@@ -109,8 +109,8 @@ def test_bvh_that_only_the_drop_in_records_hold(oracle, pk_built, mode):
 
 @pytest.mark.parametrize("lacks", ["materials", "attributes", "vertices"])
 def test_paths_need_the_whole_scene(pk_built, lacks):
-    """Differentiable and batched rendering refuse what frames refuse: a BVH
-    without materials, without vertex attributes, or with more vertices than those."""
+    """Differentiable and batched rendering refuse a BVH without materials or vertex
+    attributes, as frames do.  Vertices beyond the attributes take the first one's there."""
     torch = pytest.importorskip("torch")
     from pike_gb300.batch import Batch, scene_context
     from pike_gb300.diff import DiffScene
@@ -134,11 +134,16 @@ def test_paths_need_the_whole_scene(pk_built, lacks):
                  ptr(np.ascontiguousarray(src.pos[:m], np.float64)), ptr(np.zeros((m, 4), np.uint32)), m)
     upload_bvh(ctx, nodes, tris, verts)
     ctx.call("pk_env_build", ptr(src.env_rgbe), src.env_rgbe.shape[1], src.env_rgbe.shape[0])
-    with pytest.raises(_lib.PikeError):
-        Batch([ctx])
     part = DiffScene.__new__(DiffScene)
     part.__dict__.update(whole.__dict__, ctx=ctx, env_shape=None)
     ctx.call("pk_set_camera", C.byref(camera_struct(whole.camera_state)))
+    if lacks == "vertices":
+        Batch([ctx])
+        part.render(*params)
+        part.backward(*params, torch.ones((24, 32, 4), device="cuda"))
+        return
+    with pytest.raises(_lib.PikeError):
+        Batch([ctx])
     with pytest.raises(_lib.PikeError):
         part.render(*params)
     with pytest.raises(_lib.PikeError):
