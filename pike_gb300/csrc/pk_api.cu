@@ -176,6 +176,7 @@ int pk_create(pk_ctx** out, int device) {
     check(cudaHostAlloc(reinterpret_cast<void**>(&c->host_words), 64, cudaHostAllocMapped), "cudaHostAlloc");
     check(cudaHostGetDevicePointer(reinterpret_cast<void**>(&c->host_words_dev), c->host_words, 0),
           "cudaHostGetDevicePointer");
+    c->cast_space.alloc(cast_kept_bytes());
     c->cast_scratch = noalloc_scratch_address();
     check(cudaMemsetAsync(c->ctr.p, 0, sizeof(Counters), c->stream), "memset");
     check(cudaStreamSynchronize(c->stream), "sync");

@@ -109,9 +109,18 @@ __global__ void __launch_bounds__(LIST_THREADS) k_hit_list(const uint4* __restri
 
 // Small queries (at most CAST_ONE rays): one launch of one block traces a ray
 // per thread and lists the hits, since launches, memsets and a copy are most
-// of such a query: 257 rays in the 770-triangle scene, the whole call from
-// Python, 59 -> 45 us.
-constexpr uint32_t CAST_ONE = 1024;
+// of such a query.  Where the line lies, one block against k_cast and k_hit_list,
+// whole calls of pk_cast_rays_noalloc from Python in us, closest hits:
+//   rays                                     257      512      768     1024
+//   770 triangles, random rays            37  47   39  46   44  46   45  45
+//   1,310,730 triangles, random           60  69   65  72   69  69   75  73
+//   the same, one view                    35  43   36  44   46  45  180 176
+//   524,288 loose triangles, random      222 190  249 207  273 212  305 210
+//   the same, one view                   132 118  156 134  210 156  285 193
+// Loose triangles are many steps a ray, and one SM does not hide their latency;
+// even there a block of up to 512 rays is no slower than these queries were
+// before it (244, 256, 254, 251 us; one view 154, 168, 206, 251).
+constexpr uint32_t CAST_ONE = 512;
 constexpr int ONE_SMEM = 8;
 template <bool ANY>
 __global__ void __launch_bounds__(CAST_ONE) k_cast_one(SceneDev sc, const float4* __restrict__ o4,
@@ -159,6 +168,10 @@ struct CastScratch {
 };
 size_t cast_tiles(uint32_t n) { return ((size_t)n + LIST_TILE - 1) / LIST_TILE; }
 size_t cast_bytes(uint32_t n) { return 16 + 8 * cast_tiles(n); }
+// Queries of up to this many rays use 4 KB that the context keeps (taking the
+// scratch from the pool: 4-5 us of a call).
+constexpr uint32_t CAST_KEPT_RAYS = 1u << 20;
+size_t cast_kept_bytes() { return cast_bytes(CAST_KEPT_RAYS); }  // pk_create
 
 // The query on the context's stream; returns when it has finished.  `space`:
 // cast_bytes(n) bytes of scratch when n > CAST_ONE.
@@ -204,9 +217,10 @@ extern "C" int pk_cast_rays(pk_ctx* c, const float* ray_o4, const float* ray_d4,
     if (!c->bvh_ready) { c->err = "pk_cast_rays: no BVH"; return PK_ERR_STATE; }
     if ((n && (!ray_o4 || !ray_d4 || !hits4 || !hit_index)) || !n_hits) { c->err = "pk_cast_rays: null buffer"; return PK_ERR_ARG; }
     if (n > (1u << 30)) { c->err = "pk_cast_rays: too many rays"; return PK_ERR_ARG; }
-    TmpBuf<unsigned char> space(c->scratch(), n > CAST_ONE ? cast_bytes(n) : 0);
+    const bool kept = n <= CAST_KEPT_RAYS;
+    TmpBuf<unsigned char> space(c->scratch(), kept ? 0 : cast_bytes(n));
     return cast_run(c, "pk_cast_rays", reinterpret_cast<const float4*>(ray_o4), reinterpret_cast<const float4*>(ray_d4),
-                    n, any_hit, reinterpret_cast<uint4*>(hits4), hit_index, n_hits, space.p);
+                    n, any_hit, reinterpret_cast<uint4*>(hits4), hit_index, n_hits, kept ? c->cast_space.p : space.p);
   } catch (CudaError& e) {
     c->err = e.what();
     return PK_ERR_CUDA;
@@ -215,7 +229,8 @@ extern "C" int pk_cast_rays(pk_ctx* c, const float* ray_o4, const float* ray_d4,
 
 // ---- allocation-free variant -------------------------------------------------
 // pk_cast_rays takes its scratch (work tickets and the look-back states of the
-// hit list) from the context's pool, which can allocate.
+// hit list) for more than CAST_KEPT_RAYS rays from the context's pool, which can
+// allocate.
 // pk_cast_rays_noalloc takes it from the file-scope array below instead, so it
 // allocates and frees nothing.  Every GPU that loads the library holds one copy
 // of the array until the process exits.

@@ -60,6 +60,7 @@ struct FrameSlot {
 // Device address of pk_cast_rays_noalloc's static scratch array on the
 // current device (pk_cast.cu).
 void* noalloc_scratch_address();
+size_t cast_kept_bytes();
 
 }  // namespace pk
 
@@ -176,6 +177,7 @@ struct pk_ctx {
   // synchronise: an error status without a copy.
   uint32_t* host_words = nullptr;
   uint32_t* host_words_dev = nullptr;
+  DevBuf<unsigned char> cast_space;  // scratch of pk_cast_rays for up to CAST_KEPT_RAYS rays
   void* cast_scratch = nullptr;  // pk_cast_rays_noalloc's static scratch on this device (set by pk_create)
 
   RayQ R(int i) { return slot[0].R(i); }

@@ -7,6 +7,7 @@ import pytest
 from pike_gb300 import _lib, synth
 from pike_gb300._lib import Context, ptr
 
+import test_gpu_edges
 from helpers import Pair, assert_bits_equal, camera_struct
 
 pytestmark = pytest.mark.gpu
@@ -46,6 +47,33 @@ def cast(ctx, n=64):
     torch.cuda.synchronize()
     for call in ("pk_cast_rays", "pk_cast_rays_noalloc"):
         ctx.call(call, o.data_ptr(), d.data_ptr(), n, 0, hits.data_ptr(), idx.data_ptr(), cnt.data_ptr())
+
+
+@pytest.mark.parametrize("n", [511, 512, 513])
+@pytest.mark.parametrize("any_hit", [False, True])
+def test_queries_around_one_block(oracle, pk_built, n, any_hit):
+    test_gpu_edges.test_queries_at_block_and_tile_edges(oracle, pk_built, n, any_hit)
+
+
+def test_queries_beyond_the_kept_scratch(oracle, pk_built):
+    """2^20 rays use the context's scratch, more take theirs from the pool: one query
+    of both kinds and the same rays in two of the first."""
+    torch = pytest.importorskip("torch")
+    ctx = Pair(synth.small_scene(width=8, height=8), oracle).ctx
+    n, half = (1 << 20) + 5, 1 << 19
+    g = torch.Generator().manual_seed(1)
+    o = torch.nn.functional.pad(torch.rand((n, 3), generator=g) * 1.8 - 0.9, (0, 1)).cuda()
+    d = torch.nn.functional.pad(torch.randn((n, 3), generator=g), (0, 1)).cuda()
+
+    def query(o, d):
+        hits = torch.zeros((o.shape[0], 4), dtype=torch.int32, device="cuda")
+        idx, cnt = torch.zeros(o.shape[0], dtype=torch.int32, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+        torch.cuda.synchronize()
+        ctx.call("pk_cast_rays", o.data_ptr(), d.data_ptr(), o.shape[0], 0, hits.data_ptr(), idx.data_ptr(), cnt.data_ptr())
+        return hits, idx[:cnt.item()]
+    whole, a, b = query(o, d), query(o[:half], d[:half]), query(o[half:], d[half:])
+    assert torch.equal(whole[0], torch.cat([a[0], b[0]]))
+    assert torch.equal(whole[1], torch.cat([a[1], b[1] + half]))
 
 
 def upload_bvh(ctx, nodes, tris, verts):
