@@ -478,6 +478,7 @@ static int finish_bvh(pk_ctx* c) {
   check(cudaMemcpyAsync(back, out.p, 8, cudaMemcpyDeviceToHost, c->stream), "D2H");
   check(cudaStreamSynchronize(c->stream), "sync");
   c->root = (int)back[0];
+  check_lookback(back[1], "BVH records");
   if (back[1]) return fail(c, PK_ERR_ARG, "malformed BVH (child index, leaf size >= 128 or vertex index out of range)");
   c->bvh_ready = true;
   if (c->trace_mode & TRACE_WIDE) {

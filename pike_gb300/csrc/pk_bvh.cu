@@ -620,6 +620,7 @@ int build_bvh_binned(const Scratch& w, const double* pos3, uint32_t n_verts, con
     uint32_t lerr = 0;
     check(cudaMemcpyAsync(&lerr, derr.p, 4, cudaMemcpyDeviceToHost, s), "D2H");
     check(cudaStreamSynchronize(s), "sync");
+    check_lookback(lerr, "binned build");
     if (lerr) { why = "binned partition out of range"; return 1; }
     std::vector<NodeInfo> nl;
     for (uint32_t k = 0; k < m; k++) {

@@ -343,12 +343,15 @@ __device__ __forceinline__ float lv_limit(const Level& L, uint32_t k, uint32_t c
 }
 __device__ __forceinline__ bool beyond(uint32_t cost_bits, float limit) { return __uint_as_float(cost_bits) > limit; }
 
-__global__ void k_lv_start(Level L, uint32_t T) {  // the root alone
+// The root alone.  After a failed sort the lists hold no triangle numbers: no
+// nodes and no tiles then, so that no kernel of any level reads them.
+__global__ void k_lv_start(Level L, uint32_t T) {
   const uint32_t nt = (T + LV_TILE - 1) / LV_TILE;
   if (blockIdx.x == 0 && threadIdx.x == 0) {
+    const bool ok = L.ctl->err == 0u;
     L.node[0][0] = LNode{0u, T, 0u, nt};
-    L.ctl->n_nodes = 1;
-    L.ctl->n_tiles = nt;
+    L.ctl->n_nodes = ok ? 1u : 0u;
+    L.ctl->n_tiles = ok ? nt : 0u;
     L.big_off[0] = 0;
   }
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nt; t += gridDim.x * blockDim.x)
@@ -984,6 +987,7 @@ __device__ __forceinline__ double exact_cost(const StShared& S, const KBox* kbox
 __global__ void __launch_bounds__(ST_THREADS, ST_BLOCKS) k_subtree(Subtrees W) {
   extern __shared__ __align__(16) unsigned char st_raw[];
   StShared& S = *reinterpret_cast<StShared*>(st_raw);
+  if (W.ctl->err & ERR_LOOKBACK) return;  // the tasks were not placed; this kernel sets other bits only
   const SmallTask task = W.task[blockIdx.x];
   const uint32_t n0 = task.count, start = task.start;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
@@ -1496,7 +1500,7 @@ int build_bvh_sweep(const Scratch& w, const double* pos3, uint32_t n_verts, cons
   auto read_ctl = [&]() {
     check(cudaMemcpyAsync(&host, ctl.p, sizeof host, cudaMemcpyDeviceToHost, s), "D2H");
     check(cudaStreamSynchronize(s), "sync");
-    if (host.err & ERR_LOOKBACK) { why = "a look-back timed out"; return 1; }
+    check_lookback(host.err, "BVH build");
     if (host.err) { why = "degenerate node (no finite SAH cost) or a leaf of 128+ triangles"; return 1; }
     return 0;
   };

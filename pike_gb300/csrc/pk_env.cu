@@ -82,6 +82,7 @@ __global__ void k_env_plan(const double* __restrict__ prefix, const unsigned lon
   plan->nb = 0;
   plan->total = total;
   plan->status = 1;
+  if (plan->err) return;  // the sort failed: nothing below may follow its order
   if (!(total > 0.0) || !isfinite(total) || !(brightest > 0.0)) return;
   // numBins = min(256, max(32, 2 * ceil(total / brightest)))
   const double lo = fmin(256.0, fmax(32.0, 2.0 * ceil(total * (1.0 - rel) / brightest)));
@@ -373,7 +374,7 @@ int build_from_radiance(const Scratch& sc, uint32_t w, uint32_t h, TmpBuf<double
   EnvPlan host;
   check(cudaMemcpyAsync(&host, plan.p, sizeof host, cudaMemcpyDeviceToHost, s), "D2H");
   check(cudaStreamSynchronize(s), "sync");
-  if (host.err) { why = "radix sort look-back timed out"; return 1; }
+  check_lookback(host.err, "environment sort");
   if (host.status) {
     std::vector<double> r(n);
     std::vector<uint32_t> order(n);
@@ -441,7 +442,7 @@ int build_env_alias_gpu(const Scratch& sc, const uchar4* rgbe, uint32_t w, uint3
   check(cudaMemcpyAsync(st, status.p, 12, cudaMemcpyDeviceToHost, s), "D2H");
   check(cudaStreamSynchronize(s), "sync");
   const uint32_t nl = st[1];
-  if (st[2]) { why = "prefix sum look-back timed out"; return 1; }
+  check_lookback(st[2], "alias table");
   if (st[0]) { why = "black or non-finite environment"; return 1; }
   const uint32_t nh = n - nl;
   check(cudaMemsetAsync(ldef.p + nl, 0, 8, s), "memset");  // D(nl) after the scan: all deficits

@@ -190,6 +190,7 @@ int convert_bvh(const Scratch& w, const int32_t* nodes5, uint32_t n_nodes, const
   // nodes in index order (a depth-first order was measured no faster: 3012-3015
   // against 3022-3032 Mrays/s at 1080p)
   k_inner_flags<<<(n_nodes + 255) / 256, 256, 0, s>>>(nodes5, n_nodes, rank.p);
+  // (ranks that a timed-out look-back left too small still lie below n_nodes)
   scan_exclusive_u32(w, rank.p, rank.p, n_nodes, nullptr, err);
   k_inner_records<<<(n_nodes + 255) / 256, 256, 0, s>>>(nodes5, n_nodes, rank.p, n_tris, inner, root_code, err);
   k_inner_records32<<<(n_nodes + 255) / 256, 256, 0, s>>>(nodes5, n_nodes, rank.p, inner, inner32);

@@ -39,6 +39,19 @@ cudaMemPool_t create_scratch_pool(int device) {
   return pool;
 }
 
+void check_lookback(uint32_t err, const char* what) {
+  if (err & ERR_LOOKBACK) throw CudaError(std::string(what) + ": a look-back timed out");
+}
+
+// A test's build says which look-backs (of n elements) give up at once, so that
+// what follows a wait that ran out can be watched.
+#ifndef PK_SCAN_GIVES_UP
+#define PK_SCAN_GIVES_UP(n) false
+#endif
+#ifndef PK_SORT_GIVES_UP
+#define PK_SORT_GIVES_UP(n) false
+#endif
+
 constexpr int SCAN_THREADS = 256;
 constexpr int SCAN_ITEMS = 8;
 constexpr int SCAN_TILE = SCAN_THREADS * SCAN_ITEMS;
@@ -67,7 +80,9 @@ __global__ void __launch_bounds__(SCAN_THREADS) k_scan_u32(const uint32_t* in, u
     uint32_t ea, eb, ta, tb;
     block_scan2<SCAN_THREADS / 32>(sum, 0u, ea, eb, ta, tb, s_warp);
     if (threadIdx.x < 32) {
-      const unsigned long long e = lookback2_warp(tiles, tile, pack2(ta, 0u), err);
+      unsigned long long e = 0;
+      if (!PK_SCAN_GIVES_UP(n)) e = lookback2_warp(tiles, tile, pack2(ta, 0u), err);
+      else if (tile) atomicOr(err, ERR_LOOKBACK);
       if (threadIdx.x == 0) s_excl = e;
     }
     __syncthreads();
@@ -329,7 +344,8 @@ __global__ void __launch_bounds__(SORT_THREADS) k_sort_pass(const uint64_t* __re
   W before = 0;
   if (tile) {  // SORT_BACK earlier tiles at a time, back to the nearest inclusive prefix
     const W* p = mine;
-    bool found = false;
+    bool found = PK_SORT_GIVES_UP(n);
+    if (found) atomicOr(err, ERR_LOOKBACK);
     for (uint32_t t = tile; t && !found; p -= SORT_BACK * RADIX, t = t > SORT_BACK ? t - SORT_BACK : 0u) {
       W v[SORT_BACK];
 #pragma unroll
@@ -441,26 +457,28 @@ int tree_levels(const Scratch& w, const int32_t* nodes5, uint32_t n_nodes, TmpBu
   const cudaStream_t s = w.s;
   order.alloc(std::max<uint32_t>(n_nodes, 1u));
   check(cudaMemsetAsync(order.p, 0, 4, s), "memset");  // the root
-  TmpBuf<uint32_t> flag(w, std::max<uint32_t>(n_nodes, 1u)), tot(w, 2);  // tot: inner nodes of the level, errors
-  check(cudaMemsetAsync(tot.p, 0, 8, s), "memset");
+  // tot: inner nodes of the level, a look-back's errors, the tree's errors
+  TmpBuf<uint32_t> flag(w, std::max<uint32_t>(n_nodes, 1u)), tot(w, 3);
+  check(cudaMemsetAsync(tot.p, 0, 12, s), "memset");
   level.assign(1, 0u);
   uint32_t b = 0, e = n_nodes ? 1u : 0u;
-  uint32_t c = 0;
+  uint32_t c[2] = {0, 0};
   while (b < e) {
     level.push_back(e);
     const unsigned blocks = (e - b + 127) / 128;
     k_level_flags<<<blocks, 128, 0, s>>>(nodes5, order.p, b, e, flag.p);
     scan_exclusive_u32(w, flag.p, flag.p, e - b, tot.p, tot.p + 1);
-    check(cudaMemcpyAsync(&c, tot.p, 4, cudaMemcpyDeviceToHost, s), "D2H");
+    check(cudaMemcpyAsync(c, tot.p, 8, cudaMemcpyDeviceToHost, s), "D2H");
     check(cudaStreamSynchronize(s), "sync");
-    const uint64_t next_end = (uint64_t)e + 2ull * c;
+    check_lookback(c[1], "tree levels");  // before the ranks place anything
+    const uint64_t next_end = (uint64_t)e + 2ull * c[0];
     if (next_end > n_nodes) return 1;
-    k_level_children<<<blocks, 128, 0, s>>>(nodes5, order.p, b, e, flag.p, n_nodes, tot.p + 1);
+    k_level_children<<<blocks, 128, 0, s>>>(nodes5, order.p, b, e, flag.p, n_nodes, tot.p + 2);
     b = e;
     e = (uint32_t)next_end;
   }
   uint32_t herr = 0;
-  check(cudaMemcpyAsync(&herr, tot.p + 1, 4, cudaMemcpyDeviceToHost, s), "D2H");
+  check(cudaMemcpyAsync(&herr, tot.p + 2, 4, cudaMemcpyDeviceToHost, s), "D2H");
   check(cudaStreamSynchronize(s), "sync");
   return (e != n_nodes || herr) ? 1 : 0;
 }

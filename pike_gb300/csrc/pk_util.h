@@ -109,9 +109,14 @@ struct TmpBuf {
 // Exclusive prefix sum of n u32 values (in may alias out).  If total is not
 // null it receives the sum (device pointer).  Counts must stay below 2^31.
 // Enqueues and returns; a look-back that timed out sets ERR_LOOKBACK in *err
-// (device), which the caller reads with the rest of its results.
+// (device).  The prefixes are then too small, each by some amount, and a sort's
+// arrays hold words that were never written: whatever uses either as an index
+// comes after a check of *err, on the host (check_lookback) or in a kernel.
 void scan_exclusive_u32(const Scratch& w, const uint32_t* in, uint32_t* out, uint32_t n, uint32_t* total,
                         uint32_t* err);
+
+// Throws when the look-back bit of `err` is set.
+void check_lookback(uint32_t err, const char* what);
 
 // Exclusive prefix sum of n u64 values (in may alias out); enqueues and returns.
 void scan_exclusive_u64(const Scratch& w, const unsigned long long* in, unsigned long long* out, size_t n);

@@ -600,18 +600,20 @@ int build_wide_bvh_gpu(const Scratch& w, const int32_t* nodes5, uint32_t n_nodes
   check(cudaMemcpyAsync(items.p, &root, sizeof(Item), cudaMemcpyHostToDevice, s), "H2D");
   uint32_t n = 1, node_base = 0, tri_base = 0;
   depth = 0;
-  TmpBuf<uint32_t> n_inner(w), n_tri(w), tot(w, 2);
+  TmpBuf<uint32_t> n_inner(w), n_tri(w), tot(w, 3);  // tot: both sums, a look-back's errors
+  check(cudaMemsetAsync(tot.p, 0, 12, s), "memset");
   while (n) {
     depth++;
     n_inner.alloc(n);
     n_tri.alloc(n);
     k_wide_count<<<blocks(n), 128, 0, s>>>(V, items.p, n, n_inner.p, n_tri.p);
     check(cudaGetLastError(), "k_wide_count");
-    scan_exclusive_u32(w, n_inner.p, n_inner.p, n, tot.p, err.p);
-    scan_exclusive_u32(w, n_tri.p, n_tri.p, n, tot.p + 1, err.p);
-    uint32_t th[2];
-    check(cudaMemcpyAsync(th, tot.p, 8, cudaMemcpyDeviceToHost, s), "D2H");
+    scan_exclusive_u32(w, n_inner.p, n_inner.p, n, tot.p, tot.p + 2);
+    scan_exclusive_u32(w, n_tri.p, n_tri.p, n, tot.p + 1, tot.p + 2);
+    uint32_t th[3];
+    check(cudaMemcpyAsync(th, tot.p, 12, cudaMemcpyDeviceToHost, s), "D2H");
     check(cudaStreamSynchronize(s), "sync");
+    check_lookback(th[2], "wide BVH");
     if ((uint64_t)tri_base + th[1] > n_tris) { why = "internal: triangle count mismatch"; return 1; }
     if ((size_t)node_base + n > cap) {
       const size_t ncap = std::max((size_t)node_base + n, 2 * cap);
@@ -652,10 +654,15 @@ int build_exact_binary_gpu(const Scratch& w, const int32_t* nodes5, uint32_t n_n
   check(cudaMemsetAsync(err.p, 0, 4, s), "memset");
   Prepared P(w);
   if (prepare(w, nodes5, n_nodes, tri4, n_tris, verts4, n_verts, err, P, why)) return 1;
-  TmpBuf<uint32_t> rank(w, n_nodes), tot(w, 1);
+  TmpBuf<uint32_t> rank(w, n_nodes), tot(w, 2);  // tot: inner nodes, a look-back's errors
+  check(cudaMemsetAsync(tot.p, 0, 8, s), "memset");
   k_inner_flags<<<blocks(n_nodes), 128, 0, s>>>(nodes5, n_nodes, rank.p);
-  scan_exclusive_u32(w, rank.p, rank.p, n_nodes, tot.p, err.p);
-  const uint32_t n_inner = read_u32(s, tot.p);
+  scan_exclusive_u32(w, rank.p, rank.p, n_nodes, tot.p, tot.p + 1);
+  uint32_t th[2];
+  check(cudaMemcpyAsync(th, tot.p, 8, cudaMemcpyDeviceToHost, s), "D2H");
+  check(cudaStreamSynchronize(s), "sync");
+  check_lookback(th[1], "exact binary records");
+  const uint32_t n_inner = th[0];
   records.alloc(4 * (size_t)std::max<uint32_t>(n_inner, 1u));
   check(cudaMemsetAsync(records.p, 0, records.bytes(), s), "memset");
   TmpBuf<int32_t> rc(w, 1);
