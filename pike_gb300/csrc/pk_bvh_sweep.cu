@@ -152,8 +152,10 @@ __device__ __forceinline__ uint32_t rounded(double v, double lo, double scale) {
 }
 
 // Frame of a box: lower corner and a power of two that maps its largest extent
-// into (1/2, 1]; unusable (every cost then evaluated in double) when the extent
-// is not a positive finite number.
+// into (1/2, 1]; unusable (every cost then evaluated in double) when the double
+// areas may leave the normal numbers.  cost_bound accepts areas down to 2^-40 of
+// the squared extent: from 1e-140 on they are normal and what underflows in the
+// areas inside them is below 1e-20 of them; up to 1e150 sums of products stay finite.
 struct Frame {
   double lo[3], scale;
   bool ok;
@@ -166,7 +168,7 @@ __device__ __forceinline__ Frame frame_of(const KBox& b) {
     f.lo[a] = val_of(b.mn[a]);
     ext = fmax(ext, val_of(b.mx[a]) - f.lo[a]);
   }
-  f.ok = ext > 1e-290 && ext < 1e290;
+  f.ok = ext > 1e-140 && ext < 1e150;
   int e = 0;
   if (f.ok) frexp(ext, &e);
   f.scale = f.ok ? ldexp(1.0, -e) : 0.0;

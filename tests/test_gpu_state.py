@@ -1,4 +1,5 @@
-"""What one call leaves behind for the next on the same context."""
+"""What one call leaves behind for the next on the same context, and builds at
+scales where the reference's own arithmetic gives out."""
 import ctypes as C
 
 import numpy as np
@@ -11,6 +12,11 @@ import test_gpu_edges
 from helpers import Pair, assert_bits_equal, camera_struct
 
 pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def ctx(pk_built):
+    return Context(0)
 
 
 def pass_by_pass(pair, bounces):
@@ -176,3 +182,31 @@ def test_paths_need_the_whole_scene(pk_built, lacks):
         part.render(*params)
     with pytest.raises(_lib.PikeError):
         part.backward(*params, torch.ones((24, 32, 4), device="cuda"))
+
+
+def build_sweep(ctx, pos, tris):
+    pos = np.ascontiguousarray(pos)
+    attrs = np.zeros((pos.shape[0], 4), np.uint32)
+    ctx.call("pk_scene_upload", ptr(tris), tris.shape[0], ptr(pos), ptr(attrs), pos.shape[0])
+    ctx.call("pk_bvh_build", _lib.PK_BVH_SWEEP)
+
+
+@pytest.mark.parametrize("n", [40, 700, 1500])
+@pytest.mark.parametrize("exponent", [-175, -165, -160, -158, -150, -141, -139, 149, 151, 153, 154, 160, 170])
+def test_sweep_build_where_areas_underflow_or_overflow(ctx, oracle, n, exponent):
+    """Extents whose products leave the normal doubles: the reference's costs are
+    then inexact or not finite, and the same trees have to come out, or the same refusals."""
+    pos, tris = test_gpu_edges.soup(n, n, spread=10.0 ** exponent)
+    try:
+        ref = oracle.BVH(np.ascontiguousarray(pos), tris)
+    except Exception:  # no finite split cost
+        with pytest.raises(_lib.PikeError):
+            build_sweep(ctx, pos, tris)
+        return
+    build_sweep(ctx, pos, tris)
+    nn, nt = C.c_uint32(), C.c_uint32()
+    ctx.call("pk_bvh_info", C.byref(nn), C.byref(nt), None)
+    assert (nn.value, nt.value) == (ref.nodes.shape[0], ref.tris.shape[0])
+    nodes, leaf = np.zeros_like(ref.nodes), np.zeros_like(ref.tris)
+    ctx.call("pk_bvh_download", ptr(nodes), ptr(leaf), None)
+    assert np.array_equal(nodes, ref.nodes) and np.array_equal(leaf, ref.tris)
