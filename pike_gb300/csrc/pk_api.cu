@@ -184,7 +184,7 @@ int pk_create(pk_ctx** out, int device) {
   });
   if (rc != PK_OK) {
     std::fprintf(stderr, "pk_create: %s\n", c->err.c_str());
-    if (c->scratch_pool) cudaMemPoolDestroy(c->scratch_pool);
+    destroy_scratch_pool(c->scratch_pool);
     if (c->host_words) cudaFreeHost(c->host_words);
     delete c;
     return rc;
@@ -216,7 +216,7 @@ int pk_destroy(pk_ctx* c) {
   for (auto e : c->event_pool) cudaEventDestroy(e);
   if (c->t0) cudaEventDestroy(c->t0);
   if (c->t1) cudaEventDestroy(c->t1);
-  if (c->scratch_pool) cudaMemPoolDestroy(c->scratch_pool);
+  destroy_scratch_pool(c->scratch_pool);
   if (c->host_words) cudaFreeHost(c->host_words);
   if (c->stream) cudaStreamDestroy(c->stream);
   delete c;

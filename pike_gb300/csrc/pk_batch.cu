@@ -314,7 +314,6 @@ int pk_batch_read(pk_batch* b, uint32_t req, float* rgba_mean) {
       try {
         b->mean.alloc(part);
       } catch (CudaError&) {  // no memory for it: scaled on the host
-        cudaGetLastError();
         check(cudaMemcpyAsync(rgba_mean, b->accum.p + q.out_offset, n * 16, cudaMemcpyDeviceToHost, b->stream), "D2H");
         check(cudaStreamSynchronize(b->stream), "sync");
         for (size_t i = 0; i < 4 * n; i++) rgba_mean[i] *= inv;

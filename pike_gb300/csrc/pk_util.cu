@@ -5,7 +5,9 @@
 #include <unistd.h>
 
 #include <algorithm>
+#include <mutex>
 #include <string>
+#include <utility>
 #include <utility>
 #include <vector>
 
@@ -27,6 +29,53 @@ void touch_pages(void* p, size_t bytes) {
   if (bytes) b[bytes - 1] = b[bytes - 1];
 }
 
+// The pools that exist, for device_malloc; contexts come and go on several threads.
+// (Never destroyed: a context may be closed after this library's statics.)
+static std::mutex& g_pools_lock = *new std::mutex;
+static std::vector<std::pair<int, cudaMemPool_t>>& g_pools = *new std::vector<std::pair<int, cudaMemPool_t>>;
+
+static void give_pools_back() {
+  int device = 0;
+  cudaGetDevice(&device);
+  std::lock_guard<std::mutex> hold(g_pools_lock);
+  for (const auto& p : g_pools)
+    if (p.first == device) cudaMemPoolTrimTo(p.second, 0);
+}
+
+template <class F>
+static void* malloc_or_throw(const char* what, F attempt) {
+  void* p = nullptr;
+  cudaError_t e = attempt(&p);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    give_pools_back();
+    e = attempt(&p);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    check(e, what);
+  }
+  return p;
+}
+void* device_malloc(size_t bytes) {
+  return malloc_or_throw("cudaMalloc", [&](void** p) { return cudaMalloc(p, bytes); });
+}
+void* scratch_malloc(const Scratch& w, size_t bytes) {
+  return malloc_or_throw("cudaMallocFromPoolAsync",
+                         [&](void** p) { return cudaMallocFromPoolAsync(p, bytes, w.pool, w.s); });
+}
+
+void destroy_scratch_pool(cudaMemPool_t pool) {
+  if (!pool) return;
+  std::lock_guard<std::mutex> hold(g_pools_lock);
+  for (size_t i = 0; i < g_pools.size(); i++)
+    if (g_pools[i].second == pool) {
+      g_pools.erase(g_pools.begin() + i);
+      break;
+    }
+  cudaMemPoolDestroy(pool);
+}
+
 cudaMemPool_t create_scratch_pool(int device) {
   cudaMemPoolProps props = {};
   props.allocType = cudaMemAllocationTypePinned;
@@ -35,7 +84,13 @@ cudaMemPool_t create_scratch_pool(int device) {
   cudaMemPool_t pool = nullptr;
   check(cudaMemPoolCreate(&pool, &props), "cudaMemPoolCreate");
   uint64_t keep = SCRATCH_KEEP;
-  check(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep), "cudaMemPoolSetAttribute");
+  const cudaError_t e = cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  if (e != cudaSuccess) {
+    cudaMemPoolDestroy(pool);
+    check(e, "cudaMemPoolSetAttribute");
+  }
+  std::lock_guard<std::mutex> hold(g_pools_lock);
+  g_pools.emplace_back(device, pool);
   return pool;
 }
 

@@ -18,16 +18,21 @@ inline void check(cudaError_t e, const char* what) {
   if (e != cudaSuccess) throw CudaError(std::string(what) + ": " + cudaGetErrorString(e));
 }
 
-// Owned device allocation (cudaMalloc / cudaFree).  alloc() keeps the block it
-// has when the new size fits it and fills at least half of it: a scene that is
-// rebuilt at about its old size then costs no cudaMalloc and no cudaFree (which
-// waits for the whole device).
 // Makes the pages of a caller's pageable buffer resident, its contents kept, before the GPU
 // copies into it: where the GPU reaches pageable memory through the host's page
 // tables, the copy engine faulted fresh pages in one by one (49 MB in 16 buffers:
 // 30-52 ms, touched by this thread first 17 ms, by eight threads 20 ms).
 void touch_pages(void* p, size_t bytes);
 
+// cudaMalloc.  When memory is short, what the scratch pools of this device's
+// contexts hold between builds is given back first; throws when that is not
+// enough, and leaves no CUDA error behind for the next call to find.
+void* device_malloc(size_t bytes);
+
+// Owned device allocation (device_malloc / cudaFree).  alloc() keeps the block it
+// has when the new size fits it and fills at least half of it: a scene that is
+// rebuilt at about its old size then costs no cudaMalloc and no cudaFree (which
+// waits for the whole device).
 template <class T>
 struct DevBuf {
   T* p = nullptr;
@@ -51,7 +56,7 @@ struct DevBuf {
     }
     release();
     if (count) {
-      check(cudaMalloc(&p, need), "cudaMalloc");
+      p = static_cast<T*>(device_malloc(need));
       n = count;
       cap = need;
     }
@@ -74,6 +79,8 @@ struct Scratch {
   cudaMemPool_t pool = nullptr;
 };
 cudaMemPool_t create_scratch_pool(int device);
+void destroy_scratch_pool(cudaMemPool_t pool);
+void* scratch_malloc(const Scratch& w, size_t bytes);  // stream-ordered; short memory as in device_malloc
 
 // A temporary of a builder; freed on the stream when it goes out of scope.
 template <class T>
@@ -89,9 +96,7 @@ struct TmpBuf {
   void alloc(size_t count) {
     release();
     if (!count) return;
-    void* q = nullptr;
-    check(cudaMallocFromPoolAsync(&q, count * sizeof(T), w.pool, w.s), "cudaMallocFromPoolAsync");
-    p = static_cast<T*>(q);
+    p = static_cast<T*>(scratch_malloc(w, count * sizeof(T)));
     n = count;
   }
   void release() {
