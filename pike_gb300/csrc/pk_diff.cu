@@ -632,9 +632,11 @@ EnvDev diff_env_dev(pk_ctx* c) {
 
 // Paths per chunk: enough to fill the GPU many times over (the tail of a
 // bounce's longest rays costs as much as some 10^5 rays), within PATH_SPACE
-// bytes of workspace that the context keeps.
+// bytes of workspace that the context keeps; half as many, again and again, when
+// the device has no memory for them, down to PATH_LEAST (1 MB at the most).
 constexpr unsigned long long PATH_CHUNK = 1ull << 22;
 constexpr unsigned long long PATH_SPACE = 3ull << 30;
+constexpr unsigned long long PATH_LEAST = 1ull << 10;
 
 // Renders every path (REC: recording vertices) chunk by chunk; after(D, first,
 // last) turns a chunk into its part of the result.
@@ -644,11 +646,20 @@ int run_paths(pk_ctx* c, const char* what, const DiffParams& P, F after) {
   const uint32_t npix = c->W * c->H;
   const unsigned long long total = (unsigned long long)npix * (unsigned long long)P.spp;
   const unsigned long long per = 9 * 16 + 16 + 4 + (unsigned long long)P.depth * 16 * (REC ? 6 : 1);
-  const unsigned long long chunk = std::min(std::min(total, PATH_CHUNK), PATH_SPACE / per);
-  const size_t n = (size_t)chunk, head = 512;
+  unsigned long long chunk = std::min(std::min(total, PATH_CHUNK), PATH_SPACE / per);
+  const size_t head = 512;
   static_assert(sizeof(PathCount) + sizeof(PathTotal) <= 512, "header");
-  const size_t need = head + n * (size_t)per + 64;
-  if (c->diff_space.cap < need) c->diff_space.alloc(need);  // grows, at most to PATH_SPACE; goes with the context
+  for (;; chunk = (chunk + 1) / 2) {
+    const size_t need = head + (size_t)(chunk * per) + 64;
+    if (c->diff_space.cap >= need) break;
+    try {
+      c->diff_space.alloc(need);  // grows, at most to PATH_SPACE; goes with the context
+      break;
+    } catch (CudaError&) {
+      if (chunk <= PATH_LEAST) throw;
+    }
+  }
+  const size_t n = (size_t)chunk;
   unsigned char* at = c->diff_space.p;
   auto take = [&](size_t bytes) {
     unsigned char* p = at;

@@ -93,8 +93,42 @@ def replaced(src):
         assert np.array_equal(got.view(np.uint32), want.view(np.uint32))
 
 
+def paths(src):
+    """Differentiable rendering with less workspace than it would take: smaller chunks,
+    the same image and the same gradients (sums in another grouping)."""
+    import torch
+    from pike_gb300.diff import DiffScene
+    w, h, spp = 96, 64, 24
+    s = DiffScene(src, w, h, spp=spp, depth=3)
+    params = s.source_params(env_size=(64, 32))
+    s.set_env_sampling(params[2])
+    d = torch.rand((h, w, 4), device="cuda", generator=torch.Generator("cuda").manual_seed(3))
+    image, rays = s.render(*params), s.rays()
+    grads = s.backward(*params, d)
+    for limit in (20_000_000, 8_000_000):  # 147,456 paths take 31 MB forward, 67 MB backward
+        t = DiffScene(src, w, h, spp=spp, depth=3)
+        t.set_env_sampling(params[2])
+        memory(limit=limit)
+        got = t.render(*params)
+        assert L.pk_test_memory_failed() >= 2  # once more after the pools were given back, then halved
+        assert torch.equal(got.view(torch.int32), image.view(torch.int32)) and t.rays() == rays
+        assert torch.equal(t.render(*params).view(torch.int32), image.view(torch.int32))  # the space is kept
+        for name, a, b in zip(("albedo", "rough", "env"), t.backward(*params, d), grads):
+            assert (a - b).abs().max() <= 1e-4 * b.abs().max(), name
+        assert t.rays() == rays
+        memory()
+        del t
+    t = DiffScene(src, w, h, spp=spp, depth=3)
+    t.set_env_sampling(params[2])
+    memory(limit=1000)
+    refused(lambda: t.render(*params), _lib.PK_ERR_CUDA)
+    memory()
+    assert torch.equal(t.render(*params).view(torch.int32), image.view(torch.int32))
+
+
 if __name__ == "__main__":
     source = synth.small_scene(width=64, height=48)
     pools(source)
     replaced(source)
+    paths(source)
     print("ok")
