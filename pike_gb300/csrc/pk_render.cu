@@ -1021,6 +1021,10 @@ __global__ void k_set_state(Counters* ctr, CamDev* cam, int32_t samples, float t
   set_state(ctr, cam, samples, theta, cs, with_cam);
 }
 
+// The value two forms of one decode share, else NaN.
+__device__ __forceinline__ float agree(float a, float b) {
+  return __float_as_uint(a) == __float_as_uint(b) ? a : __int_as_float(0x7fc00000);
+}
 // Elementwise math probes (same numbering as the oracle's or_math).
 __global__ void k_math(int fn, const float* __restrict__ x, const float* __restrict__ y, float* __restrict__ out,
                        uint32_t n) {
@@ -1038,15 +1042,22 @@ __global__ void k_math(int fn, const float* __restrict__ x, const float* __restr
     case 6: r = log2_(a); break;
     case 7: r = pow_(a, b); break;
     case 8: r = snorm16_decode(__float_as_int(a)); break;
-    case 9:  // integer inputs, bit-cast; every byte of a word in turn
+    case 9:  // integer inputs, bit-cast (y: the other half of a pair); every form must agree
     case 10: {
-      const uint32_t v = (uint32_t)__float_as_int(a) & 0xffu, w = v << (8 * (i & 3u));
-      const uint32_t o = w ^ 0x80808080u;
-      switch (i & 3u) {
-        case 0: r = fn == 9 ? snorm8_pair<0, 1>(o, o).x : unorm8_byte<0>(w); break;
-        case 1: r = fn == 9 ? snorm8_pair<0, 1>(o, o).y : unorm8_byte<1>(w); break;
-        case 2: r = fn == 9 ? snorm8_offset<2>(o) : unorm8_byte<2>(w); break;
-        default: r = fn == 9 ? snorm8_offset<3>(o) : unorm8_byte<3>(w);
+      const uint32_t v = (uint32_t)__float_as_int(a) & 0xffu, u = (uint32_t)__float_as_int(b) & 0xffu;
+      if (fn == 9) {
+        const uint32_t vu = (v | (u << 8)) ^ 0x80808080u, uv = (u | (v << 8)) ^ 0x80808080u;
+        const uint32_t v2 = (v << 16) ^ 0x80808080u, u2 = (u << 16) ^ 0x80808080u;
+        r = snorm8_pair<0, 1>(vu, vu).x;
+        r = agree(r, snorm8_pair<0, 1>(uv, uv).y);
+        r = agree(r, snorm8_pair<2, 2>(v2, u2).x);
+        r = agree(r, snorm8_pair<2, 2>(u2, v2).y);
+        r = agree(r, snorm8_offset<2>(v2));
+      } else {
+        r = unorm8_byte<0>(v | (u << 8));
+        r = agree(r, unorm8_byte<1>((v << 8) | u));
+        r = agree(r, unorm8_byte<2>((v << 16) | (u << 24)));
+        r = agree(r, unorm8_byte<3>((v << 24) | (u << 16)));
       }
       break;
     }

@@ -184,6 +184,17 @@ def test_paths_need_the_whole_scene(pk_built, lacks):
         part.backward(*params, torch.ones((24, 32, 4), device="cuda"))
 
 
+@pytest.mark.parametrize("fn,div,signed", [(9, 127.0, True), (10, 255.0, False)])
+def test_byte_decodes_of_every_position_and_pair(ctx, fn, div, signed):
+    """Each byte position and each half of a packed decode, every value beside every
+    other: the IEEE quotient (max(v / d, -1) when signed)."""
+    v, u = (a.reshape(-1).astype(np.int32) for a in np.meshgrid(np.arange(256), np.arange(256)))
+    got = np.zeros(v.size, np.float32)
+    ctx.call("pk_math_eval", fn, ptr(v.view(np.float32)), ptr(u.view(np.float32)), ptr(got), v.size)
+    want = (v.astype(np.int8) if signed else v).astype(np.float32) / np.float32(div)
+    assert_bits_equal(got, np.maximum(want, np.float32(-1.0)), f"decode fn {fn}")
+
+
 def build_sweep(ctx, pos, tris):
     pos = np.ascontiguousarray(pos)
     attrs = np.zeros((pos.shape[0], 4), np.uint32)
