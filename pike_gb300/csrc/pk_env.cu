@@ -9,7 +9,7 @@
 // far the sequential sums can lie from them (k_env_next); a map where a bin's
 // edge falls within the bound, or whose sums are not finite, takes the walks
 // themselves on the host (walk_bins), as every map did before (a constant map is
-// one).  2048x1024, upload and build: 12.7 ms with the walks, of which the kernels
+// one, and some of 8192x4096 are: see the bound).  2048x1024, upload and build: 12.7 ms with the walks, of which the kernels
 // were 0.5 ms; 1.04 ms without.
 #include <cuda_runtime.h>
 
@@ -57,13 +57,18 @@ __global__ void k_env_radiance_f32(const float* __restrict__ rgb, uint32_t n, do
 // ---- the luminance bins ------------------------------------------------------
 // Radiance is not negative, so the sum of m doubles added one after the other
 // lies within (m - 1) 2^-53 (relative) of their exact sum, and so do the prefix
-// sums below with their 64 additions or fewer each.  With P the prefix sums of
-// the sorted radiance, T the total, nb the number of bins and B = T / nb the bin
-// size, the sequential sum from position i to before position k lies within
+// sums below with their 96 additions or fewer each.  With P the prefix sums of
+// the sorted radiance, T the total, nb the number of bins (32 to 256) and B = T / nb
+// the bin size, in units of 2^-53 T: the walk's sum up to a bin's end is off by at
+// most n / nb, the reference's T by n and so its B by n / nb, P(k) - P(i) by
+// 2 * 96 + 1, the B here by 98 / nb.  With
 //   tol = 2^-53 T (4 (n + 4096) / nb + 512)
-// of P(k) - P(i) even after the reference's own error in B (each of the three
-// terms counted at least twice): the walk's bin that starts at i ends at the
+// each is counted at least twice: the walk's bin that starts at i ends at the
 // first k with P(k) - P(i) >= B - tol, if that difference is also >= B + tol.
+// The mass of a texel falls with n where tol grows with it, so larger maps meet
+// an undecided edge sooner, and one is enough for the walks: of three log-normal
+// maps with a sun, replayed on the CPU, none at 1024x512, 2048x1024 or 4096x2048
+// has one, and one of three has two at 8192x4096.
 struct EnvPlan {
   double total, bin, tol;
   uint32_t status;  // 0: decided; 1: the walk has to decide

@@ -177,8 +177,10 @@ void scan_exclusive_u32(const Scratch& w, const uint32_t* in, uint32_t* out, uin
 // ---------------- exclusive scan of 64-bit values (three phases) -------------
 // Tiles of SCAN_TILE values: each block scans its tile and writes the tile's
 // sum; the tile sums are scanned recursively; a last pass adds each tile's
-// offset.  Integer sums do not depend on the grouping; a double prefix is the
-// result of at most 8 + 5 + 8 + 1 additions per level.
+// offset.  Integer sums do not depend on the grouping.  A tile's sum is the result
+// of at most 8 (thread) + 5 (warp) + 8 (warps) additions, a prefix within a tile
+// of 8 more and one, and every further level adds a tile's sum and the offset:
+// at most 30 + 2 * 22 for three levels.
 template <class T>
 __device__ __forceinline__ T warp_scan_incl(T v) {
   const int lane = threadIdx.x & 31;

@@ -127,8 +127,8 @@ void check_lookback(uint32_t err, const char* what);
 void scan_exclusive_u64(const Scratch& w, const unsigned long long* in, unsigned long long* out, size_t n);
 
 // Exclusive prefix sum of n doubles that are not negative (in may alias out);
-// enqueues and returns.  For n < 2^33 every prefix is the result of at most 64
-// additions, so it lies within 64 * 2^-53 (relative) of the exact sum.
+// enqueues and returns.  For n < 2^33 (three levels) every prefix is the result of
+// at most 96 additions, so it lies within 96 * 2^-53 (relative) of the exact sum.
 void scan_exclusive_f64(const Scratch& w, const double* in, double* out, size_t n);
 
 // Stable LSD radix sort of `segs` arrays of n (64-bit key, 32-bit value) pairs

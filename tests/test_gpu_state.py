@@ -195,6 +195,11 @@ def test_byte_decodes_of_every_position_and_pair(ctx, fn, div, signed):
     assert_bits_equal(got, np.maximum(want, np.float32(-1.0)), f"decode fn {fn}")
 
 
+def test_env_tables_of_three_scan_levels(ctx, oracle):
+    """More than 2^22 texels: the prefix sums behind the bins take a third level."""
+    test_gpu_edges.test_env_tables_at_sort_tiles_and_bin_edges(ctx, oracle, 4099, 1025, "log")
+
+
 def build_sweep(ctx, pos, tris):
     pos = np.ascontiguousarray(pos)
     attrs = np.zeros((pos.shape[0], 4), np.uint32)
